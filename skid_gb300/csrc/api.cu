@@ -325,6 +325,17 @@ void skid_ctx::collect_field_times(int nslots)
 
 // Move field at nm explicit positions from the current live copies, left in
 // probe_acc (the body of skid_field and skid_field_adjoint).
+__global__ void unsort_xyz(const int *__restrict__ perm, const float *__restrict__ in, int n,
+                           float *__restrict__ out)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const size_t o = 3 * (size_t)perm[i];
+        out[o] = in[3 * (size_t)i];
+        out[o + 1] = in[3 * (size_t)i + 1];
+        out[o + 2] = in[3 * (size_t)i + 2];
+    }
+}
+
 static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
 {
     cudaStream_t st = ctx->st;
@@ -336,9 +347,16 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
         return ctx->fail(SKID_ENOMEM);
     CK(cudaMemcpyAsync(xyz.p, mpos, 3 * (size_t)nm * sizeof(float), cudaMemcpyHostToDevice, st));
     xyz_to_pos4<<<grid_for(nm), 256, 0, st>>>(xyz.p, nm, p4.p); skid::note_launch();
-    iota_kernel<<<grid_for(nm), 256, 0, st>>>(act.p, nm); skid::note_launch();
+    // The caller's positions come in any order, and the 32 that share a warp
+    // share its walk: visited in Hilbert order, as the movers of a run are,
+    // the walk serves neighbours.  100k positions in particle order over
+    // 131k scatterers took 2.88 ms a call; sorted first, 0.48 ms with the sort.  A position's sum runs over the copies in tree order whichever
+    // positions share its warp, so the values do not change.
+    CK(curve_order(p4.p, nm, ctx->ss, st));
+    CK(cudaMemcpyAsync(act.p, ctx->ss.v0.p, (size_t)nm * sizeof(int), cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(act.p + nm, &nm, sizeof(int), cudaMemcpyHostToDevice, st));
-    FieldArgs a = ctx->field_args(0.0f, false, ctx->probe_acc.p);
+    // the kernel writes by sorted slot; xyz is free again after the packing
+    FieldArgs a = ctx->field_args(0.0f, false, xyz.p);
     a.mpos = p4.p;
     a.act = act.p;
     a.d_nA = act.p + nm;
@@ -349,6 +367,10 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
     a.touched = ctx->probe_touched();
     if (!a.touched) return ctx->fail(SKID_ENOMEM);
     CK(field_move(a, nm, st));
+    if (nm > 0) {
+        unsort_xyz<<<grid_for(nm), 256, 0, st>>>(act.p, xyz.p, nm, ctx->probe_acc.p); skid::note_launch();
+        CK(cudaGetLastError());
+    }
     return 0;
 }
 
