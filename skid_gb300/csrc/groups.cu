@@ -61,77 +61,153 @@ __device__ __forceinline__ float wrap_half(float d, float h, float L)
     return d;
 }
 
-// One warp per group.
-__global__ void group_props_kernel(const int *__restrict__ start, const int *__restrict__ count,
-                                   const int *__restrict__ members, int ng,
-                                   const float4 *__restrict__ pos4, const float4 *__restrict__ vel4,
-                                   const float4 *__restrict__ moved, float3 L, float3 hL,
-                                   float3 wrapHi, float3 wrapLo, int com, int rel_last,
-                                   skid_group *__restrict__ rec)
+// FP64 sums over members lane, lane + stride, ... of a group: mass, centre
+// terms, m v.  GP_BATCH members are loaded before any is added, so that the
+// latencies of the index and of the three gathers behind it overlap.
+constexpr int GP_BATCH = 4;
+constexpr int GP_THREADS = 256;
+
+struct GroupSums {
+    double m, cs[3], vs[3];
+};
+
+__device__ __forceinline__ void group_sums(GroupSums &S, const int *__restrict__ members, int s, int c,
+                                           int first, int stride, const float *rel,
+                                           const float4 *__restrict__ pos4,
+                                           const float4 *__restrict__ vel4,
+                                           const float4 *__restrict__ moved, float3 L, float3 hL, int com)
 {
-    int lane = threadIdx.x & 31;
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int g = warp; g < ng; g += nw) {
-        int s = start[g], c = count[g];
-        skid_group r = rec[g];
-        r.nMembers = c;
-        if (g == 0 || c == 0) {
-            if (lane == 0) {
-                if (g == 0) {
+    S.m = 0.0;
+    for (int d = 0; d < 3; ++d) S.cs[d] = S.vs[d] = 0.0;
+    for (int k0 = s + first; k0 < s + c; k0 += stride * GP_BATCH) {
+        int io[GP_BATCH];
+        float4 p[GP_BATCH], v[GP_BATCH], q[GP_BATCH];
+#pragma unroll
+        for (int b = 0; b < GP_BATCH; ++b)
+            io[b] = k0 + stride * b < s + c ? members[k0 + stride * b] : -1;
+#pragma unroll
+        for (int b = 0; b < GP_BATCH; ++b) {
+            const int i = io[b] < 0 ? 0 : io[b];
+            p[b] = pos4[i];
+            v[b] = vel4[i];
+            q[b] = com ? p[b] : moved[i];
+        }
+#pragma unroll
+        for (int b = 0; b < GP_BATCH; ++b) {
+            if (io[b] < 0) break;
+            S.m += p[b].w;
+            float del0 = wrap_half(fsub(q[b].x, rel[0]), hL.x, L.x);
+            float del1 = wrap_half(fsub(q[b].y, rel[1]), hL.y, L.y);
+            float del2 = wrap_half(fsub(q[b].z, rel[2]), hL.z, L.z);
+            if (com) {
+                S.cs[0] += fmul(p[b].w, del0); S.cs[1] += fmul(p[b].w, del1); S.cs[2] += fmul(p[b].w, del2);
+            } else {
+                S.cs[0] += del0; S.cs[1] += del1; S.cs[2] += del2;
+            }
+            S.vs[0] += fmul(p[b].w, v[b].x); S.vs[1] += fmul(p[b].w, v[b].y); S.vs[2] += fmul(p[b].w, v[b].z);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        S.m += __shfl_xor_sync(SKID_FULL, S.m, o);
+        for (int d = 0; d < 3; ++d) {
+            S.cs[d] += __shfl_xor_sync(SKID_FULL, S.cs[d], o);
+            S.vs[d] += __shfl_xor_sync(SKID_FULL, S.vs[d], o);
+        }
+    }
+}
+
+__device__ __forceinline__ void group_store(const GroupSums &S, int c, const float *rel, float3 L,
+                                            float3 wrapHi, float3 wrapLo, int com, skid_group &r)
+{
+    float fm = (float)S.m;
+    r.nMembers = c;
+    r.fMass = fm;
+    float wh[3] = {wrapHi.x, wrapHi.y, wrapHi.z}, wl[3] = {wrapLo.x, wrapLo.y, wrapLo.z};
+    float Ld[3] = {L.x, L.y, L.z};
+    for (int d = 0; d < 3; ++d) {
+        r.rel[d] = rel[d];
+        float cc = (float)S.cs[d];
+        cc = com ? cc / fm : cc / (float)c;
+        cc = fadd(cc, rel[d]);
+        if (cc > wh[d]) cc = fsub(cc, Ld[d]);
+        if (cc <= wl[d]) cc = fadd(cc, Ld[d]);
+        r.rCenter[d] = cc;
+        r.vcm[d] = (float)S.vs[d] / fm;
+        r.rBound[d] = 0.0f;
+    }
+    r.fRadius = 0.0f;
+}
+
+// One warp per group of up to GP_WARP_MAX members, the whole block for a
+// larger one: a warp alone walks 35k members in 1.04 ms (latency and the slow
+// FP64 adds), 0.155 ms for the block.
+constexpr int GP_WARP_MAX = 1024;
+
+__global__ void __launch_bounds__(GP_THREADS)
+group_props_kernel(const int *__restrict__ start, const int *__restrict__ count,
+                   const int *__restrict__ members, int ng, const float4 *__restrict__ pos4,
+                   const float4 *__restrict__ vel4, const float4 *__restrict__ moved, float3 L,
+                   float3 hL, float3 wrapHi, float3 wrapLo, int com, int rel_last,
+                   skid_group *__restrict__ rec)
+{
+    constexpr int NW = GP_THREADS / 32;
+    __shared__ GroupSums part[NW];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto reference = [&](int g, float *rel) {
+        const int s = start[g], c = count[g];
+        const float4 rp = pos4[members[rel_last ? s + c - 1 : s]];
+        rel[0] = rp.x;
+        rel[1] = rp.y;
+        rel[2] = rp.z;
+    };
+    // this block's groups: blockIdx.x + gridDim.x * k, eight at a time
+    for (int g0 = blockIdx.x; g0 < ng; g0 += gridDim.x * NW) {
+        const int g = g0 + w * gridDim.x;
+        if (g < ng) {
+            const int c = count[g];
+            if (g == 0) {
+                if (lane == 0) {
+                    skid_group r = rec[0];
+                    r.nMembers = c;
                     r.fMass = 0.0f;
                     for (int d = 0; d < 3; ++d) r.rel[d] = r.rCenter[d] = r.rBound[d] = r.vcm[d] = 0.0f;
                     r.fRadius = 0.0f;
+                    rec[0] = r;
                 }
-                rec[g] = r;
-            }
-            continue;
-        }
-        float4 rp = pos4[members[rel_last ? s + c - 1 : s]];
-        float rel[3] = {rp.x, rp.y, rp.z};
-        double m = 0.0, cs[3] = {0, 0, 0}, vs[3] = {0, 0, 0};
-        for (int k = s + lane; k < s + c; k += 32) {
-            int io = members[k];
-            float4 p = pos4[io];
-            float4 v = vel4[io];
-            float4 q = com ? p : moved[io];
-            m += p.w;
-            float del0 = wrap_half(fsub(q.x, rel[0]), hL.x, L.x);
-            float del1 = wrap_half(fsub(q.y, rel[1]), hL.y, L.y);
-            float del2 = wrap_half(fsub(q.z, rel[2]), hL.z, L.z);
-            if (com) {
-                cs[0] += fmul(p.w, del0); cs[1] += fmul(p.w, del1); cs[2] += fmul(p.w, del2);
-            } else {
-                cs[0] += del0; cs[1] += del1; cs[2] += del2;
-            }
-            vs[0] += fmul(p.w, v.x); vs[1] += fmul(p.w, v.y); vs[2] += fmul(p.w, v.z);
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            m += __shfl_xor_sync(SKID_FULL, m, o);
-            for (int d = 0; d < 3; ++d) {
-                cs[d] += __shfl_xor_sync(SKID_FULL, cs[d], o);
-                vs[d] += __shfl_xor_sync(SKID_FULL, vs[d], o);
+            } else if (c == 0) {
+                if (lane == 0) rec[g].nMembers = 0;
+            } else if (c <= GP_WARP_MAX) {
+                float rel[3];
+                GroupSums S;
+                reference(g, rel);
+                group_sums(S, members, start[g], c, lane, 32, rel, pos4, vel4, moved, L, hL, com);
+                if (lane == 0) group_store(S, c, rel, L, wrapHi, wrapLo, com, rec[g]);
             }
         }
-        if (lane == 0) {
-            float fm = (float)m;
-            r.fMass = fm;
-            float wh[3] = {wrapHi.x, wrapHi.y, wrapHi.z}, wl[3] = {wrapLo.x, wrapLo.y, wrapLo.z};
-            float Ld[3] = {L.x, L.y, L.z};
-            for (int d = 0; d < 3; ++d) {
-                r.rel[d] = rel[d];
-                float cc = (float)cs[d];
-                cc = com ? cc / fm : cc / (float)c;
-                cc = fadd(cc, rel[d]);
-                if (cc > wh[d]) cc = fsub(cc, Ld[d]);
-                if (cc <= wl[d]) cc = fadd(cc, Ld[d]);
-                r.rCenter[d] = cc;
-                r.vcm[d] = (float)vs[d] / fm;
-                r.rBound[d] = 0.0f;
+        for (int k = 0; k < NW; ++k) {
+            const int gl = g0 + k * gridDim.x;
+            if (gl >= ng) break;
+            const int c = count[gl];
+            if (gl == 0 || c <= GP_WARP_MAX) continue;
+            float rel[3];
+            GroupSums S;
+            reference(gl, rel);
+            group_sums(S, members, start[gl], c, threadIdx.x, GP_THREADS, rel, pos4, vel4, moved, L, hL, com);
+            __syncthreads();
+            if (lane == 0) part[w] = S;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                // warp sums in warp order
+                for (int q = 1; q < NW; ++q) {
+                    S.m += part[q].m;
+                    for (int d = 0; d < 3; ++d) {
+                        S.cs[d] += part[q].cs[d];
+                        S.vs[d] += part[q].vs[d];
+                    }
+                }
+                group_store(S, c, rel, L, wrapHi, wrapLo, com, rec[gl]);
             }
-            r.fRadius = 0.0f;
-            rec[g] = r;
         }
     }
 }
@@ -228,10 +304,12 @@ cudaError_t group_props(GroupState &G, const float4 *pos4, const float4 *vel4, c
     cudaError_t e;
     if ((e = dalloc(G.rec, G.nGroup))) return e;
     float3 hL = make_float3(0.5f * L.x, 0.5f * L.y, 0.5f * L.z);
-    int warps = G.nGroup;
-    int blocks = min((warps * 32 + 255) / 256, num_sms() * 16);
+    // eight groups a block, but while there are few, a block each
+    int blocks = (G.nGroup + GP_THREADS / 32 - 1) / (GP_THREADS / 32);
+    if (blocks < num_sms() * 4) blocks = min(G.nGroup, num_sms() * 4);
+    blocks = min(blocks, num_sms() * 16);
     if (blocks < 1) blocks = 1;
-    group_props_kernel<<<blocks, 256, 0, st>>>(G.start.p, G.count.p, G.members.p, G.nGroup, pos4,
+    group_props_kernel<<<blocks, GP_THREADS, 0, st>>>(G.start.p, G.count.p, G.members.p, G.nGroup, pos4,
                                                vel4, moved, L, hL, wrapHi, wrapLo, com ? 1 : 0,
                                                rel_last ? 1 : 0, G.rec.p); skid::note_launch();
     return cudaGetLastError();
