@@ -365,8 +365,6 @@ __global__ void scatter_grad(const int *__restrict__ sidx, const float *__restri
 
 // ---- group potential energy ----
 
-constexpr int PA_TILE = 128;
-
 // psi(r, e) as kdCellPot evaluates it (grav.h:11-31) and psi'(r)/r.
 // Beyond the softening (r >= 2h, certain once d2 clears (2h)^2 by the margin
 // below) and for Plummer softening, psi comes from the hardware reciprocal
@@ -406,121 +404,348 @@ __device__ __forceinline__ float wrap_rel(float d, float h)
     return d;
 }
 
+// The pair sums of the selected groups, split into items of PA_TILE rows by
+// up to `chunk` columns of one group.  FP32 issue bounds it: per pair 16 FP32
+// operations with the gradient, 10 without, and a reciprocal square root.  A
+// thread carries two rows in packed FP32 operands (half the issue slots), a
+// column read from shared memory serving both; tile pairs whose boxes are
+// further apart than the softening run without any test.  Columns are split
+// as well as rows because a group's rows alone leave the GPU idle: 24 groups
+// of up to 35k members (140k rows, 2.9e9 pairs) gave 14 warps an SM and
+// items of 35k columns, 9.9 ms a call with or without the gradient.  Now 2.5
+// and 1.75 ms.  An item's Kahan-compensated row sums are combined in FP64,
+// where adding a few floats is exact, and rounded to float once at the end,
+// which is what one compensated sum over the whole row gives.
+constexpr int PA_TILE = 128;
+constexpr int PA_THREADS = PA_TILE / 2;
+// Columns per item: long ones (fewer partial sums) once the pairs fill every
+// SM with PA_FILL items of that length, short ones below, where an item's
+// serial walk over its columns would set the time.
+constexpr int PA_CHUNK = 1024, PA_CHUNK_MIN = 128;
+constexpr long long PA_FILL = 32;
+// From this many pairs the members are packed in Hilbert order: a warp takes
+// the softened pair factor (divides, a root) whenever any of its pairs lies
+// inside the softening, and with members in file order some pair of 64 does
+// in 40-50 % of the steps of a halo whose pairs are 2-3 % inside it; in
+// Hilbert order in 12-20 %.  2.9e9 pairs: 3.14 ms
+// (with gradient) and 2.31 ms in file order, 2.49 and 1.75 ms in Hilbert
+// order, for 0.1 ms of sorting.
+constexpr double PA_SORT_PAIRS = 1.5e8;
+
+struct PotSlot {
+    long long item0;            // items of the slots before this one
+    long long row0;             // rows of the slots before this one
+    long long tile0;            // row tiles of the slots before this one
+    int g, n, nchunk;
+    float v;
+};
+
 struct PotAdjArgs {
-    const int2 *items;          // (selection slot, tile)
-    int nitems;
-    const int *gsel;            // group id per slot
-    const float *v;             // cotangent per slot (may be null: no gradient)
-    const int *gstart, *gcount, *members;
+    const PotSlot *slots;
+    int nslot, chunk;
+    long long nitems, nrows;
+    const int *gstart, *members;
     const float4 *pos4, *vel4;  // (x, y, z, m), (vx, vy, vz, soft)
     const skid_group *rec;
     float3 hP;
     float G;
     int plummer;
+    const uint32_t *perm;       // packed row -> row in member order (null: the same)
+    float4 *rm;                 // packed rows: position relative to the group's rel, mass
+    float *re;                  // packed rows: softening
+    int *rio;                   // packed rows: iOrder
+    float4 *tlo, *thi;          // per row tile: its box; tlo.w: its largest softening
+    long long ntile;
+    double *acc;                // per row: sum_j m_j psi, then (gradient) sum_j m_j psi'/r (x_i - x_j)
     double *E;                  // per slot
     float *grad;                // 3n by iOrder (zeroed) or null
 };
 
-// One (selection slot, row tile) per block iteration: PA_TILE / 2 threads,
-// each with rows t and t + PA_TILE / 2, over every column tile of the group.
-constexpr int PA_THREADS = PA_TILE / 2;
+// The slot holding row (or item) k: the last one that starts at or before it.
+template <bool ROWS>
+__device__ __forceinline__ int pa_slot(const PotAdjArgs &a, long long k)
+{
+    int lo = 0, hi = a.nslot - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if ((ROWS ? a.slots[mid].row0 : a.slots[mid].item0) <= k) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
 
-struct PaRow {
-    float3 r;
-    float e, m;
-    int io;
-    bool v;
-    float phi, phic, gx, gy, gz;   // Kahan-compensated sum_j m_j psi_ij; sum_j m_j psi'/r (x_i - x_j)
+__device__ __forceinline__ float3 pa_rel(const PotAdjArgs &a, const PotSlot &S, float4 p)
+{
+    const float *rel = a.rec[S.g].rel;
+    return make_float3(wrap_rel(fsub(p.x, rel[0]), a.hP.x), wrap_rel(fsub(p.y, rel[1]), a.hP.y),
+                       wrap_rel(fsub(p.z, rel[2]), a.hP.z));
+}
+
+// The largest |coordinate| of any row (order-preserving bits, zeroed before).
+__global__ void pa_extent(PotAdjArgs a, unsigned *ext)
+{
+    float m = 0.0f;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
+         k += (long long)gridDim.x * blockDim.x) {
+        const PotSlot S = a.slots[pa_slot<true>(a, k)];
+        const float3 r = pa_rel(a, S, a.pos4[a.members[a.gstart[S.g] + (int)(k - S.row0)]]);
+        m = fmaxf(m, fmaxf(fabsf(r.x), fmaxf(fabsf(r.y), fabsf(r.z))));
+    }
+    const unsigned u = __reduce_max_sync(SKID_FULL, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) atomicMax(ext, u);
+}
+
+// Sort keys: the slot, then the Hilbert index of the relative position on a
+// 2^13 grid.
+constexpr int PA_KEY_BITS = 39;
+
+__global__ void pa_keys(PotAdjArgs a, const unsigned *ext, uint64_t *keys, uint32_t *vals)
+{
+    const float R = fmaxf(__uint_as_float(*ext), 1e-30f), sc = 4095.5f / R;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
+         k += (long long)gridDim.x * blockDim.x) {
+        const int s = pa_slot<true>(a, k);
+        const PotSlot S = a.slots[s];
+        const float3 r = pa_rel(a, S, a.pos4[a.members[a.gstart[S.g] + (int)(k - S.row0)]]);
+        auto cell = [&](float x) {
+            return (uint32_t)fminf(fmaxf((x + R) * sc, 0.0f), 8191.0f);
+        };
+        keys[k] = ((uint64_t)s << PA_KEY_BITS) | hilbert3<13>(cell(r.x), cell(r.y), cell(r.z));
+        vals[k] = (uint32_t)k;
+    }
+}
+
+__global__ void pa_pack(PotAdjArgs a)
+{
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
+         k += (long long)gridDim.x * blockDim.x) {
+        const PotSlot S = a.slots[pa_slot<true>(a, k)];
+        const long long from = a.perm ? (long long)a.perm[k] : k;
+        const int io = a.members[a.gstart[S.g] + (int)(from - S.row0)];
+        const float4 p = a.pos4[io];
+        const float3 r = pa_rel(a, S, p);
+        a.rm[k] = make_float4(r.x, r.y, r.z, p.w);
+        a.re[k] = a.vel4[io].w;
+        a.rio[k] = io;
+    }
+}
+
+// The box and largest softening of every tile of PA_TILE packed rows, a warp
+// each.
+__global__ void pa_boxes(PotAdjArgs a)
+{
+    const int lane = threadIdx.x & 31;
+    const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long t = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); t < a.ntile;
+         t += nw) {
+        int lo_s = 0, hi_s = a.nslot - 1;
+        while (lo_s < hi_s) {
+            const int mid = (lo_s + hi_s + 1) >> 1;
+            if (a.slots[mid].tile0 <= t) lo_s = mid;
+            else hi_s = mid - 1;
+        }
+        const PotSlot S = a.slots[lo_s];
+        float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f);
+        float4 hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f);
+        const int i0 = (int)(t - S.tile0) * PA_TILE;
+        for (int i = i0 + lane; i < min(i0 + PA_TILE, S.n); i += 32) {
+            const float4 r = a.rm[S.row0 + i];
+            lo.x = fminf(lo.x, r.x); lo.y = fminf(lo.y, r.y); lo.z = fminf(lo.z, r.z);
+            hi.x = fmaxf(hi.x, r.x); hi.y = fmaxf(hi.y, r.y); hi.z = fmaxf(hi.z, r.z);
+            lo.w = fmaxf(lo.w, a.re[S.row0 + i]);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            lo.x = fminf(lo.x, __shfl_xor_sync(SKID_FULL, lo.x, o));
+            lo.y = fminf(lo.y, __shfl_xor_sync(SKID_FULL, lo.y, o));
+            lo.z = fminf(lo.z, __shfl_xor_sync(SKID_FULL, lo.z, o));
+            hi.x = fmaxf(hi.x, __shfl_xor_sync(SKID_FULL, hi.x, o));
+            hi.y = fmaxf(hi.y, __shfl_xor_sync(SKID_FULL, hi.y, o));
+            hi.z = fmaxf(hi.z, __shfl_xor_sync(SKID_FULL, hi.z, o));
+            lo.w = fmaxf(lo.w, __shfl_xor_sync(SKID_FULL, lo.w, o));
+        }
+        if (lane == 0) {
+            a.tlo[t] = lo;
+            a.thi[t] = hi;
+        }
+    }
+}
+
+// A thread's two rows, packed: position, the Kahan-compensated sum_j m_j psi
+// and sum_j m_j psi'/r (x_i - x_j).
+struct PaRows {
+    f32x2 x, y, z;
+    f32x2 phi, phic, gx, gy, gz;
 };
 
-__device__ __forceinline__ void pa_row_init(PaRow &w, const PotAdjArgs &a, int s, int n, int i,
-                                            const float *rel)
+__device__ __forceinline__ float rsqrt_ftz(float x)
 {
-    w.v = i < n;
-    w.io = w.v ? a.members[s + i] : 0;
-    float4 p = a.pos4[w.io];
-    w.m = p.w;
-    w.e = a.vel4[w.io].w;
-    w.r = make_float3(wrap_rel(fsub(p.x, rel[0]), a.hP.x), wrap_rel(fsub(p.y, rel[1]), a.hP.y),
-                      wrap_rel(fsub(p.z, rel[2]), a.hP.z));
-    w.phi = w.phic = w.gx = w.gy = w.gz = 0.0f;
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-__device__ __forceinline__ void pa_row_add(PaRow &w, float4 rj, float ej, int plummer)
+// Both rows' term for one column, given psi (and psi'/r) of each.
+template <bool GRAD>
+__device__ __forceinline__ void pa_add(PaRows &w, f32x2 dx, f32x2 dy, f32x2 dz, f32x2 m, f32x2 psi,
+                                       f32x2 gr)
 {
-    float dx = w.r.x - rj.x, dy = w.r.y - rj.y, dz = w.r.z - rj.z;
-    float psi, gr;
-    pair_psi(dx * dx + dy * dy + dz * dz, w.e + ej, plummer, psi, gr);
-    float y = rj.w * psi - w.phic;
-    float tt = w.phi + y;
-    w.phic = (tt - w.phi) - y;
+    const f32x2 y = fma2(m, psi, w.phic);       // phic holds minus the compensation
+    const f32x2 tt = add2(w.phi, y);
+    w.phic = sub2(y, sub2(tt, w.phi));
     w.phi = tt;
-    float c = rj.w * gr;
-    w.gx += c * dx;
-    w.gy += c * dy;
-    w.gz += c * dz;
+    if (GRAD) {
+        const f32x2 c = mul2(m, gr);
+        w.gx = fma2(c, dx, w.gx);
+        w.gy = fma2(c, dy, w.gy);
+        w.gz = fma2(c, dz, w.gz);
+    }
 }
 
+// A column in shared memory: (-x, -x, -y, -y), (-z, -z, m, m), both halves of
+// the packed operands.
+struct PaCol {
+    ulonglong2 xy, zm;
+};
+
+template <bool GRAD>
 __global__ void __launch_bounds__(PA_THREADS) potential_adjoint_kernel(PotAdjArgs a)
 {
-    __shared__ float4 sr[PA_TILE];
+    __shared__ PaCol sc[PA_TILE];
     __shared__ float ss[PA_TILE];
-    __shared__ double red[PA_THREADS / 32];
     const int tid = threadIdx.x;
-    for (int it = blockIdx.x; it < a.nitems; it += gridDim.x) {
-        int2 item = a.items[it];
-        int slot = item.x;
-        int g = a.gsel[slot];
-        int s = a.gstart[g], n = a.gcount[g];
-        const float *rel = a.rec[g].rel;
-        const int i0 = item.y * PA_TILE + tid, i1 = i0 + PA_THREADS;
-        PaRow r0, r1;
-        pa_row_init(r0, a, s, n, i0, rel);
-        pa_row_init(r1, a, s, n, i1, rel);
-        for (int jb = 0; jb < n; jb += PA_TILE) {
+    for (long long it = blockIdx.x; it < a.nitems; it += gridDim.x) {
+        const PotSlot S = a.slots[pa_slot<false>(a, it)];
+        const int k = (int)(it - S.item0);
+        const int tile = k / S.nchunk, ch = k - tile * S.nchunk;
+        const int n = S.n;
+        const float4 *rm = a.rm + S.row0;
+        const float *re = a.re + S.row0;
+        const int i0 = tile * PA_TILE + tid, i1 = i0 + PA_THREADS;
+        const float4 alo = a.tlo[S.tile0 + tile], ahi = a.thi[S.tile0 + tile];
+        // rows past the end repeat the last member and are not stored
+        const float4 q0 = rm[min(i0, n - 1)], q1 = rm[min(i1, n - 1)];
+        const float e0 = re[min(i0, n - 1)], e1 = re[min(i1, n - 1)];
+        PaRows w;
+        w.x = pack2(q0.x, q1.x);
+        w.y = pack2(q0.y, q1.y);
+        w.z = pack2(q0.z, q1.z);
+        w.phi = w.phic = w.gx = w.gy = w.gz = 0ull;
+        const int c0 = ch * a.chunk, c1 = min(n, c0 + a.chunk);
+        for (int jb = c0; jb < c1; jb += PA_TILE) {
+            const int cnt = min(PA_TILE, c1 - jb);
+            const float4 blo = a.tlo[S.tile0 + jb / PA_TILE], bhi = a.thi[S.tile0 + jb / PA_TILE];
             __syncthreads();
-            for (int c = tid; c < PA_TILE; c += PA_THREADS) {
-                int j = jb + c;
-                if (j < n) {
-                    int jo = a.members[s + j];
-                    float4 q = a.pos4[jo];
-                    sr[c] = make_float4(wrap_rel(fsub(q.x, rel[0]), a.hP.x), wrap_rel(fsub(q.y, rel[1]), a.hP.y),
-                                        wrap_rel(fsub(q.z, rel[2]), a.hP.z), q.w);
-                    ss[c] = a.vel4[jo].w;
+            for (int c = tid; c < cnt; c += PA_THREADS) {
+                const float4 r = rm[jb + c];
+                PaCol o;
+                o.xy = make_ulonglong2(pack2(-r.x, -r.x), pack2(-r.y, -r.y));
+                o.zm = make_ulonglong2(pack2(-r.z, -r.z), pack2(r.w, r.w));
+                sc[c] = o;
+                ss[c] = re[jb + c];
+            }
+            __syncthreads();
+            // far is at or above every pair's (2h)^2 (1 + 1e-6) in the tile
+            // pair (infinite for Plummer softening): beyond it pair_psi is
+            // the hardware 1/r, taken without forming the pair's softening
+            float far = INFINITY;
+            if (!a.plummer) far = fmaxf((alo.w + blo.w) * (alo.w + blo.w) * 1.000001f, 1e-30f);
+            // the squared gap between the tiles' boxes: float subtraction,
+            // product and sum are monotonic, so no pair's d2 is below it
+            const float gx = fmaxf(fmaxf(blo.x - ahi.x, alo.x - bhi.x), 0.0f);
+            const float gy = fmaxf(fmaxf(blo.y - ahi.y, alo.y - bhi.y), 0.0f);
+            const float gz = fmaxf(fmaxf(blo.z - ahi.z, alo.z - bhi.z), 0.0f);
+            if (__fmaf_rn(gz, gz, __fmaf_rn(gx, gx, gy * gy)) >= far) {
+                // every pair beyond the softening
+#pragma unroll 4
+                for (int c = 0; c < cnt; ++c) {
+                    const PaCol o = sc[c];
+                    const f32x2 dx = add2(w.x, o.xy.x), dy = add2(w.y, o.xy.y), dz = add2(w.z, o.zm.x);
+                    const float2 d2 = unpack2(fma2(dz, dz, fma2(dx, dx, mul2(dy, dy))));
+                    const f32x2 psi = pack2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y));
+                    f32x2 gr = 0ull;
+                    if (GRAD) gr = mul2(mul2(psi, psi), mul2(psi, 0xbf800000bf800000ull));
+                    pa_add<GRAD>(w, dx, dy, dz, o.zm.y, psi, gr);
+                }
+            } else {
+                // a step without any pair inside the softening takes the same
+                // form (a member with itself, at d2 = 0, is inside)
+                const int s0 = i0 - jb, s1 = i1 - jb;   // the rows' own columns, if here
+#pragma unroll 2
+                for (int c = 0; c < cnt; ++c) {
+                    const PaCol o = sc[c];
+                    const f32x2 dx = add2(w.x, o.xy.x), dy = add2(w.y, o.xy.y), dz = add2(w.z, o.zm.x);
+                    const float2 d2 = unpack2(fma2(dz, dz, fma2(dx, dx, mul2(dy, dy))));
+                    f32x2 psi = pack2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y)), gr = 0ull;
+                    if (GRAD) gr = mul2(mul2(psi, psi), mul2(psi, 0xbf800000bf800000ull));
+                    if (!(d2.x >= far && d2.y >= far)) {
+                        float2 p = unpack2(psi), q = unpack2(gr);
+                        if (!(d2.x >= far)) pair_psi(d2.x, e0 + ss[c], a.plummer, p.x, q.x);
+                        if (!(d2.y >= far)) pair_psi(d2.y, e1 + ss[c], a.plummer, p.y, q.y);
+                        // no pair of a member with itself
+                        if (c == s0) p.x = q.x = 0.0f;
+                        if (c == s1) p.y = q.y = 0.0f;
+                        psi = pack2(p.x, p.y);
+                        gr = pack2(q.x, q.y);
+                    }
+                    pa_add<GRAD>(w, dx, dy, dz, o.zm.y, psi, gr);
                 }
             }
-            __syncthreads();
-            const int cnt = min(PA_TILE, n - jb);
-            for (int k = 0; k < cnt; ++k) {
-                const float4 rj = sr[k];
-                const float ej = ss[k];
-                if (r0.v && jb + k != i0) pa_row_add(r0, rj, ej, a.plummer);
-                if (r1.v && jb + k != i1) pa_row_add(r1, rj, ej, a.plummer);
+        }
+        constexpr int NA = GRAD ? 4 : 1;
+        const float2 phi = unpack2(w.phi), phic = unpack2(w.phic);
+        const float2 hx = unpack2(w.gx), hy = unpack2(w.gy), hz = unpack2(w.gz);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = q ? i1 : i0;
+            if (i >= n) continue;
+            double *o = a.acc + NA * (S.row0 + i);
+            atomicAdd(o, (double)(q ? phi.y : phi.x) + (double)(q ? phic.y : phic.x));
+            if (GRAD) {
+                atomicAdd(o + 1, (double)(q ? hx.y : hx.x));
+                atomicAdd(o + 2, (double)(q ? hy.y : hy.x));
+                atomicAdd(o + 3, (double)(q ? hz.y : hz.x));
             }
         }
-        // E contribution -1/2 G m_i phi_i, summed over the tile in FP64
-        double e = (r0.v ? -0.5 * (double)a.G * (double)r0.m * (double)r0.phi : 0.0) +
-                   (r1.v ? -0.5 * (double)a.G * (double)r1.m * (double)r1.phi : 0.0);
+    }
+}
+
+// E_s = -1/2 G sum_i m_i phi_i in FP64, one block per slot, in a fixed order.
+constexpr int PE_THREADS = 512;
+
+__global__ void __launch_bounds__(PE_THREADS) pa_energy(PotAdjArgs a)
+{
+    __shared__ double red[PE_THREADS / 32];
+    for (int s = blockIdx.x; s < a.nslot; s += gridDim.x) {
+        const PotSlot S = a.slots[s];
+        const int NA = a.grad ? 4 : 1;
+        double e = 0.0;
+        for (int i = threadIdx.x; i < S.n; i += PE_THREADS)
+            e += -0.5 * (double)a.G * (double)a.rm[S.row0 + i].w *
+                 (double)(float)a.acc[NA * (S.row0 + i)];
         for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(SKID_FULL, e, o);
-        if ((tid & 31) == 0) red[tid >> 5] = e;
         __syncthreads();
-        if (tid == 0) {
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
+        __syncthreads();
+        if (threadIdx.x == 0) {
             double t = 0.0;
-            for (int k = 0; k < PA_THREADS / 32; ++k) t += red[k];
-            atomicAdd(a.E + slot, t);
+            for (int k = 0; k < PE_THREADS / 32; ++k) t += red[k];
+            a.E[s] = t;
         }
-        if (a.grad) {
-            const PaRow *rows[2] = {&r0, &r1};
-            for (int q = 0; q < 2; ++q) {
-                const PaRow &w = *rows[q];
-                if (!w.v) continue;
-                float c = -a.G * w.m * a.v[slot];
-                float *o = a.grad + 3 * (size_t)w.io;
-                o[0] = c * w.gx;
-                o[1] = c * w.gy;
-                o[2] = c * w.gz;
-            }
-        }
+    }
+}
+
+// The gradient by iOrder, one thread per packed row.
+__global__ void pa_gradient(PotAdjArgs a)
+{
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
+         k += (long long)gridDim.x * blockDim.x) {
+        const PotSlot S = a.slots[pa_slot<true>(a, k)];
+        const float c = -a.G * a.rm[k].w * S.v;
+        float *o = a.grad + 3 * (size_t)a.rio[k];
+        o[0] = c * (float)a.acc[4 * k + 1];
+        o[1] = c * (float)a.acc[4 * k + 2];
+        o[2] = c * (float)a.acc[4 * k + 3];
     }
 }
 
@@ -580,40 +805,60 @@ cudaError_t density_adjoint(const Tree &t, const float *ball2_sorted, const int 
 
 cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const float4 *vel4, int n,
                               float3 period, float Gc, int plummer, int nSel, const int *h_sel,
-                              const float *h_v, bool want_grad, AdjointState &A, cudaStream_t st)
+                              const float *h_v, bool want_grad, AdjointState &A, SortScratch &ss,
+                              cudaStream_t st)
 {
     cudaError_t e;
     std::vector<int> counts(G.nGroup);
     if ((e = cudaMemcpyAsync(counts.data(), G.count.p, G.nGroup * sizeof(int), cudaMemcpyDeviceToHost, st)))
         return e;
     if ((e = cudaStreamSynchronize(st))) return e;
-    std::vector<int2> items;
+    // items and rows per selected group: columns split into chunks of a
+    // length chosen by the pairs there are
+    double pairs = 0.0;
+    for (int s = 0; s < nSel; ++s) pairs += (double)counts[h_sel[s]] * (double)counts[h_sel[s]];
+    int chunk = PA_CHUNK;
+    while (chunk > PA_CHUNK_MIN && pairs < (double)(PA_FILL * num_sms()) * PA_TILE * chunk) chunk >>= 1;
+    std::vector<PotSlot> slots(nSel);
+    long long nitems = 0, nrows = 0, ntile = 0;
     for (int s = 0; s < nSel; ++s) {
-        int c = counts[h_sel[s]];
-        for (int t = 0; t * PA_TILE < c; ++t) items.push_back(make_int2(s, t));
+        const int c = counts[h_sel[s]];
+        PotSlot &S = slots[s];
+        S.item0 = nitems;
+        S.row0 = nrows;
+        S.tile0 = ntile;
+        S.g = h_sel[s];
+        S.n = c;
+        S.nchunk = (c + chunk - 1) / chunk;
+        S.v = h_v ? h_v[s] : 0.0f;
+        nitems += (long long)((c + PA_TILE - 1) / PA_TILE) * S.nchunk;
+        nrows += c;
+        ntile += (c + PA_TILE - 1) / PA_TILE;
     }
-    size_t ni = items.size();
-    if ((e = dalloc(A.items, ni > 0 ? ni : 1)) || (e = dalloc(A.gsel, nSel > 0 ? nSel : 1)) ||
-        (e = dalloc(A.v, nSel > 0 ? nSel : 1)) || (e = dalloc(A.E, nSel > 0 ? nSel : 1)) ||
-        (e = dalloc(A.out, 3 * (size_t)(n > 0 ? n : 1))))
-        return e;
-    if (ni && (e = cudaMemcpyAsync(A.items.p, items.data(), ni * sizeof(int2), cudaMemcpyHostToDevice, st)))
+    const int na = want_grad ? 4 : 1;
+    if ((e = dalloc(A.slots, (size_t)(nSel > 0 ? nSel : 1) * sizeof(PotSlot))) ||
+        (e = dalloc(A.E, nSel > 0 ? nSel : 1)) || (e = dalloc(A.out, 3 * (size_t)(n > 0 ? n : 1))) ||
+        (e = dalloc(A.rm, (size_t)(nrows > 0 ? nrows : 1))) ||
+        (e = dalloc(A.re, (size_t)(nrows > 0 ? nrows : 1))) ||
+        (e = dalloc(A.rio, (size_t)(nrows > 0 ? nrows : 1))) ||
+        (e = dalloc(A.tbox, 2 * (size_t)(ntile > 0 ? ntile : 1))) ||
+        (e = dalloc(A.acc, (size_t)na * (nrows > 0 ? nrows : 1))))
         return e;
     if (nSel) {
-        if ((e = cudaMemcpyAsync(A.gsel.p, h_sel, nSel * sizeof(int), cudaMemcpyHostToDevice, st))) return e;
-        if (h_v && (e = cudaMemcpyAsync(A.v.p, h_v, nSel * sizeof(float), cudaMemcpyHostToDevice, st)))
+        if ((e = cudaMemcpyAsync(A.slots.p, slots.data(), nSel * sizeof(PotSlot), cudaMemcpyHostToDevice, st)))
             return e;
         if ((e = cudaMemsetAsync(A.E.p, 0, nSel * sizeof(double), st))) return e;
     }
     if ((e = cudaMemsetAsync(A.out.p, 0, 3 * (size_t)(n > 0 ? n : 1) * sizeof(float), st))) return e;
-    if (!ni) return cudaSuccess;
+    if (!nitems) return cudaSuccess;
+    if ((e = cudaMemsetAsync(A.acc.p, 0, (size_t)na * nrows * sizeof(double), st))) return e;
     PotAdjArgs a;
-    a.items = A.items.p;
-    a.nitems = (int)ni;
-    a.gsel = A.gsel.p;
-    a.v = A.v.p;
+    a.slots = reinterpret_cast<const PotSlot *>(A.slots.p);
+    a.nslot = nSel;
+    a.chunk = chunk;
+    a.nitems = nitems;
+    a.nrows = nrows;
     a.gstart = G.start.p;
-    a.gcount = G.count.p;
     a.members = G.members.p;
     a.pos4 = pos4;
     a.vel4 = vel4;
@@ -622,10 +867,40 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
                        (float)(0.5 * (double)period.z));
     a.G = Gc;
     a.plummer = plummer;
+    a.perm = nullptr;
+    a.rm = A.rm.p;
+    a.re = A.re.p;
+    a.rio = A.rio.p;
+    a.tlo = A.tbox.p;
+    a.thi = A.tbox.p + ntile;
+    a.ntile = ntile;
+    a.acc = A.acc.p;
     a.E = A.E.p;
     a.grad = want_grad ? A.out.p : nullptr;
-    int blocks = (int)(ni < (size_t)num_sms() * 32 ? ni : (size_t)num_sms() * 32);
-    potential_adjoint_kernel<<<blocks, PA_THREADS, 0, st>>>(a); note_launch();
+    const long long most = (long long)num_sms() * 32;
+    const int rgrid = grid_for((int)(nrows < (1 << 30) ? nrows : 1 << 30));
+    if (pairs >= PA_SORT_PAIRS && nrows < (1ll << 31)) {
+        int sbits = 0;
+        while ((1ll << sbits) < nSel) ++sbits;
+        if ((e = dalloc(ss.k0, (size_t)nrows)) || (e = dalloc(ss.k1, (size_t)nrows)) ||
+            (e = dalloc(ss.v0, (size_t)nrows)) || (e = dalloc(ss.v1, (size_t)nrows)) ||
+            (e = dalloc(ss.box, 8)) || (e = cudaMemsetAsync(ss.box.p, 0, sizeof(unsigned), st)))
+            return e;
+        pa_extent<<<rgrid, 256, 0, st>>>(a, ss.box.p); note_launch();
+        pa_keys<<<rgrid, 256, 0, st>>>(a, ss.box.p, ss.k0.p, ss.v0.p); note_launch();
+        if ((e = radix_sort(ss, (int)nrows, PA_KEY_BITS + sbits, st))) return e;
+        a.perm = ss.v0.p;
+    }
+    pa_pack<<<rgrid, 256, 0, st>>>(a); note_launch();
+    pa_boxes<<<grid_for((int)(ntile < (1 << 25) ? ntile * 32 : 1 << 30)), 256, 0, st>>>(a); note_launch();
+    const int blocks = (int)(nitems < most ? nitems : most);
+    if (want_grad) potential_adjoint_kernel<true><<<blocks, PA_THREADS, 0, st>>>(a);
+    else potential_adjoint_kernel<false><<<blocks, PA_THREADS, 0, st>>>(a);
+    note_launch();
+    pa_energy<<<nSel < num_sms() * 4 ? nSel : num_sms() * 4, PE_THREADS, 0, st>>>(a); note_launch();
+    if (want_grad) {
+        pa_gradient<<<rgrid, 256, 0, st>>>(a); note_launch();
+    }
     return cudaGetLastError();
 }
 

@@ -176,7 +176,7 @@ int skid_potential_adjoint(skid_ctx *ctx, int iSoftType, float G, int nSel, cons
     cudaStream_t st = ctx->st;
     cudaError_t e = potential_adjoint(ctx->G, ctx->pos4.p, ctx->vel4.p, ctx->n, ctx->L, G,
                                       iSoftType == SKID_SOFT_PLUMMER, nSel, sel, v, dLdx != nullptr,
-                                      ctx->adj, st);
+                                      ctx->adj, ctx->ss, st);
     if (e == cudaErrorMemoryAllocation) return ctx->fail(SKID_ENOMEM);
     CK(e);
     if (nSel) CK(cudaMemcpyAsync(E, ctx->adj.E.p, nSel * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -30,6 +30,48 @@ __device__ __forceinline__ float d2of(float dx, float dy, float dz)
     return fadd(fadd(fmul(dx, dx), fmul(dy, dy)), fmul(dz, dz));
 }
 
+// Two floats in one 64-bit register pair, for sm_103a's packed FP32
+// instructions: each half rounds as the scalar instruction does, and one
+// issue slot covers both (the FP32 lanes take the same two cycles), so code
+// bound by instruction issue gains.
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a - b, exactly the scalar difference (the product b * -1 is exact)
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
+{
+    return fma2(b, 0xbf800000bf800000ull, a);
+}
+
 // Query-frame component: the query's periodic image nearest the candidate,
 // then fl(image - c).  Same rule as the oracle's img_dx.
 __device__ __forceinline__ float img_dx(float q, float c, float L, float h)

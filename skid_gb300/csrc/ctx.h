@@ -122,9 +122,12 @@ struct AdjointState {
     DBuf<int> nbr, ncnt;        // stored ball lists, `cap` per scatterer
     int cap = 0;
     bool lists = false;         // lists match the current density
-    DBuf<int2> items;           // potential work items (selection slot, tile)
-    DBuf<int> gsel;
-    DBuf<float> v;
+    DBuf<unsigned char> slots;  // selected groups of a potential call
+    DBuf<float4> rm;            // their members packed: relative position, mass
+    DBuf<float> re;             // softening
+    DBuf<int> rio;              // iOrder
+    DBuf<float4> tbox;          // boxes of their row tiles
+    DBuf<double> acc;           // their row sums
     DBuf<double> E;
 };
 cudaError_t density_adjoint(const Tree &t, const float *ball2_sorted, const int *sidx, const float *w_io,
@@ -132,7 +135,8 @@ cudaError_t density_adjoint(const Tree &t, const float *ball2_sorted, const int 
                             int *d_work, unsigned *d_status, cudaStream_t st);
 cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const float4 *vel4, int n,
                               float3 period, float Gc, int plummer, int nSel, const int *h_sel,
-                              const float *h_v, bool want_grad, AdjointState &A, cudaStream_t st);
+                              const float *h_v, bool want_grad, AdjointState &A, SortScratch &ss,
+                              cudaStream_t st);
 // unbind.cu
 cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *pos4,
                        const float4 *vel4, Tree &ut, const UnbindParams &P, int *grp,
@@ -423,7 +427,7 @@ struct skid_ctx {
         dfree(probe_f); dfree(probe_acc); dfree(probe_p4); dfree(probe_i); dfree(probe_i2);
         dfree(probe_t); dfree(stat_start); dfree(stat_out); dfree(tipsy_raw); dfree(knn_heap); dfree(split_acc); dfree(split_cnt); dfree(ms_dev);
         dfree(adj.win); dfree(adj.w); dfree(adj.g); dfree(adj.out); dfree(adj.nbr); dfree(adj.ncnt);
-        dfree(adj.items); dfree(adj.gsel); dfree(adj.v); dfree(adj.E);
+        dfree(adj.slots); dfree(adj.rm); dfree(adj.re); dfree(adj.rio); dfree(adj.tbox); dfree(adj.acc); dfree(adj.E);
         std::lock_guard<std::recursive_mutex> lk(skid::device_mutex());
         if (d_scal) cudaFree(d_scal);
         if (d_fbytes) cudaFree(d_fbytes);
