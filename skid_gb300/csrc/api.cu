@@ -254,6 +254,7 @@ FieldArgs skid_ctx::field_args(float fStep, bool initial, float *acc_out)
 {
     (void)initial;
     FieldArgs a;
+    a.zero = 0.0f;
     a.cpos = C.cpos.p;
     a.ccoef = C.ccoef.p;
     a.blo = ctree.blo.p;

@@ -66,6 +66,11 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+// x * x rounded, for sums that must not be fused: the assembler contracts
+// mul.rn.f32x2 followed by add.rn.f32x2 (measured: 40 % of random
+// d2of(x, y, z) differed), which it does not do to a fused multiply-add whose
+// addend it cannot see.  zero holds two +0 from a kernel argument.
+__device__ __forceinline__ f32x2 sq2(f32x2 x, f32x2 zero) { return fma2(x, x, zero); }
 // a - b, exactly the scalar difference (the product b * -1 is exact)
 __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
 {

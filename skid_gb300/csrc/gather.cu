@@ -33,7 +33,7 @@ constexpr int G_WARPS = 4;
 #define SKID_FIELD_UNROLL 4
 #endif
 #ifndef SKID_FIELD_MINB
-#define SKID_FIELD_MINB 12
+#define SKID_FIELD_MINB 9
 #endif
 constexpr int FIELD_UNROLL = SKID_FIELD_UNROLL;
 // Warps a split one-mover-per-warp step aims for (at most FIELD_SPLIT_CAP).
@@ -179,15 +179,30 @@ density_kernel(TreeView t, const float *__restrict__ ball2, float3 L, float3 hL,
 // of them (one cheap pass that sets a hit mask), then run the field terms for
 // their hits only, and are combined with a fixed xor-butterfly, so sums are
 // deterministic for a given G.
+//
+// Instruction issue bounds it at 32 movers per warp (85 % of the issue slots
+// at full activity of the 2^21 box), latency at few.  There (L = 1) the exact
+// tests run two candidates to a packed FP32 operation with the decision read
+// from a sign bit, and the prefilter is the exact test's own expression of the
+// gaps.  At every G the leaves under a node are walked from registers, the
+// next leaf's copies loaded while one is worked on, and the reciprocal root
+// is the flushing one behind a floor.  Field time of the 2^21 box per run 42.2
+// to 36.6 ms (a full-activity step 1.89 to 1.58 ms), the 150k mixed-species
+// run 10.75 to 9.3 ms, 5k particles 1.60 to 1.40 ms.  Nine blocks an SM (56
+// registers): 12 spill (41.5 ms), 10 took 40.1, 8 37.2.
 template <int G, bool STATS>
-__global__ void __launch_bounds__(G_WARPS * 32, G > 32 ? 10 : SKID_FIELD_MINB)
+__global__ void __launch_bounds__(G_WARPS * 32, G > 32 ? 8 : SKID_FIELD_MINB)
 field_kernel(FieldArgs a)
 {
     constexpr int MPL = G > 32 ? G / 32 : 1;   // movers per lane
     constexpr int L = G >= 32 ? 1 : 32 / G;    // lanes per mover
-    __shared__ float4 cpos_s[G_WARPS][SKID_LEAF];
+    // a leaf's survivors by component: x, y, z, -fBall2 (four at a time go
+    // into packed operands), and their (1/h^2, m/(pi h^5))
+    __shared__ __align__(16) float cand_s[G_WARPS][4][SKID_LEAF];
     __shared__ float2 ccoef_s[G_WARPS][SKID_LEAF];
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float (*cs)[SKID_LEAF] = cand_s[w];
+    float2 *cc = ccoef_s[w];
     const int nA = *a.d_nA;
     const int nC = *a.d_nC;
     // One mover per warp and few movers: each mover's walk is split over S
@@ -246,127 +261,215 @@ field_kernel(FieldArgs a)
         // so the last stride ends at the leaves: a visited node has each lane
         // test one of its 32 descendants five levels down against the movers'
         // box, and those that pass are visited in order (so leaves come in
-        // depth-first order).  A visited node is entered only if some mover
-        // lies in its ball box.  Stack level l (its first node and the
-        // descendants still to visit) is held by lane l.
+        // depth-first order).  A visited inner node is entered only if some
+        // mover lies in its ball box (with one mover per warp its box is the
+        // mover, and passing the test says so already).  Stack level l (its
+        // first node and the descendants still to visit) is held by lane l.
         auto reach = [&](int node) {
             float4 bl = a.blo[node], bh = a.bhi[node];
             return bl.x <= whi.x && bh.x >= wlo.x && bl.y <= whi.y && bh.y >= wlo.y &&
                    bl.z <= whi.z && bh.z >= wlo.z;
         };
+        // one of this lane's movers lies in the box
+        auto inside = [&](float4 blo, float4 bhi) {
+            bool in = false;
+#pragma unroll
+            for (int k = 0; k < MPL; ++k)
+                in = in || (valid[k] && y[k].x >= blo.x && y[k].x <= bhi.x && y[k].y >= blo.y &&
+                            y[k].y <= bhi.y && y[k].z >= blo.z && y[k].z <= bhi.z);
+            return in;
+        };
+        // the copy of this lane in a leaf (an empty ball past the end)
+        auto load_copy = [&](int lf) {
+            const int i = lf * SKID_LEAF + lane;
+            return i < nC ? a.cpos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        };
+        // One term of the field: the value (smooth1.c:450-458) only has to be
+        // accurate, not bit-exact: FMA and the approximate reciprocal square
+        // root (q = r2 / sqrt(r2), 1/q).  At r2 = 0 the floor under the root
+        // gives q = 0, and 1/q is not used.
+        auto add_term = [&](int k, int j) {
+            const float dx = cs[0][j] - y[k].x, dy = cs[1][j] - y[k].y, dz = cs[2][j] - y[k].z;
+            const float2 cf = cc[j];
+            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) * cf.x;
+            float iq;
+            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(iq) : "f"(fmaxf(r2, 1e-37f)));
+            const float q = r2 * iq;
+            float F = r2 < 1.0f ? __fmaf_rn(2.25f, q, -3.0f)
+                                : __fmaf_rn(-0.75f, q, 3.0f) - 3.0f * iq;
+            F *= cf.y;
+            ax[k] = __fmaf_rn(dx, F, ax[k]);
+            ay[k] = __fmaf_rn(dy, F, ay[k]);
+            az[k] = __fmaf_rn(dz, F, az[k]);
+        };
+        // A visited leaf: c4 is this lane's copy.
+        auto leaf_terms = [&](int lf, float4 c4) {
+            const int cb = lf * SKID_LEAF;
+            // with several movers per warp, a leaf box that overlaps theirs
+            // often holds none of them: this saves the leaf (box 37.8 to 36.6
+            // ms of field time); with few the copies are filtered right away
+            if (G >= 8) {
+                float4 blo = a.blo[a.leafBase + lf], bhi = a.bhi[a.leafBase + lf];
+                if (!__any_sync(SKID_FULL, inside(blo, bhi))) return;
+            }
+            if (STATS) ++st_leaves;
+            // prefilter: lane j keeps candidate j if its ball reaches the
+            // movers' box; the exact test below decides, so this only skips
+            // candidates that cannot hit (per-axis gaps to the box, zero
+            // inside).  An empty ball is rejected.
+            const float gx = fmaxf(fmaxf(wlo.x - c4.x, c4.x - whi.x), 0.0f);
+            const float gy = fmaxf(fmaxf(wlo.y - c4.y, c4.y - whi.y), 0.0f);
+            const float gz = fmaxf(fmaxf(wlo.z - c4.z, c4.z - whi.z), 0.0f);
+            bool rel;
+            if (L == 1) {
+                // float subtraction, product and sum are monotonic, so the
+                // exact test's d2 of a mover in the box is never below the
+                // same expression of the gaps
+                rel = d2of(gx, gy, gz) < c4.w;
+            } else {
+                // radius from the approximate reciprocal square root, widened
+                // to cover its error; which survivors there are decides the
+                // lane that sums each, so this form is kept to the last bit
+                float r = c4.w * rsqrtf(c4.w) * (1.0f + 4e-6f) +
+                          1e-6f * (fabsf(c4.x) + fabsf(c4.y) + fabsf(c4.z)) + 1e-30f;
+                rel = __fmaf_rn(gz, gz, __fmaf_rn(gy, gy, gx * gx)) <= r * r;
+            }
+            const unsigned R = __ballot_sync(SKID_FULL, rel);
+            if (R == 0) return;
+            const int nR = __popc(R);
+            const int rank = __popc(R & ((1u << lane) - 1u));
+            unsigned hitany = 0;
+            int slot_r;
+            if (L == 1) {
+                // Survivors go into slots in reverse order of rank, the rest
+                // as entries no mover is inside above them: with a hit's bit
+                // at its slot, the highest set bit is the first hit.
+                slot_r = rel ? nR - 1 - rank : nR + lane - rank;
+                __syncwarp();
+                cs[0][slot_r] = c4.x;
+                cs[1][slot_r] = c4.y;
+                cs[2][slot_r] = c4.z;
+                cs[3][slot_r] = rel ? -c4.w : INFINITY;
+                if (rel) {
+                    float4 co = a.ccoef[cb + lane];
+                    cc[slot_r] = make_float2(co.x, co.y);
+                }
+                __syncwarp();
+                if (STATS) st_tests += MPL * nR;
+#pragma unroll
+                for (int k = 0; k < MPL; ++k) {
+                    const f32x2 nyx = pack2(-y[k].x, -y[k].x), nyy = pack2(-y[k].y, -y[k].y),
+                                nyz = pack2(-y[k].z, -y[k].z);
+                    // smBallGather's test d2 < fBall2 (smooth1.c:365-369),
+                    // from the copy, two copies an operation: the sign of
+                    // d2 - fBall2 is shifted in
+                    const f32x2 zero = pack2(a.zero, a.zero);
+                    unsigned m = 0;
+                    for (int t = (nR - 1) & ~3; t >= 0; t -= 4) {
+                        const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&cs[0][t]);
+                        const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&cs[1][t]);
+                        const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(&cs[2][t]);
+                        const ulonglong2 W = *reinterpret_cast<const ulonglong2 *>(&cs[3][t]);
+                        f32x2 dx = add2(X.y, nyx), dy = add2(Y.y, nyy), dz = add2(Z.y, nyz);
+                        float2 d = unpack2(add2(add2(add2(sq2(dx, zero), sq2(dy, zero)), sq2(dz, zero)), W.y));
+                        m = __funnelshift_l(__float_as_uint(d.y), m, 1);
+                        m = __funnelshift_l(__float_as_uint(d.x), m, 1);
+                        dx = add2(X.x, nyx), dy = add2(Y.x, nyy), dz = add2(Z.x, nyz);
+                        d = unpack2(add2(add2(add2(sq2(dx, zero), sq2(dy, zero)), sq2(dz, zero)), W.x));
+                        m = __funnelshift_l(__float_as_uint(d.y), m, 1);
+                        m = __funnelshift_l(__float_as_uint(d.x), m, 1);
+                    }
+                    if (!valid[k]) m = 0;
+                    hitany |= m;
+                    if (STATS) st_hits += __popc(m);
+                    while (m) {
+                        const int j = 31 - __clz(m);
+                        m ^= 1u << j;
+                        add_term(k, j);
+                    }
+                }
+            } else {
+                slot_r = rank;
+                __syncwarp();
+                if (rel) {
+                    cs[0][rank] = c4.x;
+                    cs[1][rank] = c4.y;
+                    cs[2][rank] = c4.z;
+                    cs[3][rank] = -c4.w;
+                    float4 co = a.ccoef[cb + lane];
+                    cc[rank] = make_float2(co.x, co.y);
+                }
+                __syncwarp();
+                if (STATS) st_tests += (nR - sub + L - 1) / L;
+                // a mover's L lanes take every L-th survivor
+                unsigned m = 0;
+                if (valid[0]) {
+#pragma unroll FIELD_UNROLL
+                    for (int t = sub; t < nR; t += L) {
+                        float d2 = d2of(fsub(cs[0][t], y[0].x), fsub(cs[1][t], y[0].y),
+                                        fsub(cs[2][t], y[0].z));
+                        m |= (unsigned)(d2 < -cs[3][t]) << t;
+                    }
+                }
+                hitany = m;
+                if (STATS) st_hits += __popc(m);
+                for (; m; m &= m - 1) add_term(0, __ffs(m) - 1);
+            }
+            // copies that reached a mover: touched, and their density
+            // enters the floor of the cut (smooth1.c:460-461)
+            unsigned any = __reduce_or_sync(SKID_FULL, hitany);
+            if (rel && ((any >> slot_r) & 1u)) a.touched[cb + lane] = 1;
+        };
+        // The leaves that pass under one node, in order; the next one's
+        // copies are loaded while one is worked on.
+        auto visit_leaves = [&](int lf0, unsigned m) {
+            if (!m) return;
+            int lf = lf0 + __ffs(m) - 1;
+            float4 next = load_copy(lf);
+            for (;;) {
+                const float4 c4 = next;
+                const int cur = lf;
+                m &= m - 1;
+                if (m) {
+                    lf = lf0 + __ffs(m) - 1;
+                    next = load_copy(lf);
+                }
+                leaf_terms(cur, c4);
+                if (!m) break;
+            }
+        };
         unsigned smask;
         int sfirst;
+        const int d0 = a.logLeafBase % 5;
         {
-            const int d0 = a.logLeafBase % 5;
             sfirst = 1 << d0;
             smask = __ballot_sync(SKID_FULL, lane < (1 << d0) && reach(sfirst + lane));
         }
         int sp = 0;
+        if (sfirst == a.leafBase) {   // at most 16 leaves: they are the first level
+            visit_leaves(0, smask);
+            sp = -1;
+        }
         while (sp >= 0) {
             const unsigned m = __shfl_sync(SKID_FULL, smask, sp);
             if (!m) { --sp; continue; }
             const int node = __shfl_sync(SKID_FULL, sfirst, sp) + __ffs(m) - 1;
             if (lane == sp) smask = m & (m - 1);
             if (STATS) ++st_nodes;
-            {
+            if (G > 1) {
                 float4 blo = a.blo[node], bhi = a.bhi[node];
-                bool want = false;
-#pragma unroll
-                for (int k = 0; k < MPL; ++k)
-                    want = want || (valid[k] && y[k].x >= blo.x && y[k].x <= bhi.x &&
-                                    y[k].y >= blo.y && y[k].y <= bhi.y && y[k].z >= blo.z &&
-                                    y[k].z <= bhi.z);
-                if (!__any_sync(SKID_FULL, want)) continue;
-                if (node < a.leafBase) {
-                    const int cf = node << 5;
-                    unsigned cm = __ballot_sync(SKID_FULL, reach(cf + lane));
-                    if (G == 1 && S > 1 && cf >= a.leafBase)
-                        cm &= (S == 2 ? 0x55555555u : S == 4 ? 0x11111111u
-                               : S == 8 ? 0x01010101u : 0x00010001u) << part;
-                    if (cm) {
-                        ++sp;
-                        if (lane == sp) { smask = cm; sfirst = cf; }
-                    }
-                    continue;
-                }
-                int cb = (node - a.leafBase) * SKID_LEAF;
-                int cnt = min(SKID_LEAF, nC - cb);
-                if (STATS) ++st_leaves;
-                // prefilter: lane j keeps candidate j if its ball (radius
-                // rounded up) reaches the movers' box; the exact test below
-                // decides, so this only skips candidates that cannot hit
-                bool rel = false;
-                float4 c4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (lane < cnt) {
-                    c4 = a.cpos[cb + lane];
-                    // ball radius from the approximate reciprocal square root,
-                    // widened to cover its error (an empty ball, fBall2 = 0,
-                    // gives NaN and is rejected, as the exact test would)
-                    float r = c4.w * rsqrtf(c4.w) * (1.0f + 4e-6f) +
-                              1e-6f * (fabsf(c4.x) + fabsf(c4.y) + fabsf(c4.z)) + 1e-30f;
-                    // the ball itself against the box: squared distance from
-                    // the copy to the movers' box (per-axis gaps, zero inside)
-                    const float gx = fmaxf(fmaxf(wlo.x - c4.x, c4.x - whi.x), 0.0f);
-                    const float gy = fmaxf(fmaxf(wlo.y - c4.y, c4.y - whi.y), 0.0f);
-                    const float gz = fmaxf(fmaxf(wlo.z - c4.z, c4.z - whi.z), 0.0f);
-                    rel = __fmaf_rn(gz, gz, __fmaf_rn(gy, gy, gx * gx)) <= r * r;
-                }
-                // the survivors, compacted in candidate order
-                const unsigned R = __ballot_sync(SKID_FULL, rel);
-                const int nR = __popc(R);
-                const int slotR = __popc(R & ((1u << lane) - 1u));
-                __syncwarp();
-                if (rel) {
-                    cpos_s[w][slotR] = c4;
-                    float4 cc = a.ccoef[cb + lane];
-                    ccoef_s[w][slotR] = make_float2(cc.x, cc.y);
-                }
-                __syncwarp();
-                // a mover's L lanes take every L-th survivor
-                unsigned mask[MPL];
-#pragma unroll
-                for (int k = 0; k < MPL; ++k) mask[k] = 0;
-                if (want) {
-#pragma unroll FIELD_UNROLL
-                    for (int t = sub; t < nR; t += L) {
-                        float4 c = cpos_s[w][t];
-#pragma unroll
-                        for (int k = 0; k < MPL; ++k) {
-                            // smBallGather's test (smooth1.c:365-369), from the copy
-                            float d2 = d2of(fsub(c.x, y[k].x), fsub(c.y, y[k].y), fsub(c.z, y[k].z));
-                            mask[k] |= (unsigned)(d2 < c.w) << t;
-                        }
-                    }
-                    if (STATS) st_tests += MPL * ((nR - sub + L - 1) / L);
-                }
-                unsigned hitany = 0;
-#pragma unroll
-                for (int k = 0; k < MPL; ++k) {
-                    hitany |= mask[k];
-                    if (STATS) st_hits += __popc(mask[k]);
-                    for (unsigned m = mask[k]; m; m &= m - 1) {
-                        int j = __ffs(m) - 1;
-                        float4 c = cpos_s[w][j];
-                        float2 cf = ccoef_s[w][j];
-                        // the field value (smooth1.c:450-458) only has to be
-                        // accurate, not bit-exact: FMA and the approximate
-                        // reciprocal square root (q = r2 / sqrt(r2), 1/q)
-                        float dx = c.x - y[k].x, dy = c.y - y[k].y, dz = c.z - y[k].z;
-                        float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) * cf.x;
-                        float iq = rsqrtf(r2);
-                        float q = r2 > 0.0f ? r2 * iq : 0.0f;
-                        float F = r2 < 1.0f ? __fmaf_rn(2.25f, q, -3.0f)
-                                            : __fmaf_rn(-0.75f, q, 3.0f) - 3.0f * iq;
-                        F *= cf.y;
-                        ax[k] = __fmaf_rn(dx, F, ax[k]);
-                        ay[k] = __fmaf_rn(dy, F, ay[k]);
-                        az[k] = __fmaf_rn(dz, F, az[k]);
-                    }
-                }
-                // copies that reached a mover: touched, and their density
-                // enters the floor of the cut (smooth1.c:460-461)
-                unsigned any = __reduce_or_sync(SKID_FULL, hitany);
-                if (rel && ((any >> slotR) & 1u)) a.touched[cb + lane] = 1;
+                if (!__any_sync(SKID_FULL, inside(blo, bhi))) continue;
+            }
+            const int cf = node << 5;
+            unsigned cm = __ballot_sync(SKID_FULL, reach(cf + lane));
+            if (cf >= a.leafBase) {
+                if (G == 1 && S > 1)
+                    cm &= (S == 2 ? 0x55555555u : S == 4 ? 0x11111111u
+                           : S == 8 ? 0x01010101u : 0x00010001u) << part;
+                visit_leaves(cf - a.leafBase, cm);
+            } else if (cm) {
+                ++sp;
+                if (lane == sp) { smask = cm; sfirst = cf; }
             }
         }
 #pragma unroll
