@@ -52,9 +52,9 @@ constexpr int POT_TILE = 128;   // power of two
 // with an error bound, and only members within twice the bound of the
 // largest or smallest energy are evaluated exactly (the reference's FP64
 // expression rounded to float, kd.c:1396-1399), so the arg-max and arg-min,
-// ties included, are those of the reference's loop.  Groups up to this size
-// use the plain FP32 form with a per-member bound; larger ones the staged
-// a v + aH r form with one bound per pass (GB300's FP64 rate is a small
+// ties included, are those of the reference's loop.  Warps use the plain FP32
+// form with a per-member bound up to this size; blocks and larger groups the
+// staged a v + aH r form with one bound per pass (GB300's FP64 rate is a small
 // fraction of its FP32 rate, so FP64 is kept to the few candidates).
 constexpr int EXACT_E_MAX = 1024;
 
@@ -233,6 +233,9 @@ __device__ __forceinline__ float pair_dir(float d2, float twoh, int plummer)
     if (!plummer && ref_spline_ff(d2, twoh, v)) return v;
     return ref_dir_fp64(d2, twoh, plummer);
 }
+
+// The same, kept out of line where it is seldom reached.
+__device__ __noinline__ float pair_dir_call(float d2, float twoh) { return pair_dir(d2, twoh, 0); }
 
 __device__ __forceinline__ float wrap_h(float d, float h)
 {
@@ -666,7 +669,8 @@ struct RemoveArgs {
     const int *gstart, *gcount;
     int ng, nmax;
     float4 *qr, *qv;
-    float4 *qw;                     // large groups' staged a v + aH r (w: softening)
+    float4 *qa, *qw;                // block groups' member state beyond shared memory (BlockGroup)
+    int lcap;                       // members a block holds in shared memory
     int *qid;
     long long *pot;
     skid_group *rec;
@@ -781,7 +785,7 @@ __device__ __forceinline__ void write_record(const RemoveArgs &A, int g, int n, 
 
 // A small group, one warp: every lane keeps the FP64 centre itself (the same
 // values on every lane), lane 0 writes.
-__device__ void warp_group(const RemoveArgs &A, int g)
+__device__ __noinline__ void warp_group(const RemoveArgs &A, int g)
 {
     const int lane = threadIdx.x & 31;
     const int s = A.gstart[g], n0 = A.gcount[g];
@@ -933,6 +937,10 @@ __device__ void warp_group(const RemoveArgs &A, int g)
     __syncwarp();
 }
 
+// At most this many members near an extreme are evaluated exactly one warp
+// each; more bring every member's potential up to date.
+constexpr int CAND_MAX = 32;
+
 template <int BS>
 struct BlockShared {
     ArgRed smax[BS / 32], smin[BS / 32];
@@ -942,19 +950,21 @@ struct BlockShared {
     int s_n, s_go, s_have, s_imin, s_item;
     double d_cm[6], d_mass;
     double part[BS / 32][7];
-    float ext[BS / 32][4];      // per-warp FP32 energy max, min, error-bound terms
-    float s_w[3];               // a vcm + aH rcm (large groups' FP32 energies)
+    float ext[BS / 32][4];      // per-warp partials: FP32 energy max, min, error-bound terms
+    float s_w[3];               // a vcm + aH rcm (the members' FP32 energies)
     float s_mW;                 // max_j |a vcm_j| + |aH rcm_j|
     float s_mg;                 // max over members and axes of |a v_j| + |aH r_j|
     float gpart[8][4];          // a cluster's blocks' partials, gathered (rank order)
     ArgRed gmx[8], gmn[8];
-    int ccnt[BS / 32];          // per-warp arg-max candidate counts (two for a thread with two)
-    int cidx[BS / 32];          // the warp's first candidate
-    // records of each warp's first candidate (slot BS/32: the removed member
-    // when the decision needed the exact energies)
-    float4 cr[BS / 32 + 1], cv[BS / 32 + 1], cw[BS / 32 + 1];
-    long long cp[BS / 32 + 1];
-    int cid[BS / 32 + 1];
+    // block_group, by parity of the pass: per-warp largest and second largest
+    // energy, largest kinetic term (ordered bits), the largest's slot and state
+    unsigned wbest[2][BS / 32], wnext[2][BS / 32], wkin[2][BS / 32];
+    int wi[2][BS / 32];
+    float4 wa[2][BS / 32], wb[2][BS / 32];
+    float pub_w[2][3], pub_mW[2], pub_mass[2];   // W, its magnitude and the group's mass
+    int ncand;
+    ArgRed cand[CAND_MAX];
+    unsigned long long candq[CAND_MAX];
 };
 
 // max_j |a c_j| + |aH c_{j-3}| of a centre (rcm, vcm)
@@ -967,29 +977,223 @@ __device__ __forceinline__ float centre_mag(const RemoveArgs &A, const double *d
     return m * 1.0000002f;
 }
 
-// FP32 filter energy of a large group's member from its staged
-// w = a v + aH r: E = 1/2 |w - W|^2 - pot (1+z) 2^-S (dd and pe returned for
-// the pass's error bound), each operation rounded as written, so every
-// evaluation of a member gives the same value.
-__device__ __forceinline__ float staged_energy(float4 w, long long p, float wx, float wy, float wz,
-                                              float epot, float &dd, float &pe)
-{
-    const float dx = __fsub_rn(w.x, wx), dy = __fsub_rn(w.y, wy), dz = __fsub_rn(w.z, wz);
-    dd = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-    pe = __fmul_rn(ll2f_fast(p), epot);
-    return __fsub_rn(__fmul_rn(0.5f, dd), pe);
-}
-
 // A large group, the whole block.
+//
+// A group's removals are a serial chain -- one pass over its members per
+// removed member -- and the largest groups' chains set the time of the whole
+// unbinding, so a pass is made short:
+//  - Between the few exact decisions a member's potential is kept only as a
+//    compensated float that each removal changes by the hardware 1/r: about
+//    25 issue slots a member instead of about 170 for the reference's pair
+//    factor in fixed point, and no 64-bit arithmetic.  The exact potential of
+//    a member is its stored one less the terms of the members removed since
+//    (they lie behind the live ones, slots [n, nfl)); it is formed only for
+//    the members an exact decision needs, or for every member at once (flush)
+//    when those are many.
+//  - Members sit in shared memory (32 B each, the first A.lcap of them; the
+//    rest in global memory), two to a record so that a thread takes both in
+//    packed FP32 operations.
+//  - One barrier carries the warps' two largest energies, the largest's state
+//    and the largest kinetic term, from which every warp forms the same
+//    decision and the next centre to one float step; the block's last warp
+//    (the keeper) meanwhile brings the FP64 centre and the records in global
+//    memory up to date behind the pass that follows.
+// Removal at 2^21 (264 groups above 1024 members, the largest 10.7k, up to
+// 1008 removed from one) 10.4 ms with the exact terms every pass, members in
+// L2 and three barriers, now 4.6; 300 groups of up to 6.6k 2.2 to 0.73; 5k
+// particles 1.51 to 0.63.  A pass over 600 members takes 3300 cycles, over
+// 3700 3700, over 9000 (2300 of them in global memory) 11000.  What was
+// measured and left out: members in packed records in global memory too, the
+// next record loaded ahead, and velocities instead of w in the records (so
+// that the keeper reads none) were each no faster.
 template <int BS>
-__device__ void block_group(const RemoveArgs &A, int g, BlockShared<BS> &S)
+struct BlockGroup {
+    static constexpr int NW = BS / 32;
+    static constexpr int BC = BS - 32;   // threads that carry members
+    const RemoveArgs &A;
+    BlockShared<BS> &S;
+    float4 *qr, *qv;
+    int *qid;
+    long long *pot;
+    float *sm;                       // records in shared memory
+    float4 *ga, *gb;                 // state in global memory, by slot
+    int cap;                         // slots in shared memory
+    int tid, lane, w;
+    int n, nfl;                      // live members; slots below nfl have potentials as of then
+    float epot;
+    bool force;                      // exact potentials every pass
+
+    // Slot i (thread i % BC, its k-th member) lies in half k & 1 of record
+    // (k >> 1) BC + i % BC: x x' y y' | z z' p p' | u u' v v' | w w' c c', with
+    // p = -(potential energy), c its compensation, (u, v, w) = a v + aH r.  The
+    // four quarters of the records are arrays of their own, so that a warp's
+    // 16-byte accesses are contiguous.
+    static __device__ __forceinline__ int word(int i)
+    {
+        const int k = i / BC, t = i - k * BC;
+        return (((k >> 1) * BC + t) << 2) + (k & 1);
+    }
+    // (x, y, z, p) and (u, v, w, c) of a slot
+    __device__ __forceinline__ void get(int i, float4 &a, float4 &b) const
+    {
+        if (i < cap) {
+            const float *q = sm + word(i);
+            const int c2 = 2 * cap;
+            a = make_float4(q[0], q[2], q[c2], q[c2 + 2]);
+            b = make_float4(q[2 * c2], q[2 * c2 + 2], q[3 * c2], q[3 * c2 + 2]);
+        } else {
+            a = ga[i];
+            b = gb[i];
+        }
+    }
+    __device__ __forceinline__ void put(int i, float4 a, float4 b) const
+    {
+        if (i < cap) {
+            float *q = sm + word(i);
+            const int c2 = 2 * cap;
+            q[0] = a.x; q[2] = a.y; q[c2] = a.z; q[c2 + 2] = a.w;
+            q[2 * c2] = b.x; q[2 * c2 + 2] = b.y; q[3 * c2] = b.z; q[3 * c2 + 2] = b.w;
+        } else {
+            ga[i] = a;
+            gb[i] = b;
+        }
+    }
+
+    // FP32 filter energy E = 1/2 |w - W|^2 + p, each operation rounded as
+    // written (the packed form's too), so every evaluation of a member gives
+    // the same value.
+    static __device__ __forceinline__ float energy(float4 a, float4 b, float wx, float wy, float wz,
+                                                   float &dd)
+    {
+        const float dx = __fsub_rn(b.x, wx), dy = __fsub_rn(b.y, wy), dz = __fsub_rn(b.z, wz);
+        dd = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+        return __fmaf_rn(0.5f, dd, a.w);
+    }
+
+    // Exact fixed-point terms of the removed members in slots [from, nfl), a
+    // stride apart, on a member (kdSubPot, grav.c:44-59).
+    __device__ __forceinline__ long long pending(float4 r, float soft, int from, int stride) const
+    {
+        long long q = 0;
+        for (int e = from; e < nfl; e += stride) {
+            const float4 rs = qr[e];
+            const float d2 = d2of(fsub(rs.x, r.x), fsub(rs.y, r.y), fsub(rs.z, r.z));
+            q += fx(fmul(fmul(A.G, rs.w) * A.scale, pair_dir(d2, fadd(qv[e].w, soft), A.plummer)), 1.0f);
+        }
+        return q;
+    }
+
+    // The exact arg-max (or arg-min), first member on ties, among the members
+    // whose FP32 energy against (wx, wy, wz) reaches lim.  Called by the whole
+    // block, on a copy of the view (so that the caller's stays in registers),
+    // with the published FP64 centre current; *flushed says whether every
+    // member's potential is now exact.
+    template <bool MAX>
+    static __device__ __noinline__ ArgRed decide(BlockGroup B, float wx, float wy, float wz, float lim,
+                                                 bool *flushed)
+    {
+        return B.template decide_in<MAX>(wx, wy, wz, lim, flushed);
+    }
+
+    template <bool MAX>
+    __device__ __forceinline__ ArgRed decide_in(float wx, float wy, float wz, float lim, bool *flushed)
+    {
+        *flushed = false;
+        const double inv_d = 1.0 / (double)A.scale, opz_d = 1.0 + (double)A.z;
+        double dcm[6];
+        for (int d = 0; d < 6; ++d) dcm[d] = S.d_cm[d];
+        __syncthreads();
+        if (tid == 0) S.ncand = 0;
+        if (tid < CAND_MAX) S.candq[tid] = 0;
+        __syncthreads();
+        for (int i = tid; i < n; i += BS) {
+            float4 a, b;
+            float dd;
+            get(i, a, b);
+            const float E = energy(a, b, wx, wy, wz, dd);
+            if (MAX ? E >= lim : E <= lim) {
+                const int k = atomicAdd(&S.ncand, 1);
+                if (k < CAND_MAX) S.cand[k].i = i;
+            }
+        }
+        __syncthreads();
+        const int nc = S.ncand;
+        ArgRed best{MAX ? -FLT_MAX : FLT_MAX, 0x7fffffff};
+        auto better = [&](ArgRed x) {
+            return MAX ? x.v > best.v || (x.v == best.v && x.i < best.i)
+                       : x.v < best.v || (x.v == best.v && x.i < best.i);
+        };
+        if (nc <= CAND_MAX && !force) {
+            if (A.subpot && nfl > n) {
+                for (int k = 0; k < nc; ++k) {
+                    const int i = S.cand[k].i;
+                    long long q = pending(qr[i], qv[i].w, n + tid, BS);
+#pragma unroll
+                    for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(SKID_FULL, q, o);
+                    if (lane == 0 && q) atomicAdd(&S.candq[k], (unsigned long long)q);
+                }
+                __syncthreads();
+            }
+            if (tid < nc) {
+                const int i = S.cand[tid].i;
+                S.cand[tid].v =
+                    exact_energy(A, qr[i], qv[i], pot[i] - (long long)S.candq[tid], dcm, inv_d, opz_d);
+            }
+            __syncthreads();
+            for (int k = 0; k < nc; ++k)
+                if (better(S.cand[k])) best = S.cand[k];
+            __syncthreads();
+            return best;
+        }
+        for (int i = tid; i < n; i += BS) {
+            float4 a, b;
+            float dd;
+            get(i, a, b);
+            const float E = energy(a, b, wx, wy, wz, dd);
+            const float4 r = qr[i], v = qv[i];
+            const long long p = pot[i] - (A.subpot ? pending(r, v.w, n, 1) : 0);
+            pot[i] = p;
+            a.w = -(ll2f_approx(p) * epot);
+            b.w = 0.0f;
+            put(i, a, b);
+            if (force || (MAX ? E >= lim : E <= lim)) {
+                const ArgRed x{exact_energy(A, r, v, p, dcm, inv_d, opz_d), i};
+                if (better(x)) best = x;
+            }
+        }
+        *flushed = true;
+        best = MAX ? warp_argmax(best) : warp_argmin(best);
+        if (lane == 0) S.smax[w] = best;
+        __syncthreads();
+        best = S.smax[0];
+        for (int k = 1; k < NW; ++k)
+            if (better(S.smax[k])) best = S.smax[k];
+        __syncthreads();
+        return best;
+    }
+};
+
+template <int BS>
+__device__ void block_group(const RemoveArgs &A, int g, BlockShared<BS> &S, float4 *dyn)
 {
+    using BG = BlockGroup<BS>;
+    constexpr int NW = BG::NW, BC = BG::BC;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const bool keeper = w == NW - 1;
     const int s = A.gstart[g], n0 = A.gcount[g];
-    float4 *qr = A.qr + s;
-    float4 *qv = A.qv + s;
+    float4 *qr = A.qr + s, *qv = A.qv + s;
     int *qid = A.qid + s;
     long long *pot = A.pot + s;
+    // slots in shared memory: whole records of a row of BC threads
+    const int cap = A.lcap / (2 * BC) * (2 * BC);
+    float *sm = reinterpret_cast<float *>(dyn);
+    float4 *ga = A.qa + s, *gb = A.qw + s;
+    int n = n0, nfl = n0;
+    bool force = false;
+    const float epot = A.inv_scale * A.opz;
+    auto view = [&]() {
+        return BG{A, S, qr, qv, qid, pot, sm, ga, gb, cap, tid, lane, w, n, nfl, epot, force};
+    };
     double m = 0.0, c[6] = {0, 0, 0, 0, 0, 0};
     for (int i = tid; i < n0; i += BS) {
         float4 r = qr[i], v = qv[i];
@@ -1007,349 +1211,382 @@ __device__ void block_group(const RemoveArgs &A, int g, BlockShared<BS> &S)
         S.part[w][0] = m;
         for (int d = 0; d < 6; ++d) S.part[w][1 + d] = c[d];
     }
-    __syncthreads();
-    if (tid == 0) {
-        // warp partials in warp order: the same sums on every run
-        double t[7] = {0, 0, 0, 0, 0, 0, 0};
-        for (int k = 0; k < BS / 32; ++k)
-            for (int d = 0; d < 7; ++d) t[d] += S.part[k][d];
-        S.d_mass = t[0];
-        for (int d = 0; d < 6; ++d) {
-            S.d_cm[d] = t[1 + d] / t[0];
-            S.s_cm[d] = (float)S.d_cm[d];
-        }
-        S.s_n = n0;
-        S.s_have = 0;
-        S.s_go = 1;
-        S.s_imin = 0;
-        for (int d = 0; d < 3; ++d)
-            S.s_w[d] = (float)((double)A.fShift * S.d_cm[3 + d] + (double)A.fCosmo * S.d_cm[d]);
-    }
-    __syncthreads();
-    int nrem = 0;
-    const bool exact = n0 <= EXACT_E_MAX;
-    const double opz_d = 1.0 + (double)A.z, inv_d = 1.0 / (double)A.scale;
-    float4 *qw = A.qw + s;
-    if (!exact) {
-        // FP32 filter energies E_i = 1/2 |w_i - W|^2 - pot_i (1+z), with
-        // w_i = a v_i + aH r_i fixed per member and W = a vcm + aH rcm per
-        // pass; their error bound needs the largest |a v_j| + |aH r_j|
-        float mg = 0.0f;
+    // Every member's state: FP32 filter energies E_i = 1/2 |w_i - W|^2 + p_i,
+    // with w_i = a v_i + aH r_i fixed per member and W = a vcm + aH rcm per
+    // pass; their error bound needs the largest |a v_j| + |aH r_j| and the
+    // largest |p|.
+    float mg = 0.0f, gpe = 0.0f;
+    float emax = -FLT_MAX, emin = FLT_MAX, mmax = -FLT_MAX, mmin = FLT_MAX;
+    bool odd = !(A.G >= 0.0f) || !(A.opz >= 0.0f);
+    {
+        const BG B = view();
         for (int i = tid; i < n0; i += BS) {
-            float4 r = qr[i], v = qv[i];
-            qw[i] = make_float4(__fmaf_rn(A.fShift, v.x, A.fCosmo * r.x),
-                                __fmaf_rn(A.fShift, v.y, A.fCosmo * r.y),
-                                __fmaf_rn(A.fShift, v.z, A.fCosmo * r.z), v.w);
+            const float4 r = qr[i], v = qv[i];
+            const float p = -(ll2f_approx(pot[i]) * epot);
+            B.put(i, make_float4(r.x, r.y, r.z, p),
+                  make_float4(__fmaf_rn(A.fShift, v.x, A.fCosmo * r.x),
+                              __fmaf_rn(A.fShift, v.y, A.fCosmo * r.y),
+                              __fmaf_rn(A.fShift, v.z, A.fCosmo * r.z), 0.0f));
             mg = fmaxf(mg, fabsf(A.fShift * v.x) + fabsf(A.fCosmo * r.x));
             mg = fmaxf(mg, fabsf(A.fShift * v.y) + fabsf(A.fCosmo * r.y));
             mg = fmaxf(mg, fabsf(A.fShift * v.z) + fabsf(A.fCosmo * r.z));
+            gpe = fmaxf(gpe, fabsf(p));
+            emax = fmaxf(emax, v.w);
+            emin = fminf(emin, v.w);
+            mmax = fmaxf(mmax, r.w);
+            mmin = fminf(mmin, r.w);
+            // the bound takes every removed term as part of the first
+            // potential, which a negative mass, G or softening would break
+            odd = odd || !(r.w >= 0.0f) || !(v.w >= 0.0f);
         }
-        mg = __uint_as_float(__reduce_max_sync(SKID_FULL, __float_as_uint(mg)));
-        if (lane == 0) S.ext[w][0] = mg;
-        __syncthreads();
-        if (tid == 0) {
-            float t = 0.0f;
-            for (int k = 0; k < BS / 32; ++k) t = fmaxf(t, S.ext[k][0]);
-            S.s_mg = t * 1.0000002f;
-            S.s_mW = centre_mag(A, S.d_cm);
-        }
-        __syncthreads();
     }
-    const float epot = A.inv_scale * A.opz;
+    mg = __uint_as_float(__reduce_max_sync(SKID_FULL, __float_as_uint(mg)));
+    gpe = __uint_as_float(__reduce_max_sync(SKID_FULL, __float_as_uint(gpe)));
+    emax = ord2f(__reduce_max_sync(SKID_FULL, f2ord(emax)));
+    emin = ord2f(__reduce_min_sync(SKID_FULL, f2ord(emin)));
+    mmax = ord2f(__reduce_max_sync(SKID_FULL, f2ord(mmax)));
+    mmin = ord2f(__reduce_min_sync(SKID_FULL, f2ord(mmin)));
+    odd = __any_sync(SKID_FULL, odd);
+    if (lane == 0) {
+        S.wa[0][w] = make_float4(mg, gpe, emax, emin);
+        S.wb[0][w] = make_float4(mmax, mmin, 0.0f, 0.0f);
+        S.wi[0][w] = odd;
+    }
+    __syncthreads();
+    for (int k = 0; k < NW; ++k) {
+        const float4 x = S.wa[0][k], y = S.wb[0][k];
+        mg = fmaxf(mg, x.x);
+        gpe = fmaxf(gpe, x.y);
+        emax = fmaxf(emax, x.z);
+        emin = fminf(emin, x.w);
+        mmax = fmaxf(mmax, y.x);
+        mmin = fminf(mmin, y.y);
+        force = force || S.wi[0][k];
+    }
+    mg *= 1.0000002f;
+    // one mass and one softening: a pass reads no record from global memory
+    const bool uniform = mmin == mmax && emin == emax;
+    if (tid == 0) {
+        // warp partials in warp order: the same sums on every run
+        double t[7] = {0, 0, 0, 0, 0, 0, 0};
+        for (int k = 0; k < NW; ++k)
+            for (int d = 0; d < 7; ++d) t[d] += S.part[k][d];
+        S.d_mass = t[0];
+        for (int d = 0; d < 6; ++d) S.d_cm[d] = t[1 + d] / t[0];
+        for (int d = 0; d < 3; ++d)
+            S.pub_w[0][d] = (float)((double)A.fShift * S.d_cm[3 + d] + (double)A.fCosmo * S.d_cm[d]);
+        S.pub_mW[0] = centre_mag(A, S.d_cm);
+        S.pub_mass[0] = (float)t[0];
+        S.s_imin = 0;
+    }
+    __syncthreads();
+    int nrem = 0, par = 0;           // the same on every thread
+    int ib = 0;                      // the last removed member's slot, and its state
+    float4 ra = make_float4(0.0f, 0.0f, 0.0f, 0.0f), rb = ra;
+    float gms = 0.0f, es = 0.0f;     // its G m (1+z) and softening
+    float f = 0.0f;                  // its m / (mass left)
+    float wx = S.pub_w[0][0], wy = S.pub_w[0][1], wz = S.pub_w[0][2];
+    // The keeper: FP64 centre (kd.c:1424-1431, a lane per component) and, with
+    // uniform members, the records' swap with the last member (kd.c:1435-1440)
+    // for the member removed last; n is the slot it goes to.
+    auto keep = [&]() {
+        const float4 r = qr[ib], v = qv[ib];
+        const int qb = qid[ib];
+        const float4 rl = qr[n], vl = qv[n];
+        const int ql = qid[n];
+        const long long pl = pot[n];
+        // a known mass lets the division run while the records arrive
+        const double dm = (double)(uniform ? mmax : r.w);
+        const double mm = __dsub_rn(S.d_mass, dm);
+        const double fd = __ddiv_rn(dm, mm);
+        const int d = lane < 6 ? lane : 0;
+        const double x =
+            (double)(d == 0 ? r.x : d == 1 ? r.y : d == 2 ? r.z : d == 3 ? v.x : d == 4 ? v.y : v.z);
+        const double o = S.d_cm[d];
+        const double cn = __dadd_rn(o, __dmul_rn(fd, __dsub_rn(o, x)));
+        const double vd = __shfl_sync(SKID_FULL, cn, (d % 3) + 3);
+        const double rd = __shfl_sync(SKID_FULL, cn, d % 3);
+        const float W = (float)((double)A.fShift * vd + (double)A.fCosmo * rd);
+        const float mag = (fabsf(A.fShift * (float)vd) + fabsf(A.fCosmo * (float)rd)) * 1.0000002f;
+        const float mW = __uint_as_float(__reduce_max_sync(SKID_FULL, __float_as_uint(mag)));
+        __syncwarp();
+        if (lane < 6) S.d_cm[lane] = cn;
+        if (lane < 3) S.pub_w[par][lane] = W;
+        if (lane == 0) {
+            S.d_mass = mm;
+            S.pub_mass[par] = (float)mm;
+            S.pub_mW[par] = mW;
+            if (uniform) {
+                A.grp[qb] = 0;
+                qr[ib] = rl; qv[ib] = vl; qid[ib] = ql; pot[ib] = pl;
+                qr[n] = r; qv[n] = v; qid[n] = qb;
+            }
+        }
+    };
     for (;;) {
-        const int n = S.s_n;
-        const bool have = S.s_have != 0;
-        const float4 rs = S.s_r;
-        const float es = S.s_eps;
-        double dcm[6];
-        float scm[6];
-        for (int d = 0; d < 6; ++d) { dcm[d] = S.d_cm[d]; scm[d] = S.s_cm[d]; }
-        const float wx = S.s_w[0], wy = S.s_w[1], wz = S.s_w[2];
-        // the thread's two largest and two smallest FP32 energies (first
-        // index first on ties), the block's extremes, and the pass's bound
-        // on |FP32 energy - reference energy| (bnd)
-        ArgRed mx{-FLT_MAX, 0x7fffffff}, mn{FLT_MAX, 0x7fffffff};
-        ArgRed x2 = mx, n2 = mn;
-        float gmax = -FLT_MAX, gmin = FLT_MAX, bnd = 0.0f;
-        // The lane holding its warp's largest FP32 energy (the only lane of
-        // the warp that can hold the member removed in the usual pass)
-        // prefetches that member's records into L1 while the block meets at
-        // the barrier.
-        auto prefetch_top = [&](float wmax) {
-            if (mx.v == wmax && mx.i < n) {
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(qr + mx.i));
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(qv + mx.i));
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(pot + mx.i));
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(qid + mx.i));
-                if (!exact) asm volatile("prefetch.global.L1 [%0];" ::"l"(qw + mx.i));
-            }
-        };
-        if (exact) {
-            float dmax = 0.0f;
-            for (int i = tid; i < n; i += BS) {
-                float4 r = qr[i], v = qv[i];
-                long long p = pot[i];
-                if (have && A.subpot) {
-                    p = sub_pot(A, rs, es, r, v, p);
-                    pot[i] = p;
-                }
-                float E = member_energy(false, A, r, v, p, dcm, scm, inv_d, opz_d);
-                keep_top2(mx, x2, E, i);
-                keep_bot2(mn, n2, E, i);
-                dmax = fmaxf(dmax, energy_err(A, r, v, p, scm, E));
-            }
-            float a0 = mx.v, a1 = mn.v;
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                a0 = fmaxf(a0, __shfl_xor_sync(SKID_FULL, a0, o));
-                a1 = fminf(a1, __shfl_xor_sync(SKID_FULL, a1, o));
-                dmax = fmaxf(dmax, __shfl_xor_sync(SKID_FULL, dmax, o));
-            }
-            prefetch_top(a0);
-            if (lane == 0) {
-                S.ext[w][0] = a0;
-                S.ext[w][1] = a1;
-                S.ext[w][2] = dmax;
-            }
+        const bool sub = nrem > 0 && A.subpot;
+        // after a member that held much of the mass the float step is not
+        // good enough: the pass waits for the FP64 centre
+        const bool late = f <= 0.25f;
+        if (!late) {
+            if (keeper) keep();
             __syncthreads();
-            for (int k = 0; k < BS / 32; ++k) {
-                gmax = fmaxf(gmax, S.ext[k][0]);
-                gmin = fminf(gmin, S.ext[k][1]);
-                bnd = fmaxf(bnd, S.ext[k][2]);
-            }
-        } else {
-            const float gms = fmul(A.G, rs.w) * A.scale;   // the removed member's G m 2^S
-            const bool sub = have && A.subpot;
-            float ddmx = 0.0f, pemx = 0.0f;
-            // RB members per thread per batch, all loaded before any is used,
-            // so their memory latencies overlap
-            constexpr int RB = BS >= 1024 ? 2 : 4;
-            for (int i0 = tid; i0 < n; i0 += RB * BS) {
-                float4 r[RB], wv[RB];
-                long long p[RB];
-#pragma unroll
-                for (int k = 0; k < RB; ++k) {
-                    const int i = i0 + k * BS;
-                    if (i < n) { r[k] = qr[i]; wv[k] = qw[i]; p[k] = pot[i]; }
+            wx = S.pub_w[par][0];
+            wy = S.pub_w[par][1];
+            wz = S.pub_w[par][2];
+            f = 0.0f;
+        }
+        // beyond far every member's pair with the removed one is 1/r
+        const float far = A.plummer ? INFINITY : fmaxf((es + emax) * (es + emax) * 1.000001f, 1e-30f);
+        float m1 = -FLT_MAX, m2 = -FLT_MAX, ddmx = 0.0f;
+        int i1 = 0x7fffffff;
+        if (!keeper) {
+            // the pair factor of the removed member for one nearer than far
+            auto near_dir = [&](float dx, float dy, float dz, int i) {
+                const float e = uniform ? emax : qv[i].w;
+                if (A.plummer) {
+                    const float t = es + e;
+                    return rsqrtf(__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx)) + 0.25f * t * t);
                 }
-#pragma unroll
-                for (int k = 0; k < RB; ++k) {
-                    const int i = i0 + k * BS;
-                    if (i >= n) break;
+                return pair_dir_call(d2of(dx, dy, dz), fadd(es, e));
+            };
+            auto track = [&](float E, float dd, int i) {
+                m2 = fmaxf(m2, fminf(m1, E));
+                if (E > m1) i1 = i;
+                m1 = fmaxf(m1, E);
+                ddmx = fmaxf(ddmx, dd);
+            };
+            auto single = [&](int i, float4 &a, float4 &b) {
+                if (sub) {
+                    const float dx = a.x - ra.x, dy = a.y - ra.y, dz = a.z - ra.z;
+                    const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
+                    float dir;
+                    if (d2 >= far) asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(dir) : "f"(d2));
+                    else dir = near_dir(dx, dy, dz, i);
+                    const float y = __fmaf_rn(gms, dir, b.w), t = __fadd_rn(a.w, y);
+                    b.w = __fsub_rn(y, __fsub_rn(t, a.w));
+                    a.w = t;
+                }
+                float dd;
+                const float E = BG::energy(a, b, wx, wy, wz, dd);
+                track(E, dd, i);
+            };
+            const int ns = min(n, cap);
+            int i = tid;
+            {
+                const f32x2 nrx = pack2(-ra.x, -ra.x), nry = pack2(-ra.y, -ra.y), nrz = pack2(-ra.z, -ra.z);
+                const f32x2 nwx = pack2(-wx, -wx), nwy = pack2(-wy, -wy), nwz = pack2(-wz, -wz);
+                const f32x2 gm2 = pack2(gms, gms), half2 = pack2(0.5f, 0.5f);
+                ulonglong2 *q0 = reinterpret_cast<ulonglong2 *>(sm) + tid;
+                const int h = cap >> 1;
+                ulonglong2 *q1 = q0 + h, *q2 = q1 + h, *q3 = q2 + h;
+#pragma unroll 2
+                for (; i + BC < ns; i += 2 * BC, q0 += BC, q1 += BC, q2 += BC, q3 += BC) {
+                    const ulonglong2 r0 = *q0, r1 = *q1, r2 = *q2, r3 = *q3;
+                    f32x2 P = r1.y;
                     if (sub) {
-                        // kdSubPot (grav.c:44-59): the term the potentials added
-                        float d2 = d2of(fsub(rs.x, r[k].x), fsub(rs.y, r[k].y), fsub(rs.z, r[k].z));
-                        p[k] -= fx(fmul(gms, pair_dir(d2, fadd(es, wv[k].w), A.plummer)), 1.0f);
-                        pot[i] = p[k];
+                        const f32x2 dx = add2(r0.x, nrx), dy = add2(r0.y, nry), dz = add2(r1.x, nrz);
+                        const float2 d2 = unpack2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))));
+                        float2 dir;
+                        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(dir.x) : "f"(d2.x));
+                        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(dir.y) : "f"(d2.y));
+                        if (!(fminf(d2.x, d2.y) >= far)) {
+                            const float2 X = unpack2(dx), Y = unpack2(dy), Z = unpack2(dz);
+                            if (!(d2.x >= far)) dir.x = near_dir(X.x, Y.x, Z.x, i);
+                            if (!(d2.y >= far)) dir.y = near_dir(X.y, Y.y, Z.y, i + BC);
+                        }
+                        // p + G m (1+z) dir, compensated
+                        const f32x2 y = fma2(gm2, pack2(dir.x, dir.y), r3.y);
+                        const f32x2 t = add2(P, y);
+                        q3->y = sub2(y, sub2(t, P));
+                        q1->y = t;
+                        P = t;
                     }
-                    float dd, pe;
-                    const float E = staged_energy(wv[k], p[k], wx, wy, wz, epot, dd, pe);
-                    keep_top2(mx, x2, E, i);
-                    keep_bot2(mn, n2, E, i);
-                    ddmx = fmaxf(ddmx, dd);
-                    pemx = fmaxf(pemx, fabsf(pe));
+                    const f32x2 ux = add2(r2.x, nwx), uy = add2(r2.y, nwy), uz = add2(r3.x, nwz);
+                    const f32x2 dd2 = fma2(uz, uz, fma2(uy, uy, mul2(ux, ux)));
+                    const float2 E = unpack2(fma2(half2, dd2, P)), dd = unpack2(dd2);
+                    track(E.x, dd.x, i);
+                    track(E.y, dd.y, i + BC);
                 }
             }
-            // Bound on |E_i(FP32) - E_i(reference)|: with C = max |a v| +
-            // |aH r| over members plus the same for the centre, each
-            // component of w_i - W is within 2^-21 C of the reference's dv,
-            // so 2^-19 (C (sqrt(3 dd) + 3 C) + 1.5 dd + 2 |pe|) over the
-            // pass's largest dd and |pe| covers every member, several times
-            // over.
-            float a0 = mx.v, a1 = mn.v;
+            const BG B = view();
+            if (i < ns) {
+                float4 a, b;
+                B.get(i, a, b);
+                single(i, a, b);
+                if (sub) B.put(i, a, b);
+                i += BC;
+            }
+            // a thread's first slot past the shared ones has its own column
+            if (i < cap) i += (cap - i + BC - 1) / BC * BC;
+            constexpr int RG = 4;    // loads in flight
+            for (; i < n; i += RG * BC) {
+                float4 a[RG], b[RG];
 #pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                a0 = fmaxf(a0, __shfl_xor_sync(SKID_FULL, a0, o));
-                a1 = fminf(a1, __shfl_xor_sync(SKID_FULL, a1, o));
-                ddmx = fmaxf(ddmx, __shfl_xor_sync(SKID_FULL, ddmx, o));
-                pemx = fmaxf(pemx, __shfl_xor_sync(SKID_FULL, pemx, o));
-            }
-            prefetch_top(a0);
-            if (lane == 0) {
-                S.ext[w][0] = a0;
-                S.ext[w][1] = a1;
-                S.ext[w][2] = ddmx;
-                S.ext[w][3] = pemx;
-            }
-            __syncthreads();
-            float gdd = 0.0f, gpe = 0.0f;
-            for (int k = 0; k < BS / 32; ++k) {
-                gmax = fmaxf(gmax, S.ext[k][0]);
-                gmin = fminf(gmin, S.ext[k][1]);
-                gdd = fmaxf(gdd, S.ext[k][2]);
-                gpe = fmaxf(gpe, S.ext[k][3]);
-            }
-            const float C = S.s_mg + S.s_mW;
-            bnd = 1.9073486e-06f * (C * (1.7320509f * sqrtf(gdd) + 3.0f * C) + 1.5f * gdd + 2.0f * gpe) +
-                  1e-30f;
-        }
-        // Only members within twice the bound of the extremes can be the
-        // exact arg-max or arg-min.
-        const float hi = gmax - 2.0f * bnd, lo = gmin + 2.0f * bnd;
-        const ArgRed t1 = mx, b1 = mn;
-        // the last member's records, final for this pass now (their owners
-        // wrote the potentials before the barrier), for the swap
-        float4 lr = make_float4(0.0f, 0.0f, 0.0f, 0.0f), lv = lr, lw = lr;
-        long long lp = 0;
-        int lq = 0;
-        if (tid == 32 && n > 1) {
-            lr = qr[n - 1];
-            lv = qv[n - 1];
-            lp = pot[n - 1];
-            lq = qid[n - 1];
-            if (!exact) lw = qw[n - 1];
-        }
-        // members again, in the same order with the same FP32 energies: the
-        // candidates on the asked side exactly (FP64, as the reference)
-        auto rescan = [&](bool scan_hi, bool scan_lo) {
-            for (int i = tid; i < n; i += BS) {
-                float E;
-                if (exact) {
-                    E = member_energy(false, A, qr[i], qv[i], pot[i], dcm, scm, inv_d, opz_d);
-                } else {
-                    float dd, pe;
-                    E = staged_energy(qw[i], pot[i], wx, wy, wz, epot, dd, pe);
-                }
-                const bool ch = scan_hi && E >= hi, cl = scan_lo && E <= lo;
-                if (ch || cl) {
-                    const float X = exact_energy(A, qr[i], qv[i], pot[i], dcm, inv_d, opz_d);
-                    if (ch && X > mx.v) { mx.v = X; mx.i = i; }
-                    if (cl && X < mn.v) { mn.v = X; mn.i = i; }
+                for (int k = 0; k < RG; ++k)
+                    if (i + k * BC < n) { a[k] = ga[i + k * BC]; b[k] = gb[i + k * BC]; }
+#pragma unroll
+                for (int k = 0; k < RG; ++k) {
+                    if (i + k * BC >= n) break;
+                    single(i + k * BC, a[k], b[k]);
+                    if (sub) { ga[i + k * BC].w = a[k].w; gb[i + k * BC].w = b[k].w; }
                 }
             }
-        };
-        // The arg-max.  One candidate alone is the exact arg-max (every other
-        // member's exact energy is below gmax - bnd, its own at least that),
-        // and the sign of its exact energy is known when gmax >= bnd or
-        // gmax < -bnd: the usual pass evaluates no FP64 energy.  The warps'
-        // candidate counts ride on the barrier the block needs anyway (a
-        // thread with two candidates counts as two).
-        {
-            const unsigned bal = __ballot_sync(SKID_FULL, t1.v >= hi);
-            const int first = __shfl_sync(SKID_FULL, t1.i, bal ? __ffs(bal) - 1 : 0);
-            const bool two = __any_sync(SKID_FULL, x2.v >= hi);
-            if (lane == 0) {
-                S.ccnt[w] = __popc(bal) + (two ? 2 : 0);
-                S.cidx[w] = first;
+            // the warp's largest energy and its member, and its second largest
+            const unsigned u = f2ord(m1), best = __reduce_max_sync(SKID_FULL, u);
+            const int fl = __ffs(__ballot_sync(SKID_FULL, u == best)) - 1;
+            const unsigned next = __reduce_max_sync(SKID_FULL, lane == fl ? f2ord(m2) : u);
+            const unsigned kin = __reduce_max_sync(SKID_FULL, __float_as_uint(ddmx));
+            if (lane == fl) {
+                S.wbest[par][w] = best;
+                S.wnext[par][w] = next;
+                S.wkin[par][w] = kin;
+                S.wi[par][w] = i1;
+                if (i1 < n) {
+                    float4 a, b;
+                    B.get(i1, a, b);
+                    S.wa[par][w] = a;
+                    S.wb[par][w] = b;
+                }
             }
-            if (bal && lane == __ffs(bal) - 1) {
-                S.cr[w] = qr[t1.i];
-                S.cv[w] = qv[t1.i];
-                S.cw[w] = exact ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : qw[t1.i];
-                S.cp[w] = pot[t1.i];
-                S.cid[w] = qid[t1.i];
-            }
+        } else if (nrem > 0 && late) {
+            keep();
         }
         __syncthreads();
-        int ccnt = 0, cidx = 0, kw = 0;
-        for (int k = 0; k < BS / 32; ++k) {
-            const int c = S.ccnt[k];
-            if (c && !ccnt) {
-                cidx = S.cidx[k];
-                kw = k;
-            }
-            ccnt += c;
+        // Published for every removal so far.
+        const float pwx = S.pub_w[par][0], pwy = S.pub_w[par][1], pwz = S.pub_w[par][2];
+        const float mW = S.pub_mW[par], mass = S.pub_mass[par];
+        float gmax, gnext, gdd;
+        int kw;
+        {
+            const bool in = lane < NW - 1;
+            const unsigned u = in ? S.wbest[par][lane] : 0u;
+            const unsigned best = __reduce_max_sync(SKID_FULL, u);
+            kw = __ffs(__ballot_sync(SKID_FULL, in && u == best)) - 1;
+            const unsigned x = in ? S.wnext[par][lane] : 0u;
+            const unsigned next = __reduce_max_sync(SKID_FULL, lane == kw ? x : u);
+            gdd = __uint_as_float(__reduce_max_sync(SKID_FULL, in ? S.wkin[par][lane] : 0u));
+            gmax = ord2f(best);
+            gnext = ord2f(next);
         }
+        // Bound on |E_i(FP32) - E_i(reference)|.  With C at or above every
+        // |a v_j| + |aH r_j| of a member plus the centre's: w_i - W is within
+        // 2^-23 C + 2^-23 |dv| of the reference's dv in each component (w_i's
+        // two roundings 2^-23 of a member's magnitude; W, one float step from
+        // the published rounding of the FP64 centre, 2^-23 of the centre's and
+        // 2^-22 f C; the subtraction's and the reference's own rounding 2^-24
+        // |dv| each), so 1/2 |dv|^2 is within 2^-23 (1.7321 C sqrt(dd) +
+        // 3.25 dd) (both sides' sums of squares 3 x 2^-24 x dd / 2 included).
+        // p starts within 2^-22 of the potential's energy; a removed term is
+        // within 10 x 2^-24 of the exact one (hardware root 2^-22.9, squared
+        // distance 2.8, products 2, the exact term's two float roundings 2,
+        // the sum's 1) besides its rounding to the fixed-point quantum, and
+        // together the terms are no more than the first potential; the
+        // compensated sum adds 2 x 2^-24: in all 2^-20 of the group's largest.
+        // Both energies' last rounding: 2^-24 (dd + 2 |p|).  Twice all that:
+        const float C = (mg + mW) * (1.0f + 4.0f * f);
+        const float bnd = 2.0f * (1.1920929e-07f * (1.7320509f * C * sqrtf(gdd) + 3.75f * gdd) +
+                                  1e-12f * C * C + 1.1e-06f * gpe + (float)nrem * epot) +
+                          1e-30f;
+        // Only members within twice the bound of the extremes can be the
+        // exact arg-max or arg-min.  One candidate alone is the exact arg-max
+        // (every other member's exact energy is below gmax - bnd, its own at
+        // least that), and the sign of its exact energy is known when
+        // gmax >= bnd or gmax < -bnd: the usual pass evaluates no FP64 energy.
+        const float hi = gmax - 2.0f * bnd;
         bool go;
-        int ib = cidx;
-        if (ccnt == 1 && gmax >= bnd) {
+        if (A.nounbind || n == 0) {
+            go = false;
+        } else if (!force && gnext < hi && gmax >= bnd) {
             go = true;
-        } else if (ccnt == 1 && gmax < -bnd) {
+            ib = S.wi[par][kw];
+            ra = S.wa[par][kw];
+            rb = S.wb[par][kw];
+        } else if (!force && gnext < hi && gmax < -bnd) {
             go = false;
         } else {
-            mx = ArgRed{-FLT_MAX, 0x7fffffff};
-            if (t1.i < n && t1.v >= hi && x2.v < hi) {
-                mx.v = exact_energy(A, qr[t1.i], qv[t1.i], pot[t1.i], dcm, inv_d, opz_d);
-                mx.i = t1.i;
+            bool flushed;
+            const ArgRed x = BG::template decide<true>(view(), wx, wy, wz, hi, &flushed);
+            if (flushed) nfl = n;
+            go = x.v >= 0.0f;   // kd.c:1389-1409: fTotBig starts at -1
+            if (go) {
+                ib = x.i;
+                view().get(ib, ra, rb);
+                __syncthreads();     // before the slot is overwritten
             }
-            if (x2.v >= hi) rescan(true, false);
-            mx = warp_argmax(mx);
-            if (lane == 0) S.smax[w] = mx;
-            __syncthreads();
-            ArgRed a = S.smax[0];
-            for (int k = 1; k < BS / 32; ++k) {
-                const ArgRed x = S.smax[k];
-                if (x.v > a.v || (x.v == a.v && x.i < a.i)) a = x;
-            }
-            go = a.v >= 0.0f;   // kd.c:1389-1409: fTotBig starts at -1
-            ib = a.i;
-            kw = BS / 32;
-            if (go && tid == 0) {
-                S.cr[kw] = qr[ib];
-                S.cv[kw] = qv[ib];
-                S.cw[kw] = exact ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : qw[ib];
-                S.cp[kw] = pot[ib];
-                S.cid[kw] = qid[ib];
-            }
-            __syncthreads();
         }
-        if (A.nounbind || n == 0) go = false;
         if (!go) {
             // the group's most bound member (fTotMin starts at 1), needed
             // only once the removals stop
-            mn = ArgRed{FLT_MAX, 0x7fffffff};
-            if (b1.i < n && b1.v <= lo && n2.v > lo) {
-                mn.v = exact_energy(A, qr[b1.i], qv[b1.i], pot[b1.i], dcm, inv_d, opz_d);
-                mn.i = b1.i;
-            }
-            if (n2.v <= lo) rescan(false, true);
-            mn = warp_argmin(mn);
-            if (lane == 0) S.smin[w] = mn;
-            __syncthreads();
-            if (tid == 0) {
-                ArgRed b = S.smin[0];
-                for (int k = 1; k < BS / 32; ++k) {
-                    const ArgRed y = S.smin[k];
-                    if (y.v < b.v || (y.v == b.v && y.i < b.i)) b = y;
+            float gmin = FLT_MAX;
+            {
+                const BG B = view();
+                for (int k = tid; k < n; k += BS) {
+                    float4 a, b;
+                    float dd;
+                    B.get(k, a, b);
+                    gmin = fminf(gmin, BG::energy(a, b, wx, wy, wz, dd));
                 }
-                S.s_imin = b.v < 1.0f ? b.i : 0;
+            }
+            gmin = ord2f(__reduce_min_sync(SKID_FULL, f2ord(gmin)));
+            if (lane == 0) S.ext[w][0] = gmin;
+            __syncthreads();
+            for (int k = 0; k < NW; ++k) gmin = fminf(gmin, S.ext[k][0]);
+            bool flushed;
+            const ArgRed x =
+                BG::template decide<false>(view(), wx, wy, wz, gmin + 2.0f * bnd, &flushed);
+            if (tid == 0) S.s_imin = x.v < 1.0f ? x.i : 0;
+            break;
+        }
+        // Remove member ib: the last member takes its slot.
+        const float ms = uniform ? mmax : qr[ib].w;
+        es = uniform ? emax : qv[ib].w;
+        gms = fmul(A.G, ms) * A.opz;
+        ++nrem;
+        --n;
+        if (n == 0) {
+            if (tid == 0) {
+                A.grp[qid[ib]] = 0;
+                S.d_mass = 0.0;
+                for (int d = 3; d < 6; ++d) S.d_cm[d] = 0.0;
             }
             break;
         }
-        // Remove member ib, swapping the last member into its slot
-        // (kd.c:1424-1440): thread 0 updates the FP64 centre while thread 32
-        // moves the records, both from records already read.
-        const int nn = n - 1;
-        if (tid == 0) {
-            const float4 r_ib = S.cr[kw], v_ib = S.cv[kw];
-            A.grp[S.cid[kw]] = 0;
-            ++nrem;
-            if (nn == 0) {
-                S.d_mass = 0.0;
-                for (int d = 3; d < 6; ++d) S.d_cm[d] = 0.0;
-            } else {
-                double mm = S.d_mass;
-                rcm_update(mm, dcm, r_ib, v_ib);
-                S.d_mass = mm;
-                for (int d = 0; d < 6; ++d) {
-                    S.d_cm[d] = dcm[d];
-                    S.s_cm[d] = (float)dcm[d];
-                }
-                if (!exact) {
-                    for (int d = 0; d < 3; ++d)
-                        S.s_w[d] = (float)((double)A.fShift * dcm[3 + d] + (double)A.fCosmo * dcm[d]);
-                    S.s_mW = centre_mag(A, dcm);
-                }
-                S.s_r = r_ib;
-                S.s_eps = v_ib.w;
-                S.s_have = 1;
+        // the centre without it, one float step from the published one
+        f = __fdividef(ms, mass - ms);
+        wx = __fmaf_rn(f, pwx - rb.x, pwx);
+        wy = __fmaf_rn(f, pwy - rb.y, pwy);
+        wz = __fmaf_rn(f, pwz - rb.z, pwz);
+        if (!uniform) {
+            // masses and softenings are read from the records during a pass:
+            // they move before it
+            __syncthreads();
+            if (tid == 0) {
+                const float4 r = qr[ib], v = qv[ib], rl = qr[n], vl = qv[n];
+                const int qb = qid[ib], ql = qid[n];
+                A.grp[qb] = 0;
+                qr[ib] = rl; qv[ib] = vl; qid[ib] = ql; pot[ib] = pot[n];
+                qr[n] = r; qv[n] = v; qid[n] = qb;
             }
-            S.s_n = nn;
-        } else if (tid == 32 && nn > 0) {
-            qr[ib] = lr; qv[ib] = lv; qid[ib] = lq; pot[ib] = lp;
-            qr[nn] = S.cr[kw]; qv[nn] = S.cv[kw]; qid[nn] = S.cid[kw]; pot[nn] = S.cp[kw];
-            if (!exact) {
-                qw[ib] = lw;
-                qw[nn] = S.cw[kw];
+            __syncthreads();
+            if (keeper) ib = n;      // where its record is now
+        }
+        if (!keeper) {
+            // its owner moves the state before it comes to the slot
+            if (ib % BC == tid && ib != n) {
+                const BG B = view();
+                float4 a, b;
+                B.get(n, a, b);
+                B.put(ib, a, b);
             }
         }
-        __syncthreads();
-        if (nn == 0) break;
+        par ^= 1;
     }
+    __syncthreads();
     if (tid == 0) {
         double dcm[6];
         for (int d = 0; d < 6; ++d) dcm[d] = S.d_cm[d];
-        write_record(A, g, S.s_n, S.d_mass, dcm, qr[S.s_imin], nrem);
+        write_record(A, g, n, S.d_mass, dcm, qr[S.s_imin], nrem);
     }
     __syncthreads();
 }
@@ -1667,13 +1904,14 @@ __device__ void cluster_group(const RemoveArgs &A, int g, BlockShared<BS> &S, Cl
 // each), then chunks of BS/32 small groups (one warp each), all largest
 // first.  With A.single > 0 one block processes just that group.
 template <int BS, int CS>
-__global__ void __launch_bounds__(BS) remove_kernel(RemoveArgs A)
+__global__ void __launch_bounds__(BS) remove_kernel(const __grid_constant__ RemoveArgs A)
 {
     __shared__ BlockShared<BS> S;
     __shared__ int s_item;
+    extern __shared__ float4 dyn[];
     constexpr int W = BS / 32;
     if (A.single > 0) {
-        block_group<BS>(A, A.single, S);
+        block_group<BS>(A, A.single, S, dyn);
         return;
     }
     int first = 0;
@@ -1681,7 +1919,6 @@ __global__ void __launch_bounds__(BS) remove_kernel(RemoveArgs A)
         // launched as clusters of CS blocks: the largest groups first, one
         // cluster each, then every block goes on alone
         __shared__ ClusterShared C;
-        extern __shared__ float4 dyn[];
         cg::cluster_group cl = cg::this_cluster();
         const int nclu = *A.d_ccnt;
         for (;;) {
@@ -1704,7 +1941,7 @@ __global__ void __launch_bounds__(BS) remove_kernel(RemoveArgs A)
         __syncthreads();
         if (item >= nitems) break;
         if (item < nb) {
-            block_group<BS>(A, (int)A.order[first + item], S);
+            block_group<BS>(A, (int)A.order[first + item], S, dyn);
         } else {
             int k = nbig + (item - nb) * W + (threadIdx.x >> 5);
             if (k < nvalid) warp_group(A, (int)A.order[k]);
@@ -1712,22 +1949,73 @@ __global__ void __launch_bounds__(BS) remove_kernel(RemoveArgs A)
     }
 }
 
-template <int BS>
-cudaError_t launch_remove(const RemoveArgs &A, int blocks, cudaStream_t st)
+// Raise a removal kernel's shared-memory limit to all it can have, once per
+// device (the attribute is only an upper bound; contexts on other threads
+// launch with other sizes).
+template <int BS, int CS>
+cudaError_t remove_smem_limit(int *dyn_max)
 {
-    remove_kernel<BS, 1><<<blocks, BS, 0, st>>>(A); note_launch();
+    static std::mutex mu;
+    static int most[SKID_MAX_DEVICES] = {};
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e) return e;
+    if (dev < 0 || dev >= SKID_MAX_DEVICES) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!most[dev]) {
+        cudaFuncAttributes fa;
+        if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) ||
+            (e = cudaFuncGetAttributes(&fa, remove_kernel<BS, CS>)))
+            return e;
+        const int d = optin - (int)fa.sharedSizeBytes;
+        if ((e = cudaFuncSetAttribute(remove_kernel<BS, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, d)))
+            return e;
+        most[dev] = d;
+    }
+    *dyn_max = most[dev];
+    return cudaSuccess;
+}
+
+// Shared memory a block of a plain removal launch takes: 32 B for each member
+// of the largest group, up to LCAP_KB.
+#ifndef SKID_LCAP_KB
+#define SKID_LCAP_KB 220
+#endif
+constexpr int LCAP_BYTES = SKID_LCAP_KB * 1024;
+constexpr int LMEMBER = 2 * (int)sizeof(float4);
+
+template <int BS>
+cudaError_t launch_remove(RemoveArgs A, int nlargest, int single, cudaStream_t st)
+{
+    int most = 0, perSM = 0;
+    cudaError_t e = remove_smem_limit<BS, 1>(&most);
+    if (e) return e;
+    if (most > LCAP_BYTES) most = LCAP_BYTES;
+    constexpr int row = 2 * BlockGroup<BS>::BC;
+    const long long want = ((long long)nlargest + row - 1) / row * row * LMEMBER;
+    A.lcap = (int)(want < most ? want : most) / LMEMBER;
+    const size_t smem = (size_t)A.lcap * LMEMBER;
+    int blocks = 1;
+    if (!single) {
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, remove_kernel<BS, 1>, BS, smem)))
+            return e;
+        blocks = num_sms() * (perSM > 0 ? perSM : 1);
+    }
+    remove_kernel<BS, 1><<<blocks, BS, smem, st>>>(A); note_launch();
     return cudaGetLastError();
 }
 
 // Cluster launch: as many clusters of CS blocks as fit at once, each block
 // with A.qcap members' worth of dynamic shared memory.
 template <int BS, int CS>
-cudaError_t launch_remove_clusters(const RemoveArgs &A, cudaStream_t st)
+cudaError_t launch_remove_clusters(RemoveArgs A, cudaStream_t st)
 {
     const size_t smem = (size_t)A.qcap * (2 * sizeof(float4) + sizeof(long long));
-    cudaError_t e = cudaFuncSetAttribute(remove_kernel<BS, CS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int most = 0;
+    cudaError_t e = remove_smem_limit<BS, CS>(&most);
     if (e) return e;
+    if (smem > (size_t)most) return cudaErrorInvalidValue;
+    A.lcap = (int)smem / LMEMBER;   // the same memory, once the blocks go on alone
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1749,8 +2037,9 @@ cudaError_t launch_remove_clusters(const RemoveArgs &A, cudaStream_t st)
     return e ? e : cudaGetLastError();
 }
 
-// cs: 1 (no clusters), 4 or 8
-cudaError_t remove_launch(const RemoveArgs &A, int bs, int cs, int blocks, cudaStream_t st)
+// cs: 1 (no clusters), 4 or 8; nlargest: the members of the largest group a
+// block will take; single: one block for A.single alone
+cudaError_t remove_launch(const RemoveArgs &A, int bs, int cs, int nlargest, bool single, cudaStream_t st)
 {
     if (cs == 4 || cs == 8) {
         switch (bs) {
@@ -1760,23 +2049,11 @@ cudaError_t remove_launch(const RemoveArgs &A, int bs, int cs, int blocks, cudaS
         }
     }
     switch (bs) {
-    case 128: return launch_remove<128>(A, blocks, st);
-    case 512: return launch_remove<512>(A, blocks, st);
-    case 1024: return launch_remove<1024>(A, blocks, st);
-    default: return launch_remove<256>(A, blocks, st);
+    case 128: return launch_remove<128>(A, nlargest, single, st);
+    case 512: return launch_remove<512>(A, nlargest, single, st);
+    case 1024: return launch_remove<1024>(A, nlargest, single, st);
+    default: return launch_remove<256>(A, nlargest, single, st);
     }
-}
-
-int remove_blocks(int bs)
-{
-    int perSM = 0;
-    switch (bs) {
-    case 128: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, remove_kernel<128, 1>, 128, 0); break;
-    case 512: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, remove_kernel<512, 1>, 512, 0); break;
-    case 1024: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, remove_kernel<1024, 1>, 1024, 0); break;
-    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, remove_kernel<256, 1>, 256, 0); break;
-    }
-    return num_sms() * (perSM > 0 ? perSM : 1);
 }
 
 }  // namespace
@@ -1791,7 +2068,7 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
 {
     cudaError_t e;
     int ng = G.nGroup;
-    if ((e = dalloc(U.qr, nslots)) || (e = dalloc(U.qv, nslots)) || (e = dalloc(U.qw, nslots)) ||
+    if ((e = dalloc(U.qr, nslots)) || (e = dalloc(U.qv, nslots)) || (e = dalloc(U.qw, nslots)) || (e = dalloc(U.qa, nslots)) ||
         (e = dalloc(U.qid, nslots)) ||
         (e = dalloc(U.pot, nslots)) || (e = dalloc(U.scnt, ng)) || (e = dalloc(U.soff, ng + 1)) ||
         (e = dalloc(U.nt, ng)) || (e = dalloc(U.toff, ng + 1)) || (e = dalloc(U.cnt, 16)) ||
@@ -1840,10 +2117,8 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
     const int clu_min = P.clu_min > P.tw && P.clu_min > 1024 ? P.clu_min : 0;
     const int clu_kmax = num_sms() / 8 > 1 ? num_sms() / 8 : 1;
     if ((e = cudaMemsetAsync(U.cnt.p + 8, 0, 4 * sizeof(int), st))) return e;
-    if (clu_min > 0) {
-        cluster_groups<<<1, 32, 0, st>>>(U.order.p, U.cnt.p + 2, G.count.p, clu_min, clu_kmax,
-                                         U.cnt.p + 9); note_launch();
-    }
+    cluster_groups<<<1, 32, 0, st>>>(U.order.p, U.cnt.p + 2, G.count.p, clu_min,
+                                     clu_min > 0 ? clu_kmax : 0, U.cnt.p + 9); note_launch();
     int hc[11] = {0};
     if ((e = cudaMemcpyAsync(hc, U.cnt.p + 1, 11 * sizeof(int), cudaMemcpyDeviceToHost, st))) return e;
     if ((e = cudaStreamSynchronize(st))) return e;
@@ -1869,7 +2144,9 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
     A.nmax = P.nmax;
     A.qr = U.qr.p;
     A.qv = U.qv.p;
+    A.qa = U.qa.p;
     A.qw = U.qw.p;
+    A.lcap = 0;
     A.qid = U.qid.p;
     A.pot = U.pot.p;
     A.rec = G.rec.p;
@@ -1910,7 +2187,8 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
         sched_counts<<<grid_for(ng), 256, 0, st>>>(G.count.p, ng, P.nmax, tw, U.cnt.p + 4); note_launch();
         if ((e2 = cudaMemsetAsync(d_unbound, 0, sizeof(int), st))) return e2;
         if (nvalid <= 0) return cudaSuccess;
-        return remove_launch(A, bs, bs >= 256 ? ucs : 1, remove_blocks(bs), st);
+        // groups of up to tw members take no block
+        return remove_launch(A, bs, bs >= 256 ? ucs : 1, nlargest > tw ? nlargest : 0, false, st);
     };
 
     if (P.per_group) {
@@ -1931,7 +2209,7 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
                 U.scnt.p, U.slist.p, U.ssoft.p, P.G, P.plummer, P.scale, U.pot.p); note_launch();
             RemoveArgs A1 = A;
             A1.single = (int)order[k];
-            if ((e = remove_launch(A1, 256, 1, 1, st))) return e;
+            if ((e = remove_launch(A1, 256, 1, nlargest, true, st))) return e;
         }
         return cudaGetLastError();
     }
