@@ -147,6 +147,27 @@ __device__ __forceinline__ float boxbox_lb(float4 alo, float4 ahi, float4 blo, f
     return (dx * dx + dy * dy + dz * dz) * (1.0f - 4e-6f);
 }
 
+// No point of box a is nearer to a point of box b through a periodic image:
+// every coordinate difference lies within half a period (img_class 0, which
+// float subtraction, being monotonic, decides from the boxes' ends).
+__device__ __forceinline__ bool boxes_direct(float4 alo, float4 ahi, float4 blo, float4 bhi, float3 h)
+{
+    return fsub(ahi.x, blo.x) <= h.x && fsub(bhi.x, alo.x) <= h.x && fsub(ahi.y, blo.y) <= h.y &&
+           fsub(bhi.y, alo.y) <= h.y && fsub(ahi.z, blo.z) <= h.z && fsub(bhi.z, alo.z) <= h.z;
+}
+
+// Largest lower bound of d2of over two direct boxes' points (a point is its
+// own box): the gaps between them under the same roundings.  Subtraction,
+// product and sum round monotonically, so no slack is needed, against about
+// 60 instructions with images and slack.
+__device__ __forceinline__ float gap2(float3 alo, float3 ahi, float4 blo, float4 bhi)
+{
+    return d2of(fmaxf(fmaxf(fsub(blo.x, ahi.x), fsub(alo.x, bhi.x)), 0.0f),
+                fmaxf(fmaxf(fsub(blo.y, ahi.y), fsub(alo.y, bhi.y)), 0.0f),
+                fmaxf(fmaxf(fsub(blo.z, ahi.z), fsub(alo.z, bhi.z)), 0.0f));
+}
+__device__ __forceinline__ float3 xyz(float4 v) { return make_float3(v.x, v.y, v.z); }
+
 // Spread the low 21 bits of v to every third bit.
 __device__ __forceinline__ uint64_t spread3(uint64_t v)
 {

@@ -112,6 +112,302 @@ __device__ __forceinline__ float warp_max(float v)
     return v;
 }
 
+// ---- k from KB_MINK to KB_MAXK: unsorted buffers ----
+//
+// The heaps' sift-down runs for the whole warp whenever any lane takes a
+// candidate, some 50k of 79k instructions for 32 queries at k = 64.  Here a
+// lane appends what lies below its bound to a buffer of cap values in shared
+// memory (value i of lane l at i * 32 + l) and, when some lane's is nearly
+// full, all lanes cut theirs back at once: a threshold that leaves k values or
+// somewhat more is found by counting (a guess from the counts and the 3/2
+// power law of squared distances, usually one or two counts), the rest
+// dropped, and the threshold is the lane's new bound.  The k-th smallest is
+// found exactly at the end.  Candidates are tested two to a packed FP32
+// operation, and where no periodic image can be nearer (nearly every leaf of
+// a query away from the box's faces) the bounds are exact and cheap.
+//
+// At 2^20 points, k = 64: 82k instructions a leaf to 52k, 4.04 ms to 3.34; the
+// call with its tree, 2^18 points: k = 128 3.81 to 2.78 ms, 32 1.24 to 1.05, 24
+// 1.06 to 0.94, 16 0.83 to 0.84 (so the heaps keep small k; above 128 the
+// buffers would leave too few warps an SM).  Bound by instruction issue at
+// half the slots: 12 warps an SM, each a chain.  Room for 48 or 96 values
+// beyond k, and cutting closer or less, were slower.  Counting distances into
+// radial bins instead, with a second walk to pick from the k-th one's, took
+// 62k instructions and had a longer tail: no faster.
+constexpr int KB_MINK = 24, KB_MAXK = 128;
+constexpr int KB_WARPS = 1;
+constexpr int KB_SLACK = 64;         // values a buffer holds beyond k
+constexpr int KB_STEP = 8;           // candidates tested between checks for room
+
+struct KnnBuf {
+    float *b;        // this lane's values, stride 32
+    int n;           // values held
+    float thr;       // at or above the k-th smallest so far; new values lie below
+};
+
+// Values at or below T (entries past a lane's last are infinite).
+__device__ __forceinline__ int kb_count(const KnnBuf &B, int m, float T)
+{
+    // non-negative floats order as their bit patterns: the sign of the
+    // difference to the pattern after T's is the comparison
+    const int after = __float_as_int(T) + 1;
+    const int *b = reinterpret_cast<const int *>(B.b);
+    unsigned c = 0;
+#pragma unroll 16
+    for (int i = 0; i < m; ++i) c += (unsigned)(b[i * 32] - after) >> 31;
+    return (int)c;
+}
+
+// The largest value (0 without any).
+__device__ __forceinline__ float kb_largest(const KnnBuf &B, int m)
+{
+    float v = 0.0f;
+#pragma unroll 8
+    for (int i = 0; i < m; ++i) {
+        const float x = B.b[i * 32];
+        v = x < INFINITY ? fmaxf(v, x) : v;
+    }
+    return v;
+}
+
+// The k-th smallest value of a lane that holds at least k, between lo (fewer
+// than k values at or below it; -1: none are) and hi (k or more): guesses from
+// the counts, then bisection of the bit patterns.
+__device__ __forceinline__ float kb_kth(const KnnBuf &B, int m, int k, int lo, float hi, int cl)
+{
+    int l = lo, h = __float_as_int(hi), ch = B.n;
+    bool done = B.n < k, largest = false;
+    for (int it = 0; __any_sync(SKID_FULL, !done); ++it) {
+        if (!done && h - l <= 1) done = true;      // h is the answer
+        int mid = l + (h - l) / 2;
+        if (it < 6) {
+            const float a = l < 0 ? 0.0f : __int_as_float(l), b = __int_as_float(h);
+            float t = (k + 0.0f - cl) / fmaxf((float)(ch - cl), 1.0f);
+            if (cl == 0) t = exp2f(0.6666667f * log2f(t));
+            const int g = __float_as_int(fmaf(b - a, fminf(fmaxf(t, 0.02f), 0.98f), a));
+            if (g > l && g < h) mid = g;
+        }
+        const int c = kb_count(B, m, __int_as_float(mid));
+        if (!done) {
+            if (c < k) {
+                l = mid;
+                cl = c;
+            } else {
+                h = mid;
+                ch = c;
+                if (c == k) done = largest = true;
+            }
+        }
+    }
+    // a lane that stopped at exactly k values takes the largest of them
+    const float T = __int_as_float(h);
+    if (!__any_sync(SKID_FULL, largest)) return T;
+    float v = 0.0f;
+#pragma unroll 8
+    for (int i = 0; i < m; ++i) {
+        const float x = B.b[i * 32];
+        v = x <= T ? fmaxf(v, x) : v;
+    }
+    return largest ? v : T;
+}
+
+// Cut every lane's buffer back: at least k values stay, at most `most`.
+__device__ __noinline__ KnnBuf kb_cut(KnnBuf B, int k, int most)
+{
+    const int m = __reduce_max_sync(SKID_FULL, B.n);
+    float hi = B.thr;
+    if (__any_sync(SKID_FULL, B.thr == FLT_MAX)) hi = fminf(hi, kb_largest(B, m));
+    float lo = 0.0f, T = hi;
+    int cl = 0, ch = B.n;
+    // lanes with little to drop keep what they have
+    bool done = B.n <= k + (most - k) / 4;
+    const bool skip = done;
+    const float aim = k + 0.15f * (most - k);
+    for (int it = 0; it < 6 && __any_sync(SKID_FULL, !done); ++it) {
+        float t = (aim - cl) / fmaxf((float)(ch - cl), 1.0f);
+        if (cl == 0) t = exp2f(0.6666667f * log2f(t));
+        const float mid = fmaf(hi - lo, fminf(fmaxf(t, 0.02f), 0.98f), lo);
+        const int c = kb_count(B, m, mid);
+        if (!done) {
+            if (c < k) {
+                lo = mid;
+                cl = c;
+            } else {
+                hi = T = mid;
+                ch = c;
+                done = c <= most;
+            }
+        }
+    }
+    // ties or an uneven spread: the exact k-th value, and of its copies only
+    // as many as make k
+    const bool tight = !done && B.n >= k;
+    int room = 0x7fffffff;
+    if (__any_sync(SKID_FULL, tight)) {
+        const float e = kb_kth(B, m, k, cl == 0 ? -1 : __float_as_int(lo), hi, cl);
+        int below = 0;
+#pragma unroll 8
+        for (int i = 0; i < m; ++i) below += B.b[i * 32] < e;
+        if (tight) {
+            T = e;
+            room = k - below;
+        }
+    }
+    if (skip) T = FLT_MAX;
+    int o = 0;
+    if (__any_sync(SKID_FULL, tight)) {
+        for (int i = 0; i < m; ++i) {
+            const float x = B.b[i * 32];
+            bool keep = x <= T;
+            if (keep && x == T) keep = room-- > 0;
+            if (keep) B.b[o++ * 32] = x;
+        }
+    } else {
+#pragma unroll 8
+        for (int i = 0; i < m; ++i) {
+            const float x = B.b[i * 32];
+            if (x <= T) B.b[o++ * 32] = x;
+        }
+    }
+    for (int i = __reduce_min_sync(SKID_FULL, o); i < m; ++i)
+        if (i >= o) B.b[i * 32] = INFINITY;
+    B.n = o;
+    if (!skip) B.thr = fminf(B.thr, T);
+    return B;
+}
+
+__global__ void __launch_bounds__(KB_WARPS * 32)
+knn_buffer_kernel(TreeView t, int k, int cap, float3 L, float3 hL, bool per, int logLeafBase,
+                  int subShift, float zero_arg, float *__restrict__ ball2, int *work)
+{
+    extern __shared__ float4 smem4[];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // candidates by component, then the lanes' buffers
+    float *cx = reinterpret_cast<float *>(smem4) + w * 3 * SKID_LEAF;
+    float *cy = cx + SKID_LEAF, *cz = cy + SKID_LEAF;
+    float *bufs = reinterpret_cast<float *>(smem4) + KB_WARPS * 3 * SKID_LEAF;
+    const int rootLo = t.leafBase >> subShift;
+    const int most = k + (cap - k) / 2;
+    const f32x2 zero = pack2(zero_arg, zero_arg);
+    KnnBuf B;
+    B.b = bufs + (size_t)w * cap * 32 + lane;
+    for (;;) {
+        int leaf = 0;
+        if (lane == 0) leaf = atomicAdd(work, 1);
+        leaf = __shfl_sync(SKID_FULL, leaf, 0);
+        if (leaf >= t.nLeaf) break;
+        const int base = leaf * SKID_LEAF, qi = base + lane;
+        const bool valid = qi < t.n;
+        const float4 qp = t.pos[valid ? qi : base];
+        const float3 q = make_float3(qp.x, qp.y, qp.z);
+        const f32x2 nqx = pack2(-q.x, -q.x), nqy = pack2(-q.y, -q.y), nqz = pack2(-q.z, -q.z);
+        B.n = 0;
+        B.thr = FLT_MAX;
+        for (int i = 0; i < cap; ++i) B.b[i * 32] = INFINITY;
+        const int own = t.leafBase + leaf;
+        const float4 qlo = t.lo[own], qhi = t.hi[own];   // the queries' box
+        auto tmax = [&]() {
+            return __uint_as_float(__reduce_max_sync(SKID_FULL, __float_as_uint(B.thr)));
+        };
+        auto room = [&]() {
+            if (__any_sync(SKID_FULL, B.n > cap - KB_STEP)) B = kb_cut(B, k, most);
+        };
+        // lane j keeps candidate j while it may lie below some lane's bound
+        auto leaf_values = [&](int node, bool direct, bool all) {
+            const int cb = (node - t.leafBase) * SKID_LEAF;
+            float4 c4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float tm = all ? INFINITY : tmax();
+            bool rel = cb + lane < t.n;
+            if (rel) {
+                c4 = t.pos[cb + lane];
+                if (!all)
+                    rel = (direct ? gap2(xyz(c4), xyz(c4), qlo, qhi)
+                                  : box_lb(xyz(c4), qlo, qhi, L, per)) < tm;
+            }
+            const unsigned R = __ballot_sync(SKID_FULL, rel);
+            const int nR = __popc(R);
+            const int rank = __popc(R & ((1u << lane) - 1u));
+            // survivors in order, then entries no query can take
+            const int slot = rel ? rank : nR + lane - rank;
+            __syncwarp();
+            cx[slot] = rel ? c4.x : INFINITY;
+            cy[slot] = c4.y;
+            cz[slot] = c4.z;
+            __syncwarp();
+            for (int j0 = 0; j0 < nR; j0 += KB_STEP) {
+                room();
+                if (direct) {
+#pragma unroll
+                    for (int j = 0; j < KB_STEP; j += 4) {
+                        const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(cx + j0 + j);
+                        const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(cy + j0 + j);
+                        const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(cz + j0 + j);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const f32x2 dx = add2(h ? X.y : X.x, nqx), dy = add2(h ? Y.y : Y.x, nqy),
+                                        dz = add2(h ? Z.y : Z.x, nqz);
+                            const float2 d = unpack2(add2(add2(sq2(dx, zero), sq2(dy, zero)), sq2(dz, zero)));
+                            if (d.x < B.thr) B.b[B.n++ * 32] = d.x;
+                            if (d.y < B.thr) B.b[B.n++ * 32] = d.y;
+                        }
+                    }
+                } else {
+                    for (int j = j0; j < min(nR, j0 + KB_STEP); ++j) {
+                        const float d2 = d2of(img_dx(q.x, cx[j], L.x, hL.x), img_dx(q.y, cy[j], L.y, hL.y),
+                                              img_dx(q.z, cz[j], L.z, hL.z));
+                        if (d2 < B.thr) B.b[B.n++ * 32] = d2;
+                    }
+                }
+            }
+        };
+        leaf_values(own, boxes_direct(qlo, qhi, qlo, qhi, hL), true);
+        int cell = own;
+        while (cell > 1) {
+            int cp = cell ^ 1;
+            const int end = next_node(cp);
+            for (;;) {
+                const float4 blo = t.lo[cp], bhi = t.hi[cp];
+                const bool direct = boxes_direct(qlo, qhi, blo, bhi, hL);
+                if (cp >= rootLo) {
+                    // a subtree of at most 2^subShift leaves: one lane per
+                    // leaf against the queries' box and the largest bound,
+                    // then each passing leaf in order with the exact bounds
+                    const int sh = logLeafBase - (31 - __clz(cp));
+                    const int first = cp << sh;
+                    const float tm = tmax();
+                    bool pass = false;
+                    if (lane < (1 << sh) && first + lane - t.leafBase < t.nLeaf) {
+                        const float4 l = t.lo[first + lane], h = t.hi[first + lane];
+                        pass = (direct ? gap2(xyz(qlo), xyz(qhi), l, h) : boxbox_lb(qlo, qhi, l, h, L, per)) < tm;
+                    }
+                    for (unsigned lm = __ballot_sync(SKID_FULL, pass); lm; lm &= lm - 1) {
+                        const int node = first + __ffs(lm) - 1;
+                        const float4 l = t.lo[node], h = t.hi[node];
+                        const bool dl = direct || boxes_direct(qlo, qhi, l, h, hL);
+                        const bool want = (dl ? gap2(q, q, l, h) : box_lb(q, l, h, L, per)) < B.thr;
+                        if (!__any_sync(SKID_FULL, want)) continue;
+                        leaf_values(node, dl, false);
+                    }
+                } else {
+                    const bool want = (direct ? gap2(q, q, blo, bhi) : box_lb(q, blo, bhi, L, per)) < B.thr;
+                    if (__any_sync(SKID_FULL, want)) { cp <<= 1; continue; }
+                }
+                cp = next_node(cp);
+                if (cp == end) break;
+            }
+            cell >>= 1;
+        }
+        // the k-th smallest of what is left (the last bound is at or above it)
+        const int m = __reduce_max_sync(SKID_FULL, B.n);
+        float hi = B.thr;
+        if (__any_sync(SKID_FULL, B.thr == FLT_MAX)) hi = fminf(hi, kb_largest(B, m));
+        const float r = kb_kth(B, m, k, -1, hi, 0);
+        if (valid) ball2[qi] = B.n >= k ? r : FLT_MAX;
+    }
+}
+
+// ---- any k: heaps ----
+
 // Heaps live in shared memory after the candidate buffers, or -- for k too
 // large for one warp's heaps to fit -- in global scratch (gheap, one slab per
 // resident warp).
@@ -186,6 +482,24 @@ cudaError_t knn_ball2(const Tree &t, int k, float3 L, bool per, float *ball2_sor
                       DBuf<float> &gheap, cudaStream_t st)
 {
     if (t.n <= 0) return cudaSuccess;
+    float3 hL = make_float3(0.5f * L.x, 0.5f * L.y, 0.5f * L.z);
+    int logLeafBase = 0;
+    while ((2 << logLeafBase) <= t.leafBase) ++logLeafBase;
+    const int subShift = logLeafBase < 5 ? logLeafBase : 5;
+    if (k >= KB_MINK && k <= KB_MAXK) {
+        const int cap = k + KB_SLACK;
+        const size_t smem = KB_WARPS * (3 * SKID_LEAF + (size_t)cap * 32) * sizeof(float);
+        int perSM = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, knn_buffer_kernel, KB_WARPS * 32, smem);
+        if (e) return e;
+        if (perSM < 1) return cudaErrorInvalidConfiguration;
+        const int need = (t.nLeaf + KB_WARPS - 1) / KB_WARPS;
+        const int blocks = num_sms() * perSM < need ? num_sms() * perSM : need;
+        if ((e = cudaMemsetAsync(d_work, 0, sizeof(int), st))) return e;
+        knn_buffer_kernel<<<blocks, KB_WARPS * 32, smem, st>>>(t.view(), k, cap, L, hL, per, logLeafBase,
+                                                               subShift, 0.0f, ball2_sorted, d_work); skid::note_launch();
+        return cudaGetLastError();
+    }
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -226,11 +540,7 @@ cudaError_t knn_ball2(const Tree &t, int k, float3 L, bool per, float *ball2_sor
         if ((e = dalloc(gheap, (size_t)blocks * nw * k * 32))) return e;
         gh = gheap.p;
     }
-    float3 hL = make_float3(0.5f * L.x, 0.5f * L.y, 0.5f * L.z);
     if ((e = cudaMemsetAsync(d_work, 0, sizeof(int), st))) return e;
-    int logLeafBase = 0;
-    while ((2 << logLeafBase) <= t.leafBase) ++logLeafBase;
-    int subShift = logLeafBase < 5 ? logLeafBase : 5;
     knn_kernel<<<blocks, nw * 32, smem, st>>>(t.view(), k, L, hL, per, logLeafBase, subShift,
                                               ball2_sorted, d_work, gh); skid::note_launch();
     return cudaGetLastError();
