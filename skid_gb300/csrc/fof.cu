@@ -187,12 +187,25 @@ link_kernel(TreeView t, float tau2, float3 L, float3 hL, bool per, int subShift,
     }
 }
 
-// label -> smallest member iOrder per root
+// The root of x without path halving.
+__device__ __forceinline__ int uf_root(const int *par, int x)
+{
+    for (int it = 0; it < UF_SPIN_LIMIT; ++it) {
+        const int p = __ldcg(&par[x]);
+        if (p == x) return x;
+        x = p;
+    }
+    return x;
+}
+
+// label -> smallest member iOrder per root.  A thread writes its own slot
+// only: halving other slots' paths here could put an ancestor read earlier
+// over a root already written there, and what follows takes par for roots.
 __global__ void root_min_iorder(int *par, int n, const uint32_t *__restrict__ perm,
                                 const int *__restrict__ mio, int *__restrict__ minio)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int r = uf_find(par, i);
+        int r = uf_root(par, i);
         par[i] = r;
         atomicMin(&minio[r], mio[perm[i]]);
     }
