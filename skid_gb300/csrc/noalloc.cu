@@ -35,7 +35,7 @@ constexpr int NA_MAXN = SKID_NOALLOC_MAX_POINTS;
 constexpr int NA_MAXK = SKID_NOALLOC_MAX_K;
 constexpr int NA_LEAFBASE = (NA_MAXN + SKID_LEAF - 1) / SKID_LEAF;   // power of two
 constexpr int NA_NODES = 2 * NA_LEAFBASE;
-constexpr int NA_TILES = (NA_MAXN + 4095) / 4096;                   // radix-sort tiles
+constexpr int NA_TILES = (NA_MAXN + 1023) / 1024;                   // radix-sort tiles (the smaller kind)
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 

@@ -4,8 +4,8 @@
 // The sort reads the keys once up front to count every digit position's
 // histogram (one kernel for all passes), turns them into global digit
 // offsets (one small kernel), then makes one kernel launch per 8-bit pass.
-// A pass takes tiles of 4096 keys (each of 8 warps ranks 512 contiguous
-// keys with warp match, so tile order = input order) in the order blocks
+// A pass takes tiles of 4096 or 1024 keys (each of 8 warps ranks an eighth of
+// them, contiguous, with warp match, so tile order = input order) in the order blocks
 // start (a tile counter), so a tile's predecessors are always already
 // running: it counts its digits, publishes them, and finds the keys of each
 // digit before it by decoupled look-back over the predecessors' published
@@ -13,6 +13,7 @@
 // scatters its keys stably.  Each look-back wait is bounded; one that runs
 // out sets the caller's status word.
 
+#include <algorithm>
 #include <atomic>
 
 #include "internal.h"
@@ -49,9 +50,16 @@ void bump_alloc_epoch() { ++g_alloc_epoch; }
 namespace {
 
 constexpr int RS_THREADS = 256;
-constexpr int RS_ROUNDS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
 constexpr int RS_WARPS = RS_THREADS / 32;
+// Rounds of 32 keys a warp ranks in a pass: tiles of 4096 keys, or of 1024
+// while there are at most two of those an SM (311,296 keys on 152 SMs).  A
+// pass on few tiles takes the time of one tile, the serial ranking of its
+// rounds: friends-of-friends' grouping of n isolated points, an 8-pass sort
+// and little else, takes with large / small tiles 0.235 / 0.201 ms at 1,000
+// points, 0.302 / 0.261 at 20,000, 0.433 / 0.430 at 300,000, 0.488 / 0.513 at
+// 500,000 and 0.703 / 0.716 at 2^20 (four times the tiles to look back over).
+constexpr int RS_ROUNDS_MANY = 16, RS_ROUNDS_FEW = 4;
+constexpr int RS_FEW_MAX = 2;         // tiles of 1024 keys per SM
 
 // ---- one-sweep passes ----
 constexpr int OS_WARPS = RS_WARPS;
@@ -78,34 +86,33 @@ __global__ void os_histogram(const uint64_t *__restrict__ keys, int n, const int
         if (h[i]) atomicAdd(&glob[i], h[i]);
 }
 
-// Histograms -> exclusive global offsets, one pass at a time (256 threads).
-__global__ void os_offsets(uint32_t *glob, int passes)
+// Histograms -> exclusive global offsets, a block of 256 threads per pass.
+__global__ void os_offsets(uint32_t *glob)
 {
     __shared__ uint32_t ws[8];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    for (int p = 0; p < passes; ++p) {
-        const uint32_t x = glob[p * 256 + t];
-        uint32_t v = x;
+    uint32_t *h = glob + blockIdx.x * 256;
+    const uint32_t x = h[t];
+    uint32_t v = x;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(SKID_FULL, v, o);
-            if (lane >= o) v += y;
-        }
-        if (lane == 31) ws[w] = v;
-        __syncthreads();
-        uint32_t before = 0;
-        for (int j = 0; j < w; ++j) before += ws[j];
-        glob[p * 256 + t] = before + v - x;
-        __syncthreads();
+    for (int o = 1; o < 32; o <<= 1) {
+        uint32_t y = __shfl_up_sync(SKID_FULL, v, o);
+        if (lane >= o) v += y;
     }
+    if (lane == 31) ws[w] = v;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int j = 0; j < w; ++j) before += ws[j];
+    h[t] = before + v - x;
 }
 
+template <int ROUNDS>
 __global__ void __launch_bounds__(RS_THREADS)
 os_pass(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin,
         uint64_t *__restrict__ kout, uint32_t *__restrict__ vout, int n, const int *d_n, int shift,
         const uint32_t *__restrict__ goff, uint32_t *status, uint32_t *counter, unsigned *d_err)
 {
-    constexpr int WKEYS = RS_ROUNDS * 32;          // keys per warp, contiguous
+    constexpr int WKEYS = ROUNDS * 32;          // keys per warp, contiguous
     __shared__ uint32_t s_tile;
     __shared__ uint32_t wcnt[OS_WARPS][256];       // per-warp digit counts, then offsets
     __shared__ uint32_t run[256];                  // the tile's first output slot per digit
@@ -116,17 +123,17 @@ os_pass(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin,
     for (int j = 0; j < OS_WARPS; ++j) wcnt[j][tid] = 0;
     __syncthreads();
     const int tile = (int)s_tile;
-    const int base = tile * RS_TILE;
+    const int base = tile * (RS_THREADS * ROUNDS);
     if (base >= n) return;   // beyond the live keys (block-uniform)
-    // warp w ranks keys [base + w WKEYS, base + (w+1) WKEYS) in 16 rounds of
+    // warp w ranks keys [base + w WKEYS, base + (w+1) WKEYS) in rounds of
     // 32: a key's place among its warp's keys of the same digit is the
     // count from earlier rounds plus its rank among equal digits this round
     const int wbase = base + w * WKEYS;
     const unsigned lt = (1u << lane) - 1u;
-    uint64_t k[RS_ROUNDS];
-    uint32_t v[RS_ROUNDS], loc[RS_ROUNDS];
+    uint64_t k[ROUNDS];
+    uint32_t v[ROUNDS], loc[ROUNDS];
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
+    for (int r = 0; r < ROUNDS; ++r) {
         const int i = wbase + r * 32 + lane;
         const bool valid = i < n;
         k[r] = valid ? kin[i] : 0;
@@ -178,7 +185,7 @@ os_pass(const uint64_t *__restrict__ kin, const uint32_t *__restrict__ vin,
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
+    for (int r = 0; r < ROUNDS; ++r) {
         const int i = wbase + r * 32 + lane;
         if (i < n) {
             const unsigned d = (unsigned)((k[r] >> shift) & 0xff);
@@ -295,21 +302,31 @@ cudaError_t radix_sort(SortScratch &s, int n, int bits, cudaStream_t st, const i
 {
     if (n <= 0 || bits <= 0) return cudaSuccess;
     const int passes = (bits + 7) / 8 < OS_MAXPASS ? (bits + 7) / 8 : OS_MAXPASS;
-    const int nTiles = (n + RS_TILE - 1) / RS_TILE;
+    const bool few = n <= num_sms() * RS_THREADS * RS_ROUNDS_FEW * RS_FEW_MAX;
+    const int tileKeys = RS_THREADS * (few ? RS_ROUNDS_FEW : RS_ROUNDS_MANY);
+    const int nTiles = (n + tileKeys - 1) / tileKeys;
+    // a scratch that has held n keys holds any smaller sort, of either tile
+    const int scratchTiles = few ? nTiles : std::max(nTiles, num_sms() * RS_FEW_MAX);
     cudaError_t e;
-    if ((e = dalloc(s.hist, (size_t)256 * nTiles)) || (e = dalloc(s.glob, SORT_GLOB_WORDS)))
+    if ((e = dalloc(s.hist, (size_t)256 * scratchTiles)) || (e = dalloc(s.glob, SORT_GLOB_WORDS)))
         return e;
     // glob: [p*256 + d] digit histograms -> offsets; [OS_MAXPASS*256 + p] tile counters
     if ((e = cudaMemsetAsync(s.glob.p, 0, SORT_GLOB_WORDS * sizeof(uint32_t), st))) return e;
-    const int hblocks = nTiles < num_sms() * 2 ? nTiles : num_sms() * 2;
+    const int hmax = (n + 4095) / 4096;
+    const int hblocks = hmax < num_sms() * 2 ? hmax : num_sms() * 2;
     os_histogram<<<hblocks, 512, 0, st>>>(s.k0.p, n, d_n, passes, s.glob.p); skid::note_launch();
-    os_offsets<<<1, 256, 0, st>>>(s.glob.p, passes); skid::note_launch();
+    os_offsets<<<passes, 256, 0, st>>>(s.glob.p); skid::note_launch();
     for (int p = 0; p < passes; ++p) {
         if ((e = cudaMemsetAsync(s.hist.p, 0, (size_t)256 * nTiles * sizeof(uint32_t), st)))
             return e;
-        os_pass<<<nTiles, RS_THREADS, 0, st>>>(s.k0.p, s.v0.p, s.k1.p, s.v1.p, n, d_n, 8 * p,
-                                                s.glob.p + 256 * p, s.hist.p,
-                                                s.glob.p + OS_MAXPASS * 256 + p, s.d_err); skid::note_launch();
+        uint32_t *off = s.glob.p + 256 * p, *ctr = s.glob.p + OS_MAXPASS * 256 + p;
+        if (few)
+            os_pass<RS_ROUNDS_FEW><<<nTiles, RS_THREADS, 0, st>>>(s.k0.p, s.v0.p, s.k1.p, s.v1.p, n, d_n, 8 * p,
+                                                                 off, s.hist.p, ctr, s.d_err);
+        else
+            os_pass<RS_ROUNDS_MANY><<<nTiles, RS_THREADS, 0, st>>>(s.k0.p, s.v0.p, s.k1.p, s.v1.p, n, d_n, 8 * p,
+                                                                  off, s.hist.p, ctr, s.d_err);
+        skid::note_launch();
         std::swap(s.k0, s.k1);
         std::swap(s.v0, s.v1);
     }
