@@ -330,56 +330,75 @@ __global__ void prep_members(const int *__restrict__ members, const int *__restr
     }
 }
 
-// Scoop: ungrouped particles within fScoop of each group's centre.
-// pass 0 counts, pass 1 fills (offsets from an exclusive scan).
-__global__ void scoop_kernel(TreeView t, const float *__restrict__ usoft,
-                             const skid_group *__restrict__ rec, const int *__restrict__ gcount,
-                             int ng, int nmax, float fBall2, float3 L, float3 hL, bool per,
-                             int pass, int *__restrict__ cnt, const int *__restrict__ off,
-                             float4 *__restrict__ list, float *__restrict__ lsoft)
+// Scoop: ungrouped particles within fScoop of each group's centre, a warp per
+// group.  pass 0 counts, pass 1 fills (offsets from an exclusive scan), in the
+// order of the sorted particles.
+//
+// The walk is one chain of dependent loads: with a thread per group the
+// slowest lane's whole walk, its leaves' particles one by one.  A warp tests
+// the last 2^subShift leaves of a subtree one per lane, then a leaf's
+// particles one per lane, and counts with ballots: 300 groups over
+// 400,000 particles 650 to 27 us, both passes.
+constexpr int SCOOP_THREADS = 128;
+
+__global__ void __launch_bounds__(SCOOP_THREADS)
+scoop_kernel(TreeView t, const float *__restrict__ usoft, const skid_group *__restrict__ rec,
+             const int *__restrict__ gcount, int ng, int nmax, float fBall2, float3 L, float3 hL,
+             bool per, int subShift, int pass, int *__restrict__ cnt, const int *__restrict__ off,
+             float4 *__restrict__ list, float *__restrict__ lsoft)
 {
+    const int lane = threadIdx.x & 31;
+    const int rootLo = t.leafBase >> subShift;
     // every entry is written, group 0 (the ungrouped particles) with 0: the
     // counts are scanned into offsets as a whole
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
+    const int nwarps = gridDim.x * (SCOOP_THREADS / 32);
+    for (int g = (blockIdx.x * SCOOP_THREADS + threadIdx.x) >> 5; g < ng; g += nwarps) {
         int c = 0;
-        int n = gcount[g];
+        const int n = gcount[g];
         if (g > 0 && n > 0 && n < nmax && t.n > 0) {
             const float *cen = rec[g].rCenter;
             const float *rel = rec[g].rel;
-            float3 q = make_float3(cen[0], cen[1], cen[2]);
-            int o = pass ? off[g] : 0;
+            const float3 q = make_float3(cen[0], cen[1], cen[2]);
+            const int o = pass ? off[g] : 0;
             int cp = 1;
             for (;;) {
-                float4 blo = t.lo[cp], bhi = t.hi[cp];
-                if (box_lb(q, blo, bhi, L, per) < fBall2) {
-                    if (cp < t.leafBase) { cp <<= 1; continue; }
-                    int b = (cp - t.leafBase) * SKID_LEAF, e = min(b + SKID_LEAF, t.n);
-                    for (int j = b; j < e; ++j) {
-                        float4 p = t.pos[j];
-                        float d2 = d2of(img_dx(q.x, p.x, L.x, hL.x), img_dx(q.y, p.y, L.y, hL.y),
-                                        img_dx(q.z, p.z, L.z, hL.z));
-                        if (d2 < fBall2) {
-                            if (pass) {
-                                // grav.c:103-111
-                                float nx = fsub(p.x, rel[0]), ny = fsub(p.y, rel[1]), nz = fsub(p.z, rel[2]);
-                                if (nx > hL.x) nx = fsub(nx, L.x);
-                                if (nx <= -hL.x) nx = fadd(nx, L.x);
-                                if (ny > hL.y) ny = fsub(ny, L.y);
-                                if (ny <= -hL.y) ny = fadd(ny, L.y);
-                                if (nz > hL.z) nz = fsub(nz, L.z);
-                                if (nz <= -hL.z) nz = fadd(nz, L.z);
-                                list[o + c] = make_float4(nx, ny, nz, p.w);
-                                lsoft[o + c] = usoft[j];
-                            }
-                            ++c;
+                if (cp < rootLo) {
+                    if (box_lb(q, t.lo[cp], t.hi[cp], L, per) < fBall2) { cp <<= 1; continue; }
+                } else {
+                    const int leaf = (cp << subShift) + lane;
+                    const bool near = lane < (1 << subShift) && leaf - t.leafBase < t.nLeaf &&
+                                      box_lb(q, t.lo[leaf], t.hi[leaf], L, per) < fBall2;
+                    for (unsigned lm = __ballot_sync(SKID_FULL, near); lm; lm &= lm - 1) {
+                        const int j = ((cp << subShift) + __ffs(lm) - 1 - t.leafBase) * SKID_LEAF + lane;
+                        float4 p;
+                        bool in = false;
+                        if (j < t.n) {
+                            p = t.pos[j];
+                            in = d2of(img_dx(q.x, p.x, L.x, hL.x), img_dx(q.y, p.y, L.y, hL.y),
+                                      img_dx(q.z, p.z, L.z, hL.z)) < fBall2;
                         }
+                        const unsigned m = __ballot_sync(SKID_FULL, in);
+                        if (pass && in) {
+                            // grav.c:103-111
+                            float nx = fsub(p.x, rel[0]), ny = fsub(p.y, rel[1]), nz = fsub(p.z, rel[2]);
+                            if (nx > hL.x) nx = fsub(nx, L.x);
+                            if (nx <= -hL.x) nx = fadd(nx, L.x);
+                            if (ny > hL.y) ny = fsub(ny, L.y);
+                            if (ny <= -hL.y) ny = fadd(ny, L.y);
+                            if (nz > hL.z) nz = fsub(nz, L.z);
+                            if (nz <= -hL.z) nz = fadd(nz, L.z);
+                            const int k = o + c + __popc(m & ((1u << lane) - 1u));
+                            list[k] = make_float4(nx, ny, nz, p.w);
+                            lsoft[k] = usoft[j];
+                        }
+                        c += __popc(m);
                     }
                 }
                 cp = next_node(cp);
                 if (cp == 1) break;
             }
         }
-        if (!pass) cnt[g] = c;
+        if (!pass && lane == 0) cnt[g] = c;
     }
 }
 
@@ -2085,9 +2104,12 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
     // scoop lists
     float fBall2 = P.fScoop * P.fScoop;
     float3 hL = make_float3(0.5f * P.period.x, 0.5f * P.period.y, 0.5f * P.period.z);
-    scoop_kernel<<<grid_for(ng), 256, 0, st>>>(ut.view(), U.usoft.p, G.rec.p, G.count.p, ng, P.nmax,
-                                              fBall2, P.period, hL, P.per, 0, U.scnt.p, nullptr,
-                                              nullptr, nullptr); note_launch();
+    int subShift = 0;
+    while (subShift < 5 && (2 << subShift) <= ut.leafBase) ++subShift;
+    const int scoopBlocks = grid_for(ng, SCOOP_THREADS / 32);
+    scoop_kernel<<<scoopBlocks, SCOOP_THREADS, 0, st>>>(ut.view(), U.usoft.p, G.rec.p, G.count.p, ng, P.nmax,
+                                                        fBall2, P.period, hL, P.per, subShift, 0, U.scnt.p,
+                                                        nullptr, nullptr, nullptr); note_launch();
     if ((e = scan_exclusive(U.scnt.p, U.soff.p, ng, U.cnt.p, ss, st))) return e;
     int nscoop = 0;
     if ((e = cudaMemcpyAsync(&nscoop, U.cnt.p, sizeof(int), cudaMemcpyDeviceToHost, st))) return e;
@@ -2095,9 +2117,9 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
     if ((e = dalloc(U.slist, nscoop > 0 ? nscoop : 1)) || (e = dalloc(U.ssoft, nscoop > 0 ? nscoop : 1)))
         return e;
     if (nscoop > 0)
-        scoop_kernel<<<grid_for(ng), 256, 0, st>>>(ut.view(), U.usoft.p, G.rec.p, G.count.p, ng,
-                                                  P.nmax, fBall2, P.period, hL, P.per, 1, U.scnt.p,
-                                                  U.soff.p, U.slist.p, U.ssoft.p); note_launch();
+        scoop_kernel<<<scoopBlocks, SCOOP_THREADS, 0, st>>>(ut.view(), U.usoft.p, G.rec.p, G.count.p, ng, P.nmax,
+                                                            fBall2, P.period, hL, P.per, subShift, 1, U.scnt.p,
+                                                            U.soff.p, U.slist.p, U.ssoft.p); note_launch();
     // groups by descending size
     if ((e = dalloc(ss.k0, ng)) || (e = dalloc(ss.v0, ng)) || (e = dalloc(ss.k1, ng)) ||
         (e = dalloc(ss.v1, ng)))
