@@ -239,13 +239,25 @@ density_adjoint_walk(TreeView t, const float *__restrict__ ball2, const float *_
 }
 
 // Gather every ball's members (distance^2 <= fBall2, the kNN set with its
-// ties) into rows of `cap` sorted-order indices.
+// ties) into rows of `cap` sorted-order indices, each in sorted order.
+//
+// Instruction issue bounds it.  The walk goes as in the density gather: the
+// last 2^subShift leaves of a subtree one per lane against the query leaf's
+// box, then a leaf's particles one per lane against that box and the largest
+// ball of the query leaf.  Where no periodic image can be nearer the survivors
+// are tested two to a packed FP32 operation into a mask per lane, from which
+// the lane writes its members: 100,000 points, k = 64, 539 to 235 us.
 __global__ void __launch_bounds__(A_WARPS * 32)
-ball_lists(TreeView t, const float *__restrict__ ball2, float3 L, float3 hL, bool per, int cap,
-           int *__restrict__ nbr, int *__restrict__ ncnt, int *work, unsigned *status)
+ball_lists(TreeView t, const float *__restrict__ ball2, float3 L, float3 hL, bool per, int subShift,
+           float zero_arg, int cap, int *__restrict__ nbr, int *__restrict__ ncnt, int *work,
+           unsigned *status)
 {
-    __shared__ float4 cpos[A_WARPS][SKID_LEAF];
+    __shared__ __align__(16) float cand_s[A_WARPS][3][SKID_LEAF];
+    __shared__ int slot_s[A_WARPS][SKID_LEAF];
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float (*cs)[SKID_LEAF] = cand_s[w];
+    const int rootLo = t.leafBase >> subShift;
+    const f32x2 zero = pack2(zero_arg, zero_arg), neg1 = pack2(-1.0f, -1.0f);
     for (;;) {
         int leaf = 0;
         if (lane == 0) leaf = atomicAdd(work, 1);
@@ -256,33 +268,85 @@ ball_lists(TreeView t, const float *__restrict__ ball2, float3 L, float3 hL, boo
         bool valid = qi < t.n;
         float4 qp = t.pos[valid ? qi : base];
         float3 q = make_float3(qp.x, qp.y, qp.z);
-        float bi = ball2[valid ? qi : base];
+        float bi = valid ? ball2[qi] : -1.0f;
+        // the query leaf's box and its largest ball
+        const float4 qlo = t.lo[t.leafBase + leaf], qhi = t.hi[t.leafBase + leaf];
+        const float bmax = __uint_as_float(__reduce_max_sync(SKID_FULL, __float_as_uint(fmaxf(bi, 0.0f))));
+        const f32x2 nqx = pack2(-q.x, -q.x), nqy = pack2(-q.y, -q.y), nqz = pack2(-q.z, -q.z);
+        const f32x2 b2 = pack2(bi, bi);
         int c = 0;
         int *row = nbr + (size_t)(valid ? qi : 0) * cap;
         int cp = 1;
         for (;;) {
-            float4 blo = t.lo[cp], bhi = t.hi[cp];
-            bool want = valid && box_lb(q, blo, bhi, L, per) <= bi;
-            if (__any_sync(SKID_FULL, want)) {
-                if (cp < t.leafBase) { cp <<= 1; continue; }
-                int lf = cp - t.leafBase;
-                if (lf < t.nLeaf) {
-                    int cb = lf * SKID_LEAF;
-                    int cnt = min(SKID_LEAF, t.n - cb);
+            const float4 nlo = t.lo[cp], nhi = t.hi[cp];
+            const bool dnode = !per || boxes_direct(qlo, qhi, nlo, nhi, hL);
+            if (cp < rootLo) {
+                if ((dnode ? gap2(xyz(qlo), xyz(qhi), nlo, nhi) : boxbox_lb(qlo, qhi, nlo, nhi, L, per)) <= bmax) {
+                    cp <<= 1;
+                    continue;
+                }
+            } else {
+                const int first = cp << subShift;
+                bool pass = false;
+                if (lane < (1 << subShift) && first + lane - t.leafBase < t.nLeaf) {
+                    const float4 bl = t.lo[first + lane], bh = t.hi[first + lane];
+                    pass = (dnode ? gap2(xyz(qlo), xyz(qhi), bl, bh) : boxbox_lb(qlo, qhi, bl, bh, L, per)) <= bmax;
+                }
+                for (unsigned lm = __ballot_sync(SKID_FULL, pass); lm; lm &= lm - 1) {
+                    const int node = first + __ffs(lm) - 1;
+                    const float4 blo = t.lo[node], bhi = t.hi[node];
+                    const bool direct = dnode || boxes_direct(qlo, qhi, blo, bhi, hL);
+                    const bool want = (direct ? gap2(q, q, blo, bhi) : box_lb(q, blo, bhi, L, per)) <= bi;
+                    if (!__any_sync(SKID_FULL, want)) continue;
+                    const int cb = (node - t.leafBase) * SKID_LEAF;
+                    bool rel = false;
+                    float4 cj = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (cb + lane < t.n) {
+                        cj = t.pos[cb + lane];
+                        rel = (direct ? gap2(xyz(cj), xyz(cj), qlo, qhi) : box_lb(xyz(cj), qlo, qhi, L, per)) <= bmax;
+                    }
+                    const unsigned R = __ballot_sync(SKID_FULL, rel);
+                    if (R == 0) continue;
+                    const int nR = __popc(R);
+                    const int rank = __popc(R & ((1u << lane) - 1u));
+                    // survivors in reverse order of rank, so that the first
+                    // member is the highest bit; above them no members
+                    const int slot = rel ? nR - 1 - rank : nR + lane - rank;
                     __syncwarp();
-                    if (lane < cnt) cpos[w][lane] = t.pos[cb + lane];
+                    cs[0][slot] = rel ? cj.x : INFINITY;
+                    cs[1][slot] = cj.y;
+                    cs[2][slot] = cj.z;
+                    slot_s[w][slot] = cb + lane;
                     __syncwarp();
-                    if (want) {
-                        for (int j = 0; j < cnt; ++j) {
-                            float4 cj = cpos[w][j];
-                            float d = per ? d2of(img_dx(q.x, cj.x, L.x, hL.x), img_dx(q.y, cj.y, L.y, hL.y),
-                                                 img_dx(q.z, cj.z, L.z, hL.z))
-                                          : d2of(fsub(q.x, cj.x), fsub(q.y, cj.y), fsub(q.z, cj.z));
-                            if (d <= bi) {
-                                if (c < cap) row[c] = cb + j;
-                                ++c;
+                    unsigned in = 0;
+                    if (direct) {
+                        unsigned out = 0;
+                        for (int j = (nR - 1) & ~3; j >= 0; j -= 4) {
+                            const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&cs[0][j]);
+                            const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&cs[1][j]);
+                            const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(&cs[2][j]);
+#pragma unroll
+                            for (int h = 1; h >= 0; --h) {
+                                const f32x2 dx = add2(h ? X.y : X.x, nqx), dy = add2(h ? Y.y : Y.x, nqy),
+                                            dz = add2(h ? Z.y : Z.x, nqz);
+                                const f32x2 d = add2(add2(sq2(dx, zero), sq2(dy, zero)), sq2(dz, zero));
+                                const float2 a = unpack2(fma2(d, neg1, b2));   // negative: outside
+                                out = __funnelshift_l(__float_as_uint(a.y), out, 1);
+                                out = __funnelshift_l(__float_as_uint(a.x), out, 1);
                             }
                         }
+                        in = ~out & (nR < 32 ? (1u << nR) - 1u : ~0u);
+                    } else if (want) {
+                        for (int j = 0; j < nR; ++j) {
+                            const float d = d2of(img_dx(q.x, cs[0][j], L.x, hL.x), img_dx(q.y, cs[1][j], L.y, hL.y),
+                                                 img_dx(q.z, cs[2][j], L.z, hL.z));
+                            if (d <= bi) in |= 1u << j;
+                        }
+                    }
+                    for (; in; ++c) {
+                        const int j = 31 - __clz(in);
+                        in ^= 1u << j;
+                        if (c < cap) row[c] = slot_s[w][j];
                     }
                 }
             }
@@ -766,6 +830,8 @@ cudaError_t density_adjoint(const Tree &t, const float *ball2_sorted, const int 
     gather_w<<<grid_for(ns), 256, 0, st>>>(sidx, w_io, ns, A.w.p); note_launch();
     float3 hL = make_float3(0.5f * L.x, 0.5f * L.y, 0.5f * L.z);
     int need = (t.nLeaf + A_WARPS - 1) / A_WARPS;
+    int subShift = 0;
+    while (subShift < 5 && (2 << subShift) <= t.leafBase) ++subShift;
     if (mode == 2) {
         // store the lists only while they take at most a quarter of the free memory
         size_t fr = 0, tot = 0;
@@ -778,8 +844,6 @@ cudaError_t density_adjoint(const Tree &t, const float *ball2_sorted, const int 
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, density_adjoint_walk, A_WARPS * 32, 0);
         int blocks = num_sms() * (perSM > 0 ? perSM : 1);
         if (blocks > need) blocks = need;
-        int subShift = 0;
-        while (subShift < 5 && (2 << subShift) <= t.leafBase) ++subShift;
         density_adjoint_walk<<<blocks, A_WARPS * 32, 0, st>>>(t.view(), ball2_sorted, A.w.p, L, hL, per,
                                                              subShift, A.g.p, d_work, d_status); note_launch();
     } else {
@@ -791,7 +855,7 @@ cudaError_t density_adjoint(const Tree &t, const float *ball2_sorted, const int 
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, ball_lists, A_WARPS * 32, 0);
             int blocks = num_sms() * (perSM > 0 ? perSM : 1);
             if (blocks > need) blocks = need;
-            ball_lists<<<blocks, A_WARPS * 32, 0, st>>>(t.view(), ball2_sorted, L, hL, per, A.cap,
+            ball_lists<<<blocks, A_WARPS * 32, 0, st>>>(t.view(), ball2_sorted, L, hL, per, subShift, 0.0f, A.cap,
                                                        A.nbr.p, A.ncnt.p, d_work, d_status); note_launch();
             A.lists = true;
         }
