@@ -252,7 +252,6 @@ float skid_ctx::timer_stop()
 
 FieldArgs skid_ctx::field_args(float fStep, bool initial, float *acc_out)
 {
-    (void)initial;
     FieldArgs a;
     a.zero = 0.0f;
     a.cpos = C.cpos.p;
@@ -271,7 +270,8 @@ FieldArgs skid_ctx::field_args(float fStep, bool initial, float *acc_out)
     a.wrapHi = wrap_hi();
     a.wrapLo = wrap_lo();
     a.acc_out = acc_out;
-    a.touched = C.touched.p;
+    a.touched = initial ? C.touched.p : nullptr;   // only the first step's cut asks per copy
+    a.floor = C.d_floor;
     a.d_work = d_scal + SC_WORK;
     a.d_status = d_status;
     a.stats = field_stats_on ? d_fstats : nullptr;
@@ -305,7 +305,8 @@ int skid_ctx::enqueue_step(float fStep, bool initial, bool nocut, int slot, int 
     }
     CK(cudaEventRecordWithFlags(fev[2 * slot + 1], st, evflags));
     CK(scatter_cut(C, initial, nocut, rho_final.p, M.d_nA, d_fbytes, compact, st));
-    CK(tree_refit(ctree, C.cpos.p, nullptr, C.d_n, st, true, C.d_dirty));
+    // (a step without a compaction leaves the tree's boxes as they are)
+    if (compact && !nocut) CK(tree_refit(ctree, C.cpos.p, nullptr, C.d_n, st, true, C.d_dirty));
     // between prunes, re-sort the active movers while they are many (16 or
     // more per warp): the warps' boxes stay tight as the movers drift
     if (!compact && G >= 16) CK(mover_resort(M, mkey_lo, mkey_inv, ss, st, slot_bound(G), opt_curve & 1));
@@ -365,8 +366,8 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
     a.stats = nullptr;
     a.part_acc = nullptr;   // a probe walks each position in one warp
     a.part_cnt = nullptr;
-    a.touched = ctx->probe_touched();
-    if (!a.touched) return ctx->fail(SKID_ENOMEM);
+    a.touched = nullptr;
+    a.floor = nullptr;
     CK(field_move(a, nm, st));
     if (nm > 0) {
         unsort_xyz<<<grid_for(nm), 256, 0, st>>>(act.p, xyz.p, nm, ctx->probe_acc.p); skid::note_launch();

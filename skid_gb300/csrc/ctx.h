@@ -248,7 +248,6 @@ struct skid_ctx {
     skid::DBuf<float> probe_f, probe_acc;
     skid::DBuf<float4> probe_p4;
     skid::DBuf<int> probe_i, probe_i2;
-    skid::DBuf<unsigned char> probe_t;
     skid::DBuf<uint32_t> tipsy_raw;   // TIPSY record words as read (skid_set_tipsy)
     skid::DBuf<int> stat_start;      // .stat: first sorted slot of each group
     skid::DBuf<skid_stat> stat_out;  // .stat: per-group columns
@@ -340,13 +339,6 @@ struct skid_ctx {
     }
     void collect_field_times(int nslots);
 
-    unsigned char *probe_touched()
-    {
-        size_t need = C.cap > 0 ? C.cap : 1;
-        if (skid::dalloc(probe_t, need)) return nullptr;
-        return probe_t.p;
-    }
-
     void reset_pipeline()
     {
         // the move-iteration graphs stay: skid_move_iterate replays one only
@@ -425,7 +417,7 @@ struct skid_ctx {
         dfree(ss.k0); dfree(ss.k1); dfree(ss.v0); dfree(ss.v1); dfree(ss.hist); dfree(ss.glob); dfree(ss.blk);
         dfree(ss.box);
         dfree(probe_f); dfree(probe_acc); dfree(probe_p4); dfree(probe_i); dfree(probe_i2);
-        dfree(probe_t); dfree(stat_start); dfree(stat_out); dfree(tipsy_raw); dfree(knn_heap); dfree(split_acc); dfree(split_cnt); dfree(ms_dev);
+        dfree(stat_start); dfree(stat_out); dfree(tipsy_raw); dfree(knn_heap); dfree(split_acc); dfree(split_cnt); dfree(ms_dev);
         dfree(adj.win); dfree(adj.w); dfree(adj.g); dfree(adj.out); dfree(adj.nbr); dfree(adj.ncnt);
         dfree(adj.slots); dfree(adj.rm); dfree(adj.re); dfree(adj.rio); dfree(adj.tbox); dfree(adj.acc); dfree(adj.E);
         std::lock_guard<std::recursive_mutex> lk(skid::device_mutex());

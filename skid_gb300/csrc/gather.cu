@@ -15,8 +15,8 @@
 // mover walks the scatterer tree (ball boxes) and sums the copies whose ball
 // holds it, then moves itself in the same kernel; a copy is the scatterer's
 // periodic image nearest the mover, x_c = fl(x + sL), and must be live.  The
-// warp marks which scatterers it touched (for the density floor of the cut,
-// smooth1.c:460-461).
+// warp keeps the least density of the scatterers that reached a mover (the
+// floor of the cut, smooth1.c:460-461).
 #include <cfloat>
 
 #include "internal.h"
@@ -263,6 +263,7 @@ field_kernel(FieldArgs a)
     __shared__ __align__(16) float cand_s[G_WARPS][4][SKID_LEAF];
     __shared__ float2 ccoef_s[G_WARPS][SKID_LEAF];
     __shared__ float4 box_s[G_WARPS][2 * NB];
+    __shared__ unsigned floor_s[G_WARPS][32];
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float (*cs)[SKID_LEAF] = cand_s[w];
     float2 *cc = ccoef_s[w];
@@ -279,6 +280,7 @@ field_kernel(FieldArgs a)
     const int nItems = G == 1 ? nA * S : (nA + G - 1) / G;
     const int sub = lane % L;
     unsigned long long st_nodes = 0, st_leaves = 0, st_tests = 0, st_hits = 0;
+    floor_s[w][lane] = 0xffffffffu;
     for (;;) {
         int item = 0;
         if (lane == 0) item = atomicAdd(a.d_work, 1);
@@ -498,10 +500,14 @@ field_kernel(FieldArgs a)
                 if (STATS) st_hits += __popc(m);
                 for (; m; m &= m - 1) add_term(0, __ffs(m) - 1);
             }
-            // copies that reached a mover: touched, and their density
-            // enters the floor of the cut (smooth1.c:460-461)
+            // copies that reached a mover: their density enters the floor of
+            // the cut (smooth1.c:460-461), the lane's least one in shared
+            // memory (a register more in this loop costs more than it)
             unsigned any = __reduce_or_sync(SKID_FULL, hitany);
-            if (rel && ((any >> slot_r) & 1u)) a.touched[cb + lane] = 1;
+            if (rel && ((any >> slot_r) & 1u)) {
+                floor_s[w][lane] = min(floor_s[w][lane], f2ord(a.ccoef[cb + lane].z));
+                if (a.touched) a.touched[cb + lane] = 1;
+            }
         };
         // The leaves that pass under one node, in order; the next one's
         // copies are loaded while one is worked on.
@@ -607,6 +613,10 @@ field_kernel(FieldArgs a)
                 a.mpos[mi[k]] = make_float4(yk.x, yk.y, yk.z, yp[k].w);
             }
         }
+    }
+    if (a.floor) {
+        const unsigned least = __reduce_min_sync(SKID_FULL, floor_s[w][lane]);
+        if (lane == 0 && least < *(volatile unsigned *)a.floor) atomicMin(a.floor, least);
     }
     if (STATS && a.stats) {
 #pragma unroll

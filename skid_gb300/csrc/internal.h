@@ -146,7 +146,7 @@ cudaError_t density_gather(const Tree &t, const float *ball2_sorted, float3 L, b
 struct CopyState {
     int cap = 0;
     DBuf<float4> cpos, ccoef, cpos2, ccoef2;
-    DBuf<unsigned char> touched;    // reached an active mover this step
+    DBuf<unsigned char> touched;    // reached an active mover in the first step
     DBuf<int> keep, kpos;
     DBuf<int> blk;                  // kept copies per cut tile
     DBuf<unsigned> mask;            // build-time image masks
@@ -155,14 +155,14 @@ struct CopyState {
     int *d_n2 = nullptr;            // live copies after the last cut
     unsigned *d_floor = nullptr;    // ordered-uint min density (fScatDens)
     int *d_dirty = nullptr;         // copies changed since the last refit
-    int *d_done = nullptr;          // finished write-back blocks (zero between steps)
+    int *d_done = nullptr;          // finished blocks of a cut or write-back (zero between steps)
     cudaError_t alloc(int n)
     {
         cudaError_t e;
         size_t m = n > 0 ? n : 1;
         if ((e = dalloc(cpos, m)) || (e = dalloc(ccoef, m)) || (e = dalloc(cpos2, m)) ||
             (e = dalloc(ccoef2, m)) || (e = dalloc(touched, m)) || (e = dalloc(keep, m)) ||
-            (e = dalloc(kpos, m)) || (e = dalloc(blk, (m + 4095) / 4096)))
+            (e = dalloc(kpos, m)) || (e = dalloc(blk, (m + 1023) / 1024)))
             return e;
         cap = (int)m;
         return cudaSuccess;
@@ -198,7 +198,8 @@ struct FieldArgs {
     float3 wrapHi, wrapLo;           // float thresholds of kdMoveParticles' wrap
     float3 period;
     float *acc_out;                  // optional [3*nA] field output (probe)
-    unsigned char *touched;          // per copy slot
+    unsigned char *touched;          // per copy slot: set where a copy reached a mover (or null)
+    unsigned *floor;                 // least density (ordered bits) of the copies that did (or null)
     int *d_work;
     unsigned *d_status;
     unsigned long long *stats;       // optional: nodes, leaves, candidate tests, hits
@@ -219,9 +220,10 @@ cudaError_t build_copies(const float4 *spos, const float *ball2, const float *rh
                          int ns, float3 L, float3 boxlo, float3 boxhi, bool periodic,
                          CopyState &C, SortScratch &ss, int *nCopies, cudaStream_t st,
                          bool hil = true);
-// After a move pass: density floor, cut, stable compaction, counts.
-// compact = false defers the compaction: cut copies stay marked in their
-// slots (empty ball, density -inf) and only the live count is published.
+// After a move pass, which left the density floor in C.d_floor: cut, stable
+// compaction, counts.  compact = false defers the compaction: cut copies stay
+// marked in their slots (empty ball, density -inf) and only the live count is
+// published.  *d_dirty is set only by a compaction that moved something.
 cudaError_t scatter_cut(CopyState &C, bool initial, bool nocut, float *final_rho, const int *d_nA,
                         double *d_fbytes, bool compact, cudaStream_t st);
 // Re-sort the active movers by the Hilbert (hil) or Morton key of their

@@ -122,14 +122,17 @@ __global__ void copy_permute_kernel(const uint32_t *__restrict__ perm, int n,
     }
 }
 
-// ---- the cut, in tiles of CT_TILE slots: keep flags and per-tile counts,
-// then each tile compacts itself from the counts before it ----
+// ---- the cut, in tiles: keep flags and per-tile counts, then each tile
+// compacts itself from the counts before it ----
 // A tile is CT_TILE slots for one block; warp w owns the CT_ITEMS x 32
 // consecutive slots from w * CT_WSPAN, read 32 at a time (coalesced), with
-// its in-tile offsets from ballots.
+// its in-tile offsets from ballots.  Up to some 150,000 slots a launch takes the
+// time of one tile, whose length is CT_ITEMS serial rounds: tiles of 4096 slots
+// against 1024 took 0.21 ms more of a 5,000-particle run's 6.0, 0.38 of 17.1 at
+// 150,000 and 0.27 of 69.3 at 2^21, so none of that size is left.
 constexpr int CT_THREADS = 256;
-constexpr int CT_ITEMS = 16;
-constexpr int CT_TILE = CT_THREADS * CT_ITEMS;   // matches the blk sizing (4096)
+constexpr int CT_ITEMS = 4;
+constexpr int CT_TILE = CT_THREADS * CT_ITEMS;   // matches the blk sizing (1024)
 constexpr int CT_WSPAN = CT_ITEMS * 32;
 
 __device__ __forceinline__ int ct_slot(int tile, int r)
@@ -164,58 +167,64 @@ __device__ __forceinline__ int warp_offset(int wc, int *sh)
     return before;
 }
 
-// The density floor over touched copies (smooth1.c:460-461).
-__global__ void floor_kernel(const float4 *__restrict__ ccoef,
-                             const unsigned char *__restrict__ touched, const int *d_n,
-                             unsigned *d_floor)
-{
-    int n = *d_n;
-    unsigned best = 0xffffffffu;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        if (touched[i]) best = min(best, f2ord(ccoef[i].z));
-    best = __reduce_min_sync(SKID_FULL, best);
-    if ((threadIdx.x & 31) == 0 && best != 0xffffffffu) atomicMin(d_floor, best);
-}
-
-// Keep flags (smooth1.c:460-470 with the floor over the touched copies), first-step zeroed densities, touched reset; per-tile kept
-// counts.  Block 0 also accumulates the step's algorithmic field bytes.
+// Keep flags against the density floor over the copies that reached a mover
+// (smooth1.c:460-470), first-step zeroed densities and touched reset, per-tile
+// kept counts.  Block 0 also accumulates the step's algorithmic field bytes.
+// When no compaction follows (publish), the last block to finish sums the
+// counts into *d_n2 and resets the floor for the next step; else the
+// compaction does, and the cut copies stay marked in their slots.
+//
+// A tile's loads come before any of its stores: one after the other, as the
+// stores' aliasing had them, a tile of 4096 slots took 7.6 us.  With the floor
+// found by the field kernel (the copies were read again for it), the
+// count published here and the refit left out where nothing moved, a step
+// between compactions is two launches in place of five: 5,000 particles' moving
+// 2.93 to 2.45 ms, 150,000 10.94 to 9.72, 2^21 41.2 to 39.8.
 __global__ void __launch_bounds__(CT_THREADS)
-cut_tiles_kernel(float4 *__restrict__ cpos, float4 *__restrict__ ccoef,
-                 unsigned char *__restrict__ touched, const int *d_n, const unsigned *d_floor,
-                 int initial, int nocut, int *__restrict__ keep, float *__restrict__ final_rho,
-                 int *__restrict__ blk, const int *d_nA, double *fbytes)
+cut_tiles_kernel(float4 *cpos, float4 *ccoef, unsigned char *touched, const int *d_n,
+                 unsigned *d_floor, int initial, int nocut, int publish, int *__restrict__ keep,
+                 float *__restrict__ final_rho, int *blk, int *d_n2, int *d_done, const int *d_nA,
+                 double *fbytes)
 {
     __shared__ int sh[32];
+    __shared__ int last;
     const int n = *d_n;
     const unsigned fl = *d_floor;
     const float fScatDens = fl == 0xffffffffu ? 0.0f : ord2f(fl);
     int kept = 0;
+    float4 c[CT_ITEMS];
+    bool t[CT_ITEMS];
+#pragma unroll
+    for (int j = 0; j < CT_ITEMS; ++j) {
+        const int i = ct_slot(blockIdx.x, j);
+        c[j] = i < n ? ccoef[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        t[j] = initial && i < n && touched[i] != 0;
+    }
+#pragma unroll
     for (int j = 0; j < CT_ITEMS; ++j) {
         const int i = ct_slot(blockIdx.x, j);
         if (i >= n) break;
-        float4 c = ccoef[i];
-        bool t = touched[i] != 0;
-        if (t) touched[i] = 0;
+        if (t[j]) touched[i] = 0;
         int k = 1;
         if (!nocut) {
             if (initial) {
-                unsigned bits = __float_as_uint(c.w);
-                if (!t && (bits & ORIG_FLAG) && final_rho) final_rho[bits & ~ORIG_FLAG] = 0.0f;
+                unsigned bits = __float_as_uint(c[j].w);
+                if (!t[j] && (bits & ORIG_FLAG) && final_rho) final_rho[bits & ~ORIG_FLAG] = 0.0f;
                 // a copy that reached no mover counts as density 0 (smooth1.c:463-470)
-                float r = t ? c.z : 0.0f;
+                float r = t[j] ? c[j].z : 0.0f;
                 k = r >= fScatDens;
             } else {
-                k = c.z >= fScatDens;
+                k = c[j].z >= fScatDens;
             }
             // a copy cut now stays in its slot until the next compaction: an
             // empty ball (no mover is inside it) and density -inf (never
             // kept again)
-            if (!k && c.z != -INFINITY) {
+            if (!k && c[j].z != -INFINITY) {
                 cpos[i].w = 0.0f;
                 ccoef[i].z = -INFINITY;
             }
         }
-        keep[i] = k;
+        if (!publish) keep[i] = k;
         kept += k;
     }
     kept = block_sum(kept, sh);
@@ -225,19 +234,34 @@ cut_tiles_kernel(float4 *__restrict__ cpos, float4 *__restrict__ ccoef,
             fbytes[0] += 24.0 * (double)*d_nA + 20.0 * (double)n;
             fbytes[1] += 1.0;
         }
+        if (publish) {
+            __threadfence();
+            last = atomicAdd(d_done, 1) == (int)gridDim.x - 1;
+        }
+    }
+    if (!publish) return;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    int all = 0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += CT_THREADS) all += __ldcg(&blk[k]);
+    all = block_sum(all, sh);
+    if (threadIdx.x == 0) {
+        *d_n2 = all;
+        *d_floor = 0xffffffffu;
+        *d_done = 0;
     }
 }
 
 // Stable compaction into the spare arrays: tile b starts at the sum of the
 // counts of tiles before it.  Block 0 publishes the live count in *d_n2 and
 // resets the density floor for the next step.  Nothing is written when
-// nothing was cut, or when compaction is deferred (compact = 0, one block:
-// the cut copies stay marked in their slots).
+// nothing was cut.
 __global__ void __launch_bounds__(CT_THREADS)
 compact_tiles_kernel(const int *__restrict__ keep, const int *__restrict__ blk, int nb,
-                     const int *d_n, int *d_n2, unsigned *d_floor, int compact,
-                     const float4 *__restrict__ cpos, const float4 *__restrict__ ccoef,
-                     float4 *__restrict__ cpos2, float4 *__restrict__ ccoef2)
+                     const int *d_n, int *d_n2, unsigned *d_floor, const float4 *__restrict__ cpos,
+                     const float4 *__restrict__ ccoef, float4 *__restrict__ cpos2,
+                     float4 *__restrict__ ccoef2)
 {
     __shared__ int sh[32];
     const int n = *d_n;
@@ -254,7 +278,7 @@ compact_tiles_kernel(const int *__restrict__ keep, const int *__restrict__ blk, 
         *d_n2 = all;
         *d_floor = 0xffffffffu;
     }
-    if (!compact || all == n) return;
+    if (all == n) return;
     const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
     unsigned m[CT_ITEMS];
     int wc = 0;
@@ -312,12 +336,19 @@ prune_flag_kernel(const float4 *__restrict__ mpos, const float4 *__restrict__ mo
     __shared__ int sh[32];
     const int n = *d_nA;
     int kept = 0;
+    float4 r[CT_ITEMS], o[CT_ITEMS];
+#pragma unroll
+    for (int j = 0; j < CT_ITEMS; ++j) {
+        const int i = ct_slot(blockIdx.x, j);
+        const int m = i < n ? act[i] : -1;
+        r[j] = m >= 0 ? mpos[m] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        o[j] = m >= 0 ? mold[m] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
     for (int j = 0; j < CT_ITEMS; ++j) {
         const int i = ct_slot(blockIdx.x, j);
         if (i >= n) break;
-        int m = act[i];
-        float4 r = mpos[m], o = mold[m];
-        float dx = fsub(r.x, o.x), dy = fsub(r.y, o.y), dz = fsub(r.z, o.z);
+        float dx = fsub(r[j].x, o[j].x), dy = fsub(r[j].y, o[j].y), dz = fsub(r[j].z, o[j].z);
         if (dx > hP.x) dx = fsub(dx, fmul(2.0f, hP.x));
         if (dx <= -hP.x) dx = fadd(dx, fmul(2.0f, hP.x));
         if (dy > hP.y) dy = fsub(dy, fmul(2.0f, hP.y));
@@ -459,20 +490,14 @@ cudaError_t scatter_cut(CopyState &C, bool initial, bool nocut, float *final_rho
 {
     const int nb = (C.cap + CT_TILE - 1) / CT_TILE;
     if (C.blk.n < (size_t)nb) return cudaErrorInvalidValue;
-    floor_kernel<<<grid_for(C.cap), 256, 0, st>>>(C.ccoef.p, C.touched.p, C.d_n, C.d_floor); skid::note_launch();
+    const bool publish = nocut || !compact;
     cut_tiles_kernel<<<nb, CT_THREADS, 0, st>>>(C.cpos.p, C.ccoef.p, C.touched.p, C.d_n, C.d_floor,
-                                                initial ? 1 : 0, nocut ? 1 : 0, C.keep.p, final_rho,
-                                                C.blk.p, d_nA, d_fbytes); skid::note_launch();
+                                                initial ? 1 : 0, nocut ? 1 : 0, publish ? 1 : 0, C.keep.p,
+                                                final_rho, C.blk.p, C.d_n2, C.d_done, d_nA, d_fbytes); skid::note_launch();
     cudaError_t e = cudaGetLastError();
-    if (e) return e;
-    if (nocut) {
-        if ((e = cudaMemsetAsync(C.d_floor, 0xff, sizeof(unsigned), st))) return e;
-        return cudaMemcpyAsync(C.d_n2, C.d_n, sizeof(int), cudaMemcpyDeviceToDevice, st);
-    }
-    compact_tiles_kernel<<<compact ? nb : 1, CT_THREADS, 0, st>>>(C.keep.p, C.blk.p, nb, C.d_n, C.d_n2,
-                                                                  C.d_floor, compact ? 1 : 0, C.cpos.p,
-                                                                  C.ccoef.p, C.cpos2.p, C.ccoef2.p); skid::note_launch();
-    if (!compact) return cudaGetLastError();
+    if (e || publish) return e;
+    compact_tiles_kernel<<<nb, CT_THREADS, 0, st>>>(C.keep.p, C.blk.p, nb, C.d_n, C.d_n2, C.d_floor, C.cpos.p,
+                                                    C.ccoef.p, C.cpos2.p, C.ccoef2.p); skid::note_launch();
     copyback_tiles_kernel<<<grid_for(C.cap), 256, 0, st>>>(C.d_n, C.d_n2, C.cpos.p, C.ccoef.p, C.cpos2.p,
                                                            C.ccoef2.p, C.d_dirty, C.d_done); skid::note_launch();
     return cudaGetLastError();
