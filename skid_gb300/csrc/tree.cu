@@ -15,7 +15,10 @@ namespace skid {
 
 namespace {
 
-__global__ void bbox_kernel(const float4 *__restrict__ p, int n, unsigned *box)
+constexpr int BBOX_THREADS = 256;
+
+__global__ void __launch_bounds__(BBOX_THREADS)
+bbox_kernel(const float4 *__restrict__ p, int n, unsigned *box)
 {
     float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -24,19 +27,27 @@ __global__ void bbox_kernel(const float4 *__restrict__ p, int n, unsigned *box)
         mn[1] = fminf(mn[1], q.y); mx[1] = fmaxf(mx[1], q.y);
         mn[2] = fminf(mn[2], q.z); mx[2] = fmaxf(mx[2], q.z);
     }
+    // one set of atomics a block: a set a warp, six addresses for all of
+    // them, took 15 us at 100,000 points, this 2.7
+    __shared__ unsigned smn[3][BBOX_THREADS / 32], smx[3][BBOX_THREADS / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            mn[d] = fminf(mn[d], __shfl_xor_sync(SKID_FULL, mn[d], o));
-            mx[d] = fmaxf(mx[d], __shfl_xor_sync(SKID_FULL, mx[d], o));
+        const unsigned a = __reduce_min_sync(SKID_FULL, f2ord(mn[d])), b = __reduce_max_sync(SKID_FULL, f2ord(mx[d]));
+        if (lane == 0) {
+            smn[d][w] = a;
+            smx[d][w] = b;
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int d = 0; d < 3; ++d) {
-            atomicMin(&box[d], f2ord(mn[d]));
-            atomicMax(&box[3 + d], f2ord(mx[d]));
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        unsigned a = smn[lane][0], b = smx[lane][0];
+        for (int i = 1; i < BBOX_THREADS / 32; ++i) {
+            a = min(a, smn[lane][i]);
+            b = max(b, smx[lane][i]);
         }
+        atomicMin(&box[lane], a);
+        atomicMax(&box[3 + lane], b);
     }
 }
 
@@ -65,80 +76,152 @@ __global__ void gather_sorted(const float4 *__restrict__ p, const uint32_t *__re
     }
 }
 
-// One thread per leaf slot: leaf boxes, then a last-arriver walk up the heap.
-// ball2 (sorted order) builds ball boxes when given; aux (sorted order, x =
-// ball2, w = live-copy mask bits) is the alternative source for refits.
-__global__ void upward_kernel(const float4 *__restrict__ pos, const float *__restrict__ ball2,
-                              const float4 *__restrict__ aux, int ballw, int n_host, const int *d_n,
-                              int leafBase, float4 *lo, float4 *hi, float4 *blo, float4 *bhi,
-                              int *flag, int *d_dirty)
+// A node's box and ball box.
+struct NodeBox {
+    float3 lo, hi, blo, bhi;
+    float b2;        // largest ball2
+};
+
+__device__ __forceinline__ float warp_min(float v) { return ord2f(__reduce_min_sync(SKID_FULL, f2ord(v))); }
+__device__ __forceinline__ float warp_max(float v) { return ord2f(__reduce_max_sync(SKID_FULL, f2ord(v))); }
+
+// One block per 32 leaves: each warp bounds leaves of one point per lane,
+// then one warp combines the 32 boxes up five levels.  The block that is the
+// last to finish below a node five levels further up combines those 32 in
+// turn, to the root.  ball2 (sorted order) builds ball boxes when given; aux
+// (sorted order, x = ball2, w = live-copy mask bits) is the alternative source
+// for refits.
+//
+// A chain of latencies bounds it: a thread per leaf reading its 32 points one
+// after the other, then an atomic and a fence per level, took 28.6 us a pass at
+// 100,000 points and 30 to 50 at 2^20; this 9.7 and 12 to 24.
+constexpr int UP_WARPS = 8;
+
+__global__ void __launch_bounds__(UP_WARPS * 32)
+upward_kernel(const float4 *__restrict__ pos, const float *__restrict__ ball2,
+              const float4 *__restrict__ aux, int ballw, int n_host, const int *d_n, int leafBase,
+              float4 *lo, float4 *hi, float4 *blo, float4 *bhi, int *flag, int *d_dirty)
 {
-    int leaf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (leaf >= leafBase) return;
+    __shared__ NodeBox leaf_s[32];
     if (d_dirty && !*d_dirty) return;
-    int n = d_n ? *d_n : n_host;
-    float4 l = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX);
-    float4 h = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f);
-    float4 bl = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f);
-    float4 bh = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int first = blockIdx.x * 32;
+    const int n = d_n ? *d_n : n_host;
     // max ball2 (lo.w) needs ball data; ball boxes also need allocated arrays
-    bool hasb = (ball2 != nullptr) || (aux != nullptr) || ballw;
-    bool balls = hasb && blo != nullptr && bhi != nullptr;
-    int b = leaf * SKID_LEAF, e = min(b + SKID_LEAF, n);
-    for (int i = b; i < e; ++i) {
-        float4 q = pos[i];
-        float b2 = 0.0f;
-        bool live = true;
-        if (ballw) {
-            b2 = q.w;
-        } else if (aux) {
-            float4 a = aux[i];
-            b2 = a.x;
-            live = __float_as_uint(a.w) != 0u;
-        } else if (ball2) {
-            b2 = ball2[i];
-        }
-        if (!live) continue;
-        l.x = fminf(l.x, q.x); l.y = fminf(l.y, q.y); l.z = fminf(l.z, q.z);
-        h.x = fmaxf(h.x, q.x); h.y = fmaxf(h.y, q.y); h.z = fmaxf(h.z, q.z);
-        if (hasb) l.w = fmaxf(l.w, b2);
+    const bool hasb = (ball2 != nullptr) || (aux != nullptr) || ballw;
+    const bool balls = hasb && blo != nullptr && bhi != nullptr;
+    auto store = [&](int node, const NodeBox &x) {
+        lo[node] = make_float4(x.lo.x, x.lo.y, x.lo.z, x.b2);
+        hi[node] = make_float4(x.hi.x, x.hi.y, x.hi.z, 0.0f);
         if (balls) {
-            // ball radius rounded up so the box contains every d2 < b2 point
-            float r = sqrtf(b2) * (1.0f + 1e-6f) + 1e-30f;
-            r += 4.8e-7f * (fabsf(q.x) + fabsf(q.y) + fabsf(q.z) + r);
-            bl.x = fminf(bl.x, q.x - r); bl.y = fminf(bl.y, q.y - r); bl.z = fminf(bl.z, q.z - r);
-            bh.x = fmaxf(bh.x, q.x + r); bh.y = fmaxf(bh.y, q.y + r); bh.z = fmaxf(bh.z, q.z + r);
+            blo[node] = make_float4(x.blo.x, x.blo.y, x.blo.z, 0.0f);
+            bhi[node] = make_float4(x.bhi.x, x.bhi.y, x.bhi.z, 0.0f);
         }
+    };
+    const float3 top = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), bottom = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+    const int leaves = min(32, leafBase - first);
+#pragma unroll
+    for (int r = 0; r < 32 / UP_WARPS; ++r) {
+        const int l = r * UP_WARPS + w, i = (first + l) * SKID_LEAF + lane;
+        NodeBox x;
+        x.lo = x.blo = top;
+        x.hi = x.bhi = bottom;
+        x.b2 = -FLT_MAX;
+        if (l < leaves && i < n) {
+            const float4 q = pos[i];
+            float b2 = 0.0f;
+            bool live = true;
+            if (ballw) {
+                b2 = q.w;
+            } else if (aux) {
+                const float4 a = aux[i];
+                b2 = a.x;
+                live = __float_as_uint(a.w) != 0u;
+            } else if (ball2) {
+                b2 = ball2[i];
+            }
+            if (live) {
+                x.lo = make_float3(fminf(FLT_MAX, q.x), fminf(FLT_MAX, q.y), fminf(FLT_MAX, q.z));
+                x.hi = make_float3(fmaxf(-FLT_MAX, q.x), fmaxf(-FLT_MAX, q.y), fmaxf(-FLT_MAX, q.z));
+                if (hasb) x.b2 = fmaxf(-FLT_MAX, b2);
+                if (balls) {
+                    // ball radius rounded up so the box contains every d2 < b2 point
+                    float rad = sqrtf(b2) * (1.0f + 1e-6f) + 1e-30f;
+                    rad += 4.8e-7f * (fabsf(q.x) + fabsf(q.y) + fabsf(q.z) + rad);
+                    x.blo = make_float3(fminf(FLT_MAX, q.x - rad), fminf(FLT_MAX, q.y - rad), fminf(FLT_MAX, q.z - rad));
+                    x.bhi = make_float3(fmaxf(-FLT_MAX, q.x + rad), fmaxf(-FLT_MAX, q.y + rad), fmaxf(-FLT_MAX, q.z + rad));
+                }
+            }
+        }
+        x.lo = make_float3(warp_min(x.lo.x), warp_min(x.lo.y), warp_min(x.lo.z));
+        x.hi = make_float3(warp_max(x.hi.x), warp_max(x.hi.y), warp_max(x.hi.z));
+        if (hasb) x.b2 = warp_max(x.b2);
+        if (balls) {
+            x.blo = make_float3(warp_min(x.blo.x), warp_min(x.blo.y), warp_min(x.blo.z));
+            x.bhi = make_float3(warp_max(x.bhi.x), warp_max(x.bhi.y), warp_max(x.bhi.z));
+        }
+        if (lane == 0) leaf_s[l] = x;
     }
-    int node = leafBase + leaf;
-    lo[node] = l;
-    hi[node] = h;
-    if (balls) { blo[node] = bl; bhi[node] = bh; }
-    __threadfence();
-    if (leafBase == 1 && d_dirty) *d_dirty = 0;   // the only leaf is the root
-    node >>= 1;
-    while (node >= 1) {
-        int old = atomicAdd(&flag[node], 1);
-        if (old == 0) return;
-        // the second arrival finishes the node and clears its flag for the
-        // next refit (each node has exactly two arrivals per launch)
-        flag[node] = 0;
-        __threadfence();
-        float4 l0 = __ldcg(&lo[2 * node]), l1 = __ldcg(&lo[2 * node + 1]);
-        float4 h0 = __ldcg(&hi[2 * node]), h1 = __ldcg(&hi[2 * node + 1]);
-        lo[node] = make_float4(fminf(l0.x, l1.x), fminf(l0.y, l1.y), fminf(l0.z, l1.z),
-                               fmaxf(l0.w, l1.w));
-        hi[node] = make_float4(fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z), 0.0f);
-        if (balls) {
-            float4 a0 = __ldcg(&blo[2 * node]), a1 = __ldcg(&blo[2 * node + 1]);
-            float4 c0 = __ldcg(&bhi[2 * node]), c1 = __ldcg(&bhi[2 * node + 1]);
-            blo[node] = make_float4(fminf(a0.x, a1.x), fminf(a0.y, a1.y), fminf(a0.z, a1.z), 0.0f);
-            bhi[node] = make_float4(fmaxf(c0.x, c1.x), fmaxf(c0.y, c1.y), fmaxf(c0.z, c1.z), 0.0f);
+    __syncthreads();
+    if (w != 0) return;
+    NodeBox x = leaf_s[lane];
+    if (lane < leaves) store(leafBase + first + lane, x);
+    // lane i holds the box of node first_node + i, of 2^levels nodes
+    int node = leafBase + first, levels = 0;
+    while (levels < 5 && (1 << levels) < leaves) ++levels;
+    for (;;) {
+        for (int d = 0; d < levels; ++d) {
+            const int o = 1 << d;
+            x.lo = make_float3(fminf(x.lo.x, __shfl_xor_sync(SKID_FULL, x.lo.x, o)),
+                               fminf(x.lo.y, __shfl_xor_sync(SKID_FULL, x.lo.y, o)),
+                               fminf(x.lo.z, __shfl_xor_sync(SKID_FULL, x.lo.z, o)));
+            x.hi = make_float3(fmaxf(x.hi.x, __shfl_xor_sync(SKID_FULL, x.hi.x, o)),
+                               fmaxf(x.hi.y, __shfl_xor_sync(SKID_FULL, x.hi.y, o)),
+                               fmaxf(x.hi.z, __shfl_xor_sync(SKID_FULL, x.hi.z, o)));
+            x.b2 = fmaxf(x.b2, __shfl_xor_sync(SKID_FULL, x.b2, o));
+            if (balls) {
+                x.blo = make_float3(fminf(x.blo.x, __shfl_xor_sync(SKID_FULL, x.blo.x, o)),
+                                    fminf(x.blo.y, __shfl_xor_sync(SKID_FULL, x.blo.y, o)),
+                                    fminf(x.blo.z, __shfl_xor_sync(SKID_FULL, x.blo.z, o)));
+                x.bhi = make_float3(fmaxf(x.bhi.x, __shfl_xor_sync(SKID_FULL, x.bhi.x, o)),
+                                    fmaxf(x.bhi.y, __shfl_xor_sync(SKID_FULL, x.bhi.y, o)),
+                                    fmaxf(x.bhi.z, __shfl_xor_sync(SKID_FULL, x.bhi.z, o)));
+            }
+            node >>= 1;
+            if (lane < (1 << levels) && (lane & (2 * o - 1)) == 0) store(node + (lane >> (d + 1)), x);
         }
+        if (node == 1) {
+            // the root is finished after every block has read d_dirty
+            if (d_dirty && lane == 0) *d_dirty = 0;
+            return;
+        }
+        // node is finished; so is all below its ancestor `levels` up once as
+        // many blocks have come by as that has descendants here
+        levels = min(5, 31 - __clz(node));
+        const int up = node >> levels;
+        int old = 0;
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence();
+            old = atomicAdd(&flag[up], 1);
+        }
+        if (__shfl_sync(SKID_FULL, old, 0) != (1 << levels) - 1) return;
+        if (lane == 0) flag[up] = 0;   // for the next refit
         __threadfence();
-        // the root is finished after every leaf thread has read d_dirty
-        if (node == 1 && d_dirty) *d_dirty = 0;
-        node >>= 1;
+        node = up << levels;
+        x.lo = x.blo = top;
+        x.hi = x.bhi = bottom;
+        x.b2 = -FLT_MAX;
+        if (lane < (1 << levels)) {
+            const float4 a = __ldcg(&lo[node + lane]), b = __ldcg(&hi[node + lane]);
+            x.lo = xyz(a);
+            x.b2 = a.w;
+            x.hi = xyz(b);
+            if (balls) {
+                x.blo = xyz(__ldcg(&blo[node + lane]));
+                x.bhi = xyz(__ldcg(&bhi[node + lane]));
+            }
+        }
     }
 }
 
@@ -211,8 +294,7 @@ cudaError_t tree_refit(Tree &t, const float4 *pos, const float4 *aux, const int 
         if ((e = cudaMemsetAsync(t.flag.p, 0, 2 * (size_t)t.leafBase * sizeof(int), st))) return e;
         t.flag_clear = true;
     }
-    int threads = 128;
-    int blocks = (t.leafBase + threads - 1) / threads;
+    const int threads = UP_WARPS * 32, blocks = (t.leafBase + 31) / 32;
     bool nb = t.blo.n < 2 * (size_t)t.leafBase || t.bhi.n < 2 * (size_t)t.leafBase;
     upward_kernel<<<blocks, threads, 0, st>>>(pos ? pos : t.pos.p, nullptr, aux, ballw ? 1 : 0,
                                               t.n, d_n, t.leafBase, t.lo.p, t.hi.p,
