@@ -4,12 +4,14 @@
 // density gather needs fBall2 alone, and that value does not depend on how
 // equal distances are ordered.
 //
-// One warp per leaf of 32 query points, one query per lane.  Each lane keeps
-// a max-heap of its k best squared distances in shared memory (slot i of
-// lane l at i*32+l, so every heap access is bank-conflict free).  The warp
-// first scans its own leaf, then climbs to the root visiting each sibling
-// subtree depth-first (the search order of smBallSearch, smooth1.c:89-127),
-// entering a node when any lane's heap bound reaches its box.  The last five
+// One warp per leaf of 32 query points, one query per lane (several warps
+// while there are few leaves).  Each lane keeps its nearest squared distances
+// in shared memory (value i of lane l at i*32+l, so every access is
+// bank-conflict free): an unsorted buffer cut back by counting for k from 24
+// to 128, a max-heap of k otherwise.  The warp first scans its own leaf, then
+// climbs to the root visiting each sibling subtree depth-first (the search
+// order of smBallSearch, smooth1.c:89-127), entering a node when any lane's
+// bound reaches its box.  The last five
 // levels of a subtree are tested one leaf per lane against the query leaf's
 // box and the warp's largest bound; at a leaf only candidates within that
 // bound of the query box are compacted and tested.
@@ -135,7 +137,6 @@ __device__ __forceinline__ float warp_max(float v)
 // radial bins instead, with a second walk to pick from the k-th one's, took
 // 62k instructions and had a longer tail: no faster.
 constexpr int KB_MINK = 24, KB_MAXK = 128;
-constexpr int KB_WARPS = 1;
 constexpr int KB_SLACK = 64;         // values a buffer holds beyond k
 constexpr int KB_STEP = 8;           // candidates tested between checks for room
 
@@ -158,6 +159,23 @@ __device__ __forceinline__ int kb_count(const KnnBuf &B, int m, float T)
     return (int)c;
 }
 
+// A value summed or maximised over the S lanes that share a query.
+template <int S>
+__device__ __forceinline__ int kb_sum(int v)
+{
+#pragma unroll
+    for (int o = 1; o < S; o <<= 1) v += __shfl_xor_sync(SKID_FULL, v, o);
+    return v;
+}
+
+template <int S>
+__device__ __forceinline__ float kb_max(float v)
+{
+#pragma unroll
+    for (int o = 1; o < S; o <<= 1) v = fmaxf(v, __shfl_xor_sync(SKID_FULL, v, o));
+    return v;
+}
+
 // The largest value (0 without any).
 __device__ __forceinline__ float kb_largest(const KnnBuf &B, int m)
 {
@@ -170,13 +188,16 @@ __device__ __forceinline__ float kb_largest(const KnnBuf &B, int m)
     return v;
 }
 
-// The k-th smallest value of a lane that holds at least k, between lo (fewer
-// than k values at or below it; -1: none are) and hi (k or more): guesses from
-// the counts, then bisection of the bit patterns.
-__device__ __forceinline__ float kb_kth(const KnnBuf &B, int m, int k, int lo, float hi, int cl)
+// The k-th smallest of the values that S lanes hold together (each its own
+// buffer), between lo (fewer than k values at or below it; -1: none are) and hi
+// (k or more): guesses from the counts, of which lo's is cl and hi's near ch,
+// then bisection of the bit patterns.  Lanes that are done have no use for it.
+template <int S>
+__device__ __forceinline__ float kb_kth(const KnnBuf &B, int m, int k, int lo, float hi, int cl, int ch,
+                                        bool done)
 {
-    int l = lo, h = __float_as_int(hi), ch = B.n;
-    bool done = B.n < k, largest = false;
+    int l = lo, h = __float_as_int(hi);
+    bool largest = false;
     for (int it = 0; __any_sync(SKID_FULL, !done); ++it) {
         if (!done && h - l <= 1) done = true;      // h is the answer
         int mid = l + (h - l) / 2;
@@ -187,7 +208,7 @@ __device__ __forceinline__ float kb_kth(const KnnBuf &B, int m, int k, int lo, f
             const int g = __float_as_int(fmaf(b - a, fminf(fmaxf(t, 0.02f), 0.98f), a));
             if (g > l && g < h) mid = g;
         }
-        const int c = kb_count(B, m, __int_as_float(mid));
+        const int c = kb_sum<S>(kb_count(B, m, __int_as_float(mid)));
         if (!done) {
             if (c < k) {
                 l = mid;
@@ -208,19 +229,23 @@ __device__ __forceinline__ float kb_kth(const KnnBuf &B, int m, int k, int lo, f
         const float x = B.b[i * 32];
         v = x <= T ? fmaxf(v, x) : v;
     }
+    v = kb_max<S>(v);
     return largest ? v : T;
 }
 
-// Cut every lane's buffer back: at least k values stay, at most `most`.
+// Cut every lane's buffer back, to `most` values at most.  At least k of those
+// at or below the lane's bound stay, or all where there are fewer (a bound
+// that another warp found: SHARED).
+template <bool SHARED>
 __device__ __noinline__ KnnBuf kb_cut(KnnBuf B, int k, int most)
 {
     const int m = __reduce_max_sync(SKID_FULL, B.n);
     float hi = B.thr;
     if (__any_sync(SKID_FULL, B.thr == FLT_MAX)) hi = fminf(hi, kb_largest(B, m));
     float lo = 0.0f, T = hi;
-    int cl = 0, ch = B.n;
-    // lanes with little to drop keep what they have
-    bool done = B.n <= k + (most - k) / 4;
+    int cl = 0, ch = SHARED ? kb_count(B, m, hi) : B.n;
+    // lanes with little to drop keep what they have (at or below the bound)
+    bool done = ch <= k + (most - k) / 4;
     const bool skip = done;
     const float aim = k + 0.15f * (most - k);
     for (int it = 0; it < 6 && __any_sync(SKID_FULL, !done); ++it) {
@@ -241,10 +266,10 @@ __device__ __noinline__ KnnBuf kb_cut(KnnBuf B, int k, int most)
     }
     // ties or an uneven spread: the exact k-th value, and of its copies only
     // as many as make k
-    const bool tight = !done && B.n >= k;
+    const bool tight = !done && (SHARED || B.n >= k);
     int room = 0x7fffffff;
     if (__any_sync(SKID_FULL, tight)) {
-        const float e = kb_kth(B, m, k, cl == 0 ? -1 : __float_as_int(lo), hi, cl);
+        const float e = kb_kth<1>(B, m, k, cl == 0 ? -1 : __float_as_int(lo), hi, cl, ch, !tight);
         int below = 0;
 #pragma unroll 8
         for (int i = 0; i < m; ++i) below += B.b[i * 32] < e;
@@ -253,7 +278,7 @@ __device__ __noinline__ KnnBuf kb_cut(KnnBuf B, int k, int most)
             room = k - below;
         }
     }
-    if (skip) T = FLT_MAX;
+    if (skip && !SHARED) T = FLT_MAX;
     int o = 0;
     if (__any_sync(SKID_FULL, tight)) {
         for (int i = 0; i < m; ++i) {
@@ -276,25 +301,42 @@ __device__ __noinline__ KnnBuf kb_cut(KnnBuf B, int k, int most)
     return B;
 }
 
-__global__ void __launch_bounds__(KB_WARPS * 32)
+// S warps (a block) share a query leaf: of the leaves under a node warp w takes
+// every S-th from w, with buffers of its own; a bound that one finds, at or above
+// the k-th smallest of all, serves all of them through shared memory.
+template <int S>
+__global__ void __launch_bounds__(S * 32)
 knn_buffer_kernel(TreeView t, int k, int cap, float3 L, float3 hL, bool per, int logLeafBase,
                   int subShift, float zero_arg, float *__restrict__ ball2, int *work)
 {
     extern __shared__ float4 smem4[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ unsigned thr_s[32];
+    __shared__ int n_s[S][32];
+    __shared__ int leaf_s;
+    const int lane = threadIdx.x & 31, w = S > 1 ? threadIdx.x >> 5 : 0;
     // candidates by component, then the lanes' buffers
     float *cx = reinterpret_cast<float *>(smem4) + w * 3 * SKID_LEAF;
     float *cy = cx + SKID_LEAF, *cz = cy + SKID_LEAF;
-    float *bufs = reinterpret_cast<float *>(smem4) + KB_WARPS * 3 * SKID_LEAF;
+    float *bufs = reinterpret_cast<float *>(smem4) + S * 3 * SKID_LEAF;
     const int rootLo = t.leafBase >> subShift;
     const int most = k + (cap - k) / 2;
     const f32x2 zero = pack2(zero_arg, zero_arg);
+    // of 32 leaves from a multiple of 32, this warp's
+    const unsigned mine = (S == 1 ? ~0u : S == 2 ? 0x55555555u : S == 4 ? 0x11111111u : 0x01010101u) << w;
     KnnBuf B;
     B.b = bufs + (size_t)w * cap * 32 + lane;
     for (;;) {
         int leaf = 0;
-        if (lane == 0) leaf = atomicAdd(work, 1);
-        leaf = __shfl_sync(SKID_FULL, leaf, 0);
+        if (S == 1) {
+            if (lane == 0) leaf = atomicAdd(work, 1);
+            leaf = __shfl_sync(SKID_FULL, leaf, 0);
+        } else {
+            __syncthreads();
+            if (threadIdx.x == 0) leaf_s = atomicAdd(work, 1);
+            if (w == 0) thr_s[lane] = __float_as_uint(FLT_MAX);
+            __syncthreads();
+            leaf = leaf_s;
+        }
         if (leaf >= t.nLeaf) break;
         const int base = leaf * SKID_LEAF, qi = base + lane;
         const bool valid = qi < t.n;
@@ -310,12 +352,15 @@ knn_buffer_kernel(TreeView t, int k, int cap, float3 L, float3 hL, bool per, int
             return __uint_as_float(__reduce_max_sync(SKID_FULL, __float_as_uint(B.thr)));
         };
         auto room = [&]() {
-            if (__any_sync(SKID_FULL, B.n > cap - KB_STEP)) B = kb_cut(B, k, most);
+            if (!__any_sync(SKID_FULL, B.n > cap - KB_STEP)) return;
+            B = kb_cut<(S > 1)>(B, k, most);
+            if (S > 1) B.thr = fminf(B.thr, __uint_as_float(atomicMin(&thr_s[lane], __float_as_uint(B.thr))));
         };
         // lane j keeps candidate j while it may lie below some lane's bound
         auto leaf_values = [&](int node, bool direct, bool all) {
             const int cb = (node - t.leafBase) * SKID_LEAF;
             float4 c4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (S > 1) B.thr = fminf(B.thr, __uint_as_float(*(volatile unsigned *)&thr_s[lane]));
             const float tm = all ? INFINITY : tmax();
             bool rel = cb + lane < t.n;
             if (rel) {
@@ -360,7 +405,7 @@ knn_buffer_kernel(TreeView t, int k, int cap, float3 L, float3 hL, bool per, int
                 }
             }
         };
-        leaf_values(own, boxes_direct(qlo, qhi, qlo, qhi, hL), true);
+        if (S == 1 || leaf % S == w) leaf_values(own, boxes_direct(qlo, qhi, qlo, qhi, hL), true);
         int cell = own;
         while (cell > 1) {
             int cp = cell ^ 1;
@@ -380,7 +425,10 @@ knn_buffer_kernel(TreeView t, int k, int cap, float3 L, float3 hL, bool per, int
                         const float4 l = t.lo[first + lane], h = t.hi[first + lane];
                         pass = (direct ? gap2(xyz(qlo), xyz(qhi), l, h) : boxbox_lb(qlo, qhi, l, h, L, per)) < tm;
                     }
-                    for (unsigned lm = __ballot_sync(SKID_FULL, pass); lm; lm &= lm - 1) {
+                    unsigned lm = __ballot_sync(SKID_FULL, pass);
+                    // (leaves count from 0 at leafBase: lane 0's is first)
+                    if (S > 1) lm &= mine << (S - (first & (S - 1))) | mine >> (first & (S - 1));
+                    for (; lm; lm &= lm - 1) {
                         const int node = first + __ffs(lm) - 1;
                         const float4 l = t.lo[node], h = t.hi[node];
                         const bool dl = direct || boxes_direct(qlo, qhi, l, h, hL);
@@ -397,13 +445,58 @@ knn_buffer_kernel(TreeView t, int k, int cap, float3 L, float3 hL, bool per, int
             }
             cell >>= 1;
         }
-        // the k-th smallest of what is left (the last bound is at or above it)
-        const int m = __reduce_max_sync(SKID_FULL, B.n);
+        // the k-th smallest of what is left (the last bound is at or above
+        // it); of S buffers a query, S lanes look at one each
+        int n = B.n, query = lane;
         float hi = B.thr;
-        if (__any_sync(SKID_FULL, B.thr == FLT_MAX)) hi = fminf(hi, kb_largest(B, m));
-        const float r = kb_kth(B, m, k, -1, hi, 0);
-        if (valid) ball2[qi] = B.n >= k ? r : FLT_MAX;
+        if (S > 1) {
+            n_s[w][lane] = B.n;
+            __syncthreads();
+            const int part = lane & (S - 1);
+            query = w * (32 / S) + lane / S;
+            n = n_s[part][query];
+            hi = __uint_as_float(thr_s[query]);
+            B.b = bufs + (size_t)part * cap * 32 + query;
+        }
+        const int m = __reduce_max_sync(SKID_FULL, n), all = kb_sum<S>(n);
+        if (__any_sync(SKID_FULL, hi == FLT_MAX)) hi = fminf(hi, kb_max<S>(kb_largest(B, m)));
+        const float r = kb_kth<S>(B, m, k, -1, hi, 0, all, all < k);
+        if (base + query < t.n && (lane & (S - 1)) == 0) ball2[base + query] = all >= k ? r : FLT_MAX;
+        if (S > 1) B.b = bufs + (size_t)w * cap * 32 + lane;
     }
+}
+
+template <int S>
+cudaError_t launch_buffers(const Tree &t, int k, float3 L, float3 hL, bool per, int logLeafBase, int subShift,
+                           float *ball2_sorted, int *d_work, cudaStream_t st)
+{
+    const int cap = k + KB_SLACK;
+    const size_t smem = S * (3 * SKID_LEAF + (size_t)cap * 32) * sizeof(float);
+    static std::mutex attr_mu;
+    static bool attr_done[SKID_MAX_DEVICES] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e) return e;
+    if (dev < 0 || dev >= SKID_MAX_DEVICES) return cudaErrorInvalidDevice;
+    {
+        // the most any k asks for
+        std::lock_guard<std::mutex> lk(attr_mu);
+        if (!attr_done[dev]) {
+            e = cudaFuncSetAttribute(knn_buffer_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(S * (3 * SKID_LEAF + (KB_MAXK + KB_SLACK) * 32) * sizeof(float)));
+            if (e) return e;
+            attr_done[dev] = true;
+        }
+    }
+    int perSM = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, knn_buffer_kernel<S>, S * 32, smem);
+    if (e) return e;
+    if (perSM < 1) return cudaErrorInvalidConfiguration;
+    const int blocks = num_sms() * perSM < t.nLeaf ? num_sms() * perSM : t.nLeaf;
+    if ((e = cudaMemsetAsync(d_work, 0, sizeof(int), st))) return e;
+    knn_buffer_kernel<S><<<blocks, S * 32, smem, st>>>(t.view(), k, cap, L, hL, per, logLeafBase, subShift, 0.0f,
+                                                       ball2_sorted, d_work); skid::note_launch();
+    return cudaGetLastError();
 }
 
 // ---- any k: heaps ----
@@ -487,18 +580,22 @@ cudaError_t knn_ball2(const Tree &t, int k, float3 L, bool per, float *ball2_sor
     while ((2 << logLeafBase) <= t.leafBase) ++logLeafBase;
     const int subShift = logLeafBase < 5 ? logLeafBase : 5;
     if (k >= KB_MINK && k <= KB_MAXK) {
-        const int cap = k + KB_SLACK;
-        const size_t smem = KB_WARPS * (3 * SKID_LEAF + (size_t)cap * 32) * sizeof(float);
+        // Warps that share a leaf cost more in all (each collects k values
+        // before it has a bound: about the factor S on a full chip), and pay
+        // while the chip is not full.  k = 32, a call's time with S = 1 / 2 /
+        // 4 / 8: 5,003 points 0.58 / 0.45 / 0.44 / 0.36 ms, 20,000 0.61 /
+        // 0.57 / 0.51 / 0.59, 40,000 0.59 / 0.65 / 0.71 / 0.89; k = 128,
+        // 20,000 points 1.07 / 1.13 / 1.32 / 1.70.
+        const size_t smem = (3 * SKID_LEAF + (size_t)(k + KB_SLACK) * 32) * sizeof(float);
         int perSM = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, knn_buffer_kernel, KB_WARPS * 32, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, knn_buffer_kernel<1>, 32, smem);
         if (e) return e;
-        if (perSM < 1) return cudaErrorInvalidConfiguration;
-        const int need = (t.nLeaf + KB_WARPS - 1) / KB_WARPS;
-        const int blocks = num_sms() * perSM < need ? num_sms() * perSM : need;
-        if ((e = cudaMemsetAsync(d_work, 0, sizeof(int), st))) return e;
-        knn_buffer_kernel<<<blocks, KB_WARPS * 32, smem, st>>>(t.view(), k, cap, L, hL, per, logLeafBase,
-                                                               subShift, 0.0f, ball2_sorted, d_work); skid::note_launch();
-        return cudaGetLastError();
+        const int slots = num_sms() * perSM;
+        auto launch = t.nLeaf * 8 <= slots       ? launch_buffers<8>
+                      : t.nLeaf * 4 <= slots     ? launch_buffers<4>
+                      : t.nLeaf * 8 <= slots * 3 ? launch_buffers<2>
+                                                 : launch_buffers<1>;
+        return launch(t, k, L, hL, per, logLeafBase, subShift, ball2_sorted, d_work, st);
     }
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
