@@ -510,16 +510,25 @@ mass_soft_partials(const float *__restrict__ mass, const float *__restrict__ sof
     }
 }
 
-__global__ void mass_soft_total(double *out)
+// The blocks' sums in block order, one chain of FP64 additions; the least
+// softening (a float) beside it.
+__global__ void __launch_bounds__(MS_BLOCKS)
+mass_soft_total(double *out)
 {
+    __shared__ double m_s[MS_BLOCKS];
+    __shared__ float e_s[MS_BLOCKS / 32];
+    m_s[threadIdx.x] = out[2 + 2 * threadIdx.x];
+    float e = fminf(FLT_MAX, (float)out[3 + 2 * threadIdx.x]);
+    for (int o = 16; o; o >>= 1) e = fminf(e, __shfl_xor_sync(SKID_FULL, e, o));
+    if ((threadIdx.x & 31) == 0) e_s[threadIdx.x >> 5] = e;
+    __syncthreads();
     if (threadIdx.x != 0) return;
-    double m = 0.0, e = (double)FLT_MAX;
-    for (int b = 0; b < MS_BLOCKS; ++b) {
-        m += out[2 + 2 * b];
-        e = fmin(e, out[3 + 2 * b]);
-    }
+    double m = 0.0;
+#pragma unroll 16
+    for (int b = 0; b < MS_BLOCKS; ++b) m += m_s[b];
+    for (int w = 1; w < MS_BLOCKS / 32; ++w) e = fminf(e, e_s[w]);
     out[0] = m;
-    out[1] = e;
+    out[1] = (double)e;
 }
 
 }  // extern "C"
@@ -567,7 +576,7 @@ int load_finish(skid_ctx *ctx, bool have_temp)
     // total |mass| and smallest softening for the potential scale (fixed order)
     mass_soft_partials<<<MS_BLOCKS, MS_THREADS, 0, ctx->st>>>(d_raw + 2 * n3, d_raw + 2 * n3 + n, n,
                                                              ctx->ms_dev.p); skid::note_launch();
-    mass_soft_total<<<1, 32, 0, ctx->st>>>(ctx->ms_dev.p); skid::note_launch();
+    mass_soft_total<<<1, MS_BLOCKS, 0, ctx->st>>>(ctx->ms_dev.p); skid::note_launch();
     ctx->ms_pending = true;
     fill_float<<<grid_for(n), 256, 0, ctx->st>>>(ctx->rho.p, 0.0f, n); skid::note_launch();
     fill_float<<<grid_for(n), 256, 0, ctx->st>>>(ctx->rho_final.p, 0.0f, n); skid::note_launch();

