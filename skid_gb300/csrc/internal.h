@@ -66,7 +66,7 @@ constexpr size_t SORT_GLOB_WORDS = 8 * 256 + 8;
 struct SortScratch {
     DBuf<uint64_t> k0, k1;
     DBuf<uint32_t> v0, v1;
-    DBuf<uint32_t> hist;   // per-tile look-back status of a sort pass (256 per tile)
+    DBuf<uint32_t> hist;   // per-tile look-back status of every sort pass (256 per tile and pass)
     DBuf<uint32_t> glob;   // SORT_GLOB_WORDS: digit offsets of every pass, tile counters
     DBuf<int> blk;         // per-block sums for scans
     DBuf<unsigned> box;    // bounding box (ordered uints)

@@ -46,7 +46,7 @@ constexpr size_t OFF_K1 = align256(OFF_K0 + sizeof(uint64_t) * NA_MAXN);
 constexpr size_t OFF_V0 = align256(OFF_K1 + sizeof(uint64_t) * NA_MAXN);
 constexpr size_t OFF_V1 = align256(OFF_V0 + sizeof(uint32_t) * NA_MAXN);
 constexpr size_t OFF_HIST = align256(OFF_V1 + sizeof(uint32_t) * NA_MAXN);
-constexpr size_t OFF_BLK = align256(OFF_HIST + sizeof(uint32_t) * 256 * NA_TILES);
+constexpr size_t OFF_BLK = align256(OFF_HIST + sizeof(uint32_t) * 256 * NA_TILES * 8);
 constexpr size_t OFF_BOX = align256(OFF_BLK + sizeof(int) * 64);
 constexpr size_t OFF_TPOS = align256(OFF_BOX + sizeof(unsigned) * 8);
 constexpr size_t OFF_PERM = align256(OFF_TPOS + sizeof(float4) * NA_MAXN);
@@ -142,7 +142,7 @@ extern "C" int skid_knn_ball2_noalloc(const float *d_pos, int n, int k, const fl
     ss.k1 = view<uint64_t>(base, OFF_K1, NA_MAXN);
     ss.v0 = view<uint32_t>(base, OFF_V0, NA_MAXN);
     ss.v1 = view<uint32_t>(base, OFF_V1, NA_MAXN);
-    ss.hist = view<uint32_t>(base, OFF_HIST, 256 * (size_t)NA_TILES);
+    ss.hist = view<uint32_t>(base, OFF_HIST, 256 * (size_t)NA_TILES * 8);
     ss.glob = view<uint32_t>(base, OFF_GLOB, SORT_GLOB_WORDS);
     ss.blk = view<int>(base, OFF_BLK, 64);
     ss.box = view<unsigned>(base, OFF_BOX, 8);
