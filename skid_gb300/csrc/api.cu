@@ -352,7 +352,8 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
     // The caller's positions come in any order, and the 32 that share a warp
     // share its walk: visited in Hilbert order, as the movers of a run are,
     // the walk serves neighbours.  100k positions in particle order over
-    // 131k scatterers took 2.88 ms a call; sorted first, 0.48 ms with the sort.  A position's sum runs over the copies in tree order whichever
+    // 131k scatterers took 2.88 ms a call; sorted first, 0.33 ms with the
+    // sort.  A position's sum runs over the copies in tree order whichever
     // positions share its warp, so the values do not change.
     CK(curve_order(p4.p, nm, ctx->ss, st));
     CK(cudaMemcpyAsync(act.p, ctx->ss.v0.p, (size_t)nm * sizeof(int), cudaMemcpyDeviceToDevice, st));
