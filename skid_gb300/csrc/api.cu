@@ -325,8 +325,6 @@ void skid_ctx::collect_field_times(int nslots)
 // ---------------------------------------------------------------------
 // C ABI
 
-// Move field at nm explicit positions from the current live copies, left in
-// probe_acc (the body of skid_field and skid_field_adjoint).
 __global__ void unsort_xyz(const int *__restrict__ perm, const float *__restrict__ in, int n,
                            float *__restrict__ out)
 {
@@ -338,6 +336,24 @@ __global__ void unsort_xyz(const int *__restrict__ perm, const float *__restrict
     }
 }
 
+// Positions from which a probe visits them in Hilbert order.  They come in any
+// order, and the 32 that share a warp share its walk: visited in Hilbert
+// order, as the movers of a run are, the walk serves neighbours.  The sort is
+// 14 launches, about 0.08 ms, and no help to a warp's worth.  A call's time in
+// the caller's order / sorted, ms:
+//   positions                         1          32         128        512        20000
+//   random, 131,072 scatterers   .06 / .14  1.41 / 1.49 1.47 / 1.03 1.55 / .69 1.68 / .33
+//   random, 5,003 scatterers     .06 / .15   .33 / .42   .31 / .37   .34 / .27  .38 / .21
+//   neighbours, 131,072          .06 / .14   .09 / .17   .14 / .20   .20 / .20  .49 / .25
+//   neighbours, 5,003            .06 / .15   .09 / .17   .12 / .18   .14 / .19     -
+// A position's sum runs over the copies in tree order whichever positions share
+// its warp, so the order does not change the values -- but for 4, 8 or 16
+// movers per warp, when asked for: which of a position's lanes sums a copy then
+// depends on its neighbours.
+constexpr int PROBE_SORT_MIN = 128;
+
+// Move field at nm explicit positions from the current live copies, left in
+// probe_acc (the body of skid_field and skid_field_adjoint).
 static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
 {
     cudaStream_t st = ctx->st;
@@ -349,17 +365,16 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
         return ctx->fail(SKID_ENOMEM);
     CK(cudaMemcpyAsync(xyz.p, mpos, 3 * (size_t)nm * sizeof(float), cudaMemcpyHostToDevice, st));
     xyz_to_pos4<<<grid_for(nm), 256, 0, st>>>(xyz.p, nm, p4.p); skid::note_launch();
-    // The caller's positions come in any order, and the 32 that share a warp
-    // share its walk: visited in Hilbert order, as the movers of a run are,
-    // the walk serves neighbours.  100k positions in particle order over
-    // 131k scatterers took 2.88 ms a call; sorted first, 0.33 ms with the
-    // sort.  A position's sum runs over the copies in tree order whichever
-    // positions share its warp, so the values do not change.
-    CK(curve_order(p4.p, nm, ctx->ss, st));
-    CK(cudaMemcpyAsync(act.p, ctx->ss.v0.p, (size_t)nm * sizeof(int), cudaMemcpyDeviceToDevice, st));
+    const bool sorted = nm >= PROBE_SORT_MIN;
+    if (sorted) {
+        CK(curve_order(p4.p, nm, ctx->ss, st));
+        CK(cudaMemcpyAsync(act.p, ctx->ss.v0.p, (size_t)nm * sizeof(int), cudaMemcpyDeviceToDevice, st));
+    } else {
+        iota_kernel<<<grid_for(nm), 256, 0, st>>>(act.p, nm); skid::note_launch();
+    }
     CK(cudaMemcpyAsync(act.p + nm, &nm, sizeof(int), cudaMemcpyHostToDevice, st));
-    // the kernel writes by sorted slot; xyz is free again after the packing
-    FieldArgs a = ctx->field_args(0.0f, false, xyz.p);
+    // the kernel writes by slot of act; xyz is free again after the packing
+    FieldArgs a = ctx->field_args(0.0f, false, sorted ? xyz.p : ctx->probe_acc.p);
     a.mpos = p4.p;
     a.act = act.p;
     a.d_nA = act.p + nm;
@@ -370,7 +385,7 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
     a.touched = nullptr;
     a.floor = nullptr;
     CK(field_move(a, nm, st));
-    if (nm > 0) {
+    if (sorted) {
         unsort_xyz<<<grid_for(nm), 256, 0, st>>>(act.p, xyz.p, nm, ctx->probe_acc.p); skid::note_launch();
         CK(cudaGetLastError());
     }
