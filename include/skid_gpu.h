@@ -171,8 +171,10 @@ int skid_set_groups(skid_ctx *ctx, const int *grp, int nGroup, const skid_group 
 int skid_set_soft(skid_ctx *ctx, float fEps);
 
 /* kdUnbind (kd.c:1299-1466) with kdCellPot/kdSubPot/kdAddScoopPot
- * (grav.c:8-135).  a = 1/(1+z); aH = a*H(a) (kd.c:1317-1318).  Every group
- * runs in one launch.  nUnbound gets the particles removed. */
+ * (grav.c:8-135).  a = 1/(1+z); aH = a*H(a) (kd.c:1317-1318).  All
+ * groups run together: one launch for the potentials, two for the removal
+ * (groups that take a block, groups that take a warp).  nUnbound gets the
+ * particles removed. */
 int skid_unbind(skid_ctx *ctx, int iSoftType, float fScoop, int bGasAndDark, int bNoUnbind,
                 int nMaxMembers, float G, float z, float a, float aH, int *nUnbound);
 

@@ -19,16 +19,16 @@
 // potential exactly 0 (or its scoop part) and is unbound with E = 1/2 dv^2 >= 0.
 // Integer sums reproduce that exactly and in any order.
 //
-// Kernels, every group in one launch each:
-//  - scoop lists: one thread per group walks the tree of ungrouped particles;
+// Kernels, each taking every group in one launch (the removal in two):
+//  - scoop lists: one warp per group walks the tree of ungrouped particles;
 //  - potentials: work items are the upper-triangle tile pairs (I <= J) of
 //    every group, largest groups first; each pair's psi is evaluated once and
 //    added to both ends (the terms are exact integers, so the sums do not
 //    depend on the order);
-//  - removal: one persistent kernel takes groups largest first from a queue:
-//    groups above `tw` members get the whole block (BS threads, block-wide
-//    arg-max with first-index ties), smaller groups one warp each (warp
-//    shuffles only, no block barriers).
+//  - removal: two persistent kernels take groups largest first, each from a
+//    queue: one those above `tw` members, the whole block on a group (BS
+//    threads, block-wide arg-max with first-index ties), the other the smaller
+//    ones, a warp each (warp shuffles only, no block barriers), beside it.
 // (tw, BS) is picked by timing the candidates on the first call (autotune),
 // or fixed through the context's options.  A per-group mode (one potential
 // and one removal launch per group, the reference's serial loop on the GPU)
@@ -776,7 +776,7 @@ struct RemoveArgs {
     int plummer, subpot, nounbind;
     const uint32_t *order;          // valid groups, largest first
     const int *d_cnt;               // [valid groups, groups above tw]
-    int *d_queue;
+    int *d_queue, *d_wqueue;        // next group for a block, for a warp
     const int *d_ccnt;              // groups taken by clusters (the largest, a prefix of order)
     int *d_cqueue;
     int qcap;                       // members per block slice a cluster can hold
@@ -878,7 +878,7 @@ __device__ __forceinline__ void write_record(const RemoveArgs &A, int g, int n, 
 
 // A small group, one warp: every lane keeps the FP64 centre itself (the same
 // values on every lane), lane 0 writes.
-__device__ __noinline__ void warp_group(const RemoveArgs &A, int g)
+__device__ void warp_group(const RemoveArgs &A, int g)
 {
     const int lane = threadIdx.x & 31;
     const int s = A.gstart[g], n0 = A.gcount[g];
@@ -1993,16 +1993,17 @@ __device__ void cluster_group(const RemoveArgs &A, int g, BlockShared<BS> &S, Cl
     cl.sync();   // no block leaves while another may still read its shared memory
 }
 
-// Persistent removal: queue items [0, nbig) are large groups (one block
-// each), then chunks of BS/32 small groups (one warp each), all largest
-// first.  With A.single > 0 one block processes just that group.
+// Persistent removal of the groups above tw members, a block each (the
+// largest on clusters of CS blocks first, when launched so), largest first.
+// With A.single > 0 one block processes just that group.  The kernel of the
+// other groups may start once every block here has (remove_launch).
 template <int BS, int CS>
 __global__ void __launch_bounds__(BS) remove_kernel(const __grid_constant__ RemoveArgs A)
 {
     __shared__ BlockShared<BS> S;
     __shared__ int s_item;
     extern __shared__ float4 dyn[];
-    constexpr int W = BS / 32;
+    asm volatile("griddepcontrol.launch_dependents;");
     if (A.single > 0) {
         block_group<BS>(A, A.single, S, dyn);
         return;
@@ -2024,22 +2025,39 @@ __global__ void __launch_bounds__(BS) remove_kernel(const __grid_constant__ Remo
         }
         first = nclu;
     }
-    const int nvalid = A.d_cnt[0], nbig = A.d_cnt[1] > first ? A.d_cnt[1] : first;
-    const int nb = nbig - first;
-    const int nitems = nb + (nvalid - nbig + W - 1) / W;
+    const int nbig = A.d_cnt[1];
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(A.d_queue, 1);
         __syncthreads();
-        const int item = s_item;
+        const int item = first + s_item;
         __syncthreads();
-        if (item >= nitems) break;
-        if (item < nb) {
-            block_group<BS>(A, (int)A.order[first + item], S, dyn);
-        } else {
-            int k = nbig + (item - nb) * W + (threadIdx.x >> 5);
-            if (k < nvalid) warp_group(A, (int)A.order[k]);
-        }
+        if (item >= nbig) break;
+        block_group<BS>(A, (int)A.order[item], S, dyn);
     }
+}
+
+// Persistent removal of the groups of up to tw members, a warp each.
+//
+// Latency bounds it (one chain of passes a group), so warps in flight decide,
+// and it is a kernel of its own for that: 90 registers, 20 warps an SM, where
+// the block form takes 184 (128 and spills at 512 threads).  In one kernel
+// with the block form 20,000 groups of 100 members took 2.13 ms, 5,000 of 300
+// 1.28 and 3,000 of 1,000 5.32; on their own 1.39, 0.53 and 2.41.
+constexpr int RW_THREADS = 128;
+
+__global__ void __launch_bounds__(RW_THREADS) remove_warps_kernel(const __grid_constant__ RemoveArgs A)
+{
+    const int lane = threadIdx.x & 31;
+    const int nvalid = A.d_cnt[0], nbig = A.d_cnt[1];
+    for (;;) {
+        int item = 0;
+        if (lane == 0) item = atomicAdd(A.d_wqueue, 1);
+        item = nbig + __shfl_sync(SKID_FULL, item, 0);
+        if (item >= nvalid) break;
+        warp_group(A, (int)A.order[item]);
+    }
+    // the blocks' kernel, if it is still running, ends before this one does
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Raise a removal kernel's shared-memory limit to all it can have, once per
@@ -2132,13 +2150,13 @@ cudaError_t launch_remove_clusters(RemoveArgs A, cudaStream_t st)
 
 // cs: 1 (no clusters), 4 or 8; nlargest: the members of the largest group a
 // block will take; single: one block for A.single alone
-cudaError_t remove_launch(const RemoveArgs &A, int bs, int cs, int nlargest, bool single, cudaStream_t st)
+cudaError_t remove_blocks(const RemoveArgs &A, int bs, int cs, int nlargest, bool single, cudaStream_t st)
 {
     if (cs == 4 || cs == 8) {
         switch (bs) {
-        case 512: return cs == 4 ? launch_remove_clusters<512, 4>(A, st) : launch_remove_clusters<512, 8>(A, st);
-        case 1024: return cs == 4 ? launch_remove_clusters<1024, 4>(A, st) : launch_remove_clusters<1024, 8>(A, st);
-        default: return cs == 4 ? launch_remove_clusters<256, 4>(A, st) : launch_remove_clusters<256, 8>(A, st);
+        case 512: return cs == 8 ? launch_remove_clusters<512, 8>(A, st) : launch_remove_clusters<512, 4>(A, st);
+        case 1024: return cs == 8 ? launch_remove_clusters<1024, 8>(A, st) : launch_remove_clusters<1024, 4>(A, st);
+        default: return cs == 8 ? launch_remove_clusters<256, 8>(A, st) : launch_remove_clusters<256, 4>(A, st);
         }
     }
     switch (bs) {
@@ -2147,6 +2165,33 @@ cudaError_t remove_launch(const RemoveArgs &A, int bs, int cs, int nlargest, boo
     case 1024: return launch_remove<1024>(A, nlargest, single, st);
     default: return launch_remove<256>(A, nlargest, single, st);
     }
+}
+
+// All nvalid groups: those above tw members by blocks (none where the largest
+// has nlargest <= tw), the others by warps, on the SMs that the blocks leave:
+// the second launch is a dependent one that starts when every block of the
+// first has started (its inputs are older than both), so that a group that
+// takes long does not hold up the small ones.
+cudaError_t remove_launch(const RemoveArgs &A, int tw, int bs, int cs, int nvalid, int nlargest, cudaStream_t st)
+{
+    cudaError_t e;
+    const bool blocks = nlargest > tw;
+    if (blocks && (e = remove_blocks(A, bs, cs, nlargest, false, st))) return e;
+    int perSM = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, remove_warps_kernel, RW_THREADS, 0))) return e;
+    constexpr int W = RW_THREADS / 32;
+    const int need = (nvalid + W - 1) / W, most = num_sms() * (perSM > 0 ? perSM : 1);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.blockDim = dim3(RW_THREADS, 1, 1);
+    cfg.gridDim = dim3(need < most ? need : most, 1, 1);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = blocks ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, remove_warps_kernel, A); note_launch();
+    return e ? e : cudaGetLastError();
 }
 
 }  // namespace
@@ -2262,6 +2307,7 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
     A.order = U.order.p;
     A.d_cnt = U.cnt.p + 4;
     A.d_queue = U.cnt.p + 6;
+    A.d_wqueue = U.cnt.p + 7;
     A.d_ccnt = U.cnt.p + 9;
     A.d_cqueue = U.cnt.p + 10;
     A.qcap = qcap;
@@ -2278,13 +2324,12 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
     };
     auto removal = [&](int tw, int bs, int ucs) -> cudaError_t {
         cudaError_t e2;
-        if ((e2 = cudaMemsetAsync(U.cnt.p + 4, 0, 3 * sizeof(int), st))) return e2;
+        if ((e2 = cudaMemsetAsync(U.cnt.p + 4, 0, 4 * sizeof(int), st))) return e2;
         if ((e2 = cudaMemsetAsync(U.cnt.p + 10, 0, sizeof(int), st))) return e2;
         sched_counts<<<grid_for(ng), 256, 0, st>>>(G.count.p, ng, P.nmax, tw, U.cnt.p + 4); note_launch();
         if ((e2 = cudaMemsetAsync(d_unbound, 0, sizeof(int), st))) return e2;
         if (nvalid <= 0) return cudaSuccess;
-        // groups of up to tw members take no block
-        return remove_launch(A, bs, bs >= 256 ? ucs : 1, nlargest > tw ? nlargest : 0, false, st);
+        return remove_launch(A, tw, bs, bs >= 256 ? ucs : 1, nvalid, nlargest, st);
     };
 
     if (P.per_group) {
@@ -2305,7 +2350,7 @@ cudaError_t unbind_run(GroupState &G, const int *gof, int nslots, const float4 *
                 U.scnt.p, U.slist.p, U.ssoft.p, P.G, P.plummer, P.scale, 0.0f, U.pot.p); note_launch();
             RemoveArgs A1 = A;
             A1.single = (int)order[k];
-            if ((e = remove_launch(A1, 256, 1, nlargest, true, st))) return e;
+            if ((e = remove_blocks(A1, 256, 1, nlargest, true, st))) return e;
         }
         return cudaGetLastError();
     }
