@@ -37,6 +37,7 @@
 // 1/(15 r^3) + (2/e)^3 (-8/3 + 3u - 6u^2/5 + u^3/6) for u < 2, -1/r^3 beyond;
 // Plummer -(r^2 + e^2/4)^(-3/2).  Pair sums are FP32; the per-group energy
 // total is FP64.
+#include <algorithm>
 #include <cfloat>
 #include <vector>
 
@@ -477,9 +478,11 @@ __device__ __forceinline__ float wrap_rel(float d, float h)
 // as well as rows because a group's rows alone leave the GPU idle: 24 groups
 // of up to 35k members (140k rows, 2.9e9 pairs) gave 14 warps an SM and
 // items of 35k columns, 9.9 ms a call with or without the gradient.  Now 2.5
-// and 1.75 ms.  An item's Kahan-compensated row sums are combined in FP64,
-// where adding a few floats is exact, and rounded to float once at the end,
-// which is what one compensated sum over the whole row gives.
+// and 1.75 ms.  A row's sums over each chunk (the potential's Kahan-compensated)
+// go to memory, and pa_finish adds them in FP64 in chunk order, rounding to
+// float once at the end: the sums do not depend on the order in which blocks
+// run.  (The last block to finish a tile's chunks adding them here, a fence
+// and a count per item, cost 8 % at short chunks.)
 constexpr int PA_TILE = 128;
 constexpr int PA_THREADS = PA_TILE / 2;
 // Columns per item: long ones (fewer partial sums) once the pairs fill every
@@ -496,17 +499,24 @@ constexpr long long PA_FILL = 32;
 // order, for 0.1 ms of sorting.
 constexpr double PA_SORT_PAIRS = 1.5e8;
 
+// A group has at most this many chunks (longer ones from 64 x PA_CHUNK members
+// on), which bounds the memory its rows' partial sums take.
+constexpr int PA_MAX_CHUNKS = 64;
+// Rows with this many chunks on average have them added by PA_PARTS warps.
+constexpr int PA_PARTS = 4, PA_PARTS_MIN = 16;
+
 struct PotSlot {
     long long item0;            // items of the slots before this one
     long long row0;             // rows of the slots before this one
     long long tile0;            // row tiles of the slots before this one
-    int g, n, nchunk;
+    long long part0;            // partial sums of the slots before this one
+    int g, n, chunk, nchunk;
     float v;
 };
 
 struct PotAdjArgs {
     const PotSlot *slots;
-    int nslot, chunk;
+    int nslot;
     long long nitems, nrows;
     const int *gstart, *members;
     const float4 *pos4, *vel4;  // (x, y, z, m), (vx, vy, vz, soft)
@@ -520,19 +530,22 @@ struct PotAdjArgs {
     int *rio;                   // packed rows: iOrder
     float4 *tlo, *thi;          // per row tile: its box; tlo.w: its largest softening
     long long ntile;
-    double *acc;                // per row: sum_j m_j psi, then (gradient) sum_j m_j psi'/r (x_i - x_j)
-    double *E;                  // per slot
+    float2 *pphi;               // per slot, chunk and row: sum_j m_j psi and its compensation,
+    float *pgx, *pgy, *pgz;     // (gradient) sum_j m_j psi'/r (x_i - x_j)
+    double *eblock;             // per block of pa_finish: its rows' energy
+    double *E;                  // per slot (zeroed)
+    int *done;                  // such blocks finished per slot (zeroed)
     float *grad;                // 3n by iOrder (zeroed) or null
 };
 
-// The slot holding row (or item) k: the last one that starts at or before it.
-template <bool ROWS>
-__device__ __forceinline__ int pa_slot(const PotAdjArgs &a, long long k)
+// The slot holding item, row or tile k: the last one that starts at or before
+// it by that running sum.
+__device__ __forceinline__ int pa_slot(const PotAdjArgs &a, long long k, long long PotSlot::*start)
 {
     int lo = 0, hi = a.nslot - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if ((ROWS ? a.slots[mid].row0 : a.slots[mid].item0) <= k) lo = mid;
+        if (a.slots[mid].*start <= k) lo = mid;
         else hi = mid - 1;
     }
     return lo;
@@ -551,7 +564,7 @@ __global__ void pa_extent(PotAdjArgs a, unsigned *ext)
     float m = 0.0f;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
          k += (long long)gridDim.x * blockDim.x) {
-        const PotSlot S = a.slots[pa_slot<true>(a, k)];
+        const PotSlot S = a.slots[pa_slot(a, k, &PotSlot::row0)];
         const float3 r = pa_rel(a, S, a.pos4[a.members[a.gstart[S.g] + (int)(k - S.row0)]]);
         m = fmaxf(m, fmaxf(fabsf(r.x), fmaxf(fabsf(r.y), fabsf(r.z))));
     }
@@ -568,7 +581,7 @@ __global__ void pa_keys(PotAdjArgs a, const unsigned *ext, uint64_t *keys, uint3
     const float R = fmaxf(__uint_as_float(*ext), 1e-30f), sc = 4095.5f / R;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
          k += (long long)gridDim.x * blockDim.x) {
-        const int s = pa_slot<true>(a, k);
+        const int s = pa_slot(a, k, &PotSlot::row0);
         const PotSlot S = a.slots[s];
         const float3 r = pa_rel(a, S, a.pos4[a.members[a.gstart[S.g] + (int)(k - S.row0)]]);
         auto cell = [&](float x) {
@@ -583,7 +596,7 @@ __global__ void pa_pack(PotAdjArgs a)
 {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
          k += (long long)gridDim.x * blockDim.x) {
-        const PotSlot S = a.slots[pa_slot<true>(a, k)];
+        const PotSlot S = a.slots[pa_slot(a, k, &PotSlot::row0)];
         const long long from = a.perm ? (long long)a.perm[k] : k;
         const int io = a.members[a.gstart[S.g] + (int)(from - S.row0)];
         const float4 p = a.pos4[io];
@@ -602,13 +615,7 @@ __global__ void pa_boxes(PotAdjArgs a)
     const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long t = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); t < a.ntile;
          t += nw) {
-        int lo_s = 0, hi_s = a.nslot - 1;
-        while (lo_s < hi_s) {
-            const int mid = (lo_s + hi_s + 1) >> 1;
-            if (a.slots[mid].tile0 <= t) lo_s = mid;
-            else hi_s = mid - 1;
-        }
-        const PotSlot S = a.slots[lo_s];
+        const PotSlot S = a.slots[pa_slot(a, t, &PotSlot::tile0)];
         float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f);
         float4 hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f);
         const int i0 = (int)(t - S.tile0) * PA_TILE;
@@ -679,9 +686,8 @@ __global__ void __launch_bounds__(PA_THREADS) potential_adjoint_kernel(PotAdjArg
     __shared__ float ss[PA_TILE];
     const int tid = threadIdx.x;
     for (long long it = blockIdx.x; it < a.nitems; it += gridDim.x) {
-        const PotSlot S = a.slots[pa_slot<false>(a, it)];
-        const int k = (int)(it - S.item0);
-        const int tile = k / S.nchunk, ch = k - tile * S.nchunk;
+        const PotSlot S = a.slots[pa_slot(a, it, &PotSlot::item0)];
+        const int tile = (int)(it - S.item0) / S.nchunk, ch = (int)(it - S.item0) - tile * S.nchunk;
         const int n = S.n;
         const float4 *rm = a.rm + S.row0;
         const float *re = a.re + S.row0;
@@ -695,7 +701,7 @@ __global__ void __launch_bounds__(PA_THREADS) potential_adjoint_kernel(PotAdjArg
         w.y = pack2(q0.y, q1.y);
         w.z = pack2(q0.z, q1.z);
         w.phi = w.phic = w.gx = w.gy = w.gz = 0ull;
-        const int c0 = ch * a.chunk, c1 = min(n, c0 + a.chunk);
+        const int c0 = ch * S.chunk, c1 = min(n, c0 + S.chunk);
         for (int jb = c0; jb < c1; jb += PA_TILE) {
             const int cnt = min(PA_TILE, c1 - jb);
             const float4 blo = a.tlo[S.tile0 + jb / PA_TILE], bhi = a.thi[S.tile0 + jb / PA_TILE];
@@ -756,60 +762,109 @@ __global__ void __launch_bounds__(PA_THREADS) potential_adjoint_kernel(PotAdjArg
                 }
             }
         }
-        constexpr int NA = GRAD ? 4 : 1;
         const float2 phi = unpack2(w.phi), phic = unpack2(w.phic);
         const float2 hx = unpack2(w.gx), hy = unpack2(w.gy), hz = unpack2(w.gz);
+        const size_t first = S.part0 + (size_t)ch * n;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int i = q ? i1 : i0;
             if (i >= n) continue;
-            double *o = a.acc + NA * (S.row0 + i);
-            atomicAdd(o, (double)(q ? phi.y : phi.x) + (double)(q ? phic.y : phic.x));
+            a.pphi[first + i] = q ? make_float2(phi.y, phic.y) : make_float2(phi.x, phic.x);
             if (GRAD) {
-                atomicAdd(o + 1, (double)(q ? hx.y : hx.x));
-                atomicAdd(o + 2, (double)(q ? hy.y : hy.x));
-                atomicAdd(o + 3, (double)(q ? hz.y : hz.x));
+                a.pgx[first + i] = q ? hx.y : hx.x;
+                a.pgy[first + i] = q ? hy.y : hy.x;
+                a.pgz[first + i] = q ? hz.y : hz.x;
             }
         }
     }
 }
 
-// E_s = -1/2 G sum_i m_i phi_i in FP64, one block per slot, in a fixed order.
-constexpr int PE_THREADS = 512;
-
-__global__ void __launch_bounds__(PE_THREADS) pa_energy(PotAdjArgs a)
+// A sum over the block's threads in a fixed order.
+__device__ __forceinline__ double pa_block_sum(double v)
 {
-    __shared__ double red[PE_THREADS / 32];
-    for (int s = blockIdx.x; s < a.nslot; s += gridDim.x) {
-        const PotSlot S = a.slots[s];
-        const int NA = a.grad ? 4 : 1;
-        double e = 0.0;
-        for (int i = threadIdx.x; i < S.n; i += PE_THREADS)
-            e += -0.5 * (double)a.G * (double)a.rm[S.row0 + i].w *
-                 (double)(float)a.acc[NA * (S.row0 + i)];
-        for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(SKID_FULL, e, o);
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int k = 0; k < PE_THREADS / 32; ++k) t += red[k];
-            a.E[s] = t;
-        }
-    }
+    __shared__ double red[PA_TILE / 32];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(SKID_FULL, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = red[0];
+    for (int k = 1; k < PA_TILE / 32; ++k) t += red[k];
+    return t;
 }
 
-// The gradient by iOrder, one thread per packed row.
-__global__ void pa_gradient(PotAdjArgs a)
+// A block takes a row tile's rows (with PARTS = 4 a quarter of them, a warp to
+// each quarter of the chunks): their sums over all chunks, their gradient by
+// iOrder, and their energy -1/2 G sum_i m_i phi_i in FP64; the block that is
+// the last to finish of a slot's adds the blocks' energies.  A chain of
+// latencies bounds it; four parts shorten it where there are many chunks, and
+// cost a second wave of blocks where there are few (PA_PARTS).
+template <bool GRAD, int PARTS>
+__global__ void __launch_bounds__(PA_TILE) pa_finish(PotAdjArgs a)
 {
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
-         k += (long long)gridDim.x * blockDim.x) {
-        const PotSlot S = a.slots[pa_slot<true>(a, k)];
-        const float c = -a.G * a.rm[k].w * S.v;
-        float *o = a.grad + 3 * (size_t)a.rio[k];
-        o[0] = c * (float)a.acc[4 * k + 1];
-        o[1] = c * (float)a.acc[4 * k + 2];
-        o[2] = c * (float)a.acc[4 * k + 3];
+    constexpr int NA = GRAD ? 4 : 1, ROWS = PA_TILE / PARTS;
+    __shared__ double sums[PARTS][NA][ROWS];
+    __shared__ int last;
+    const int tid = threadIdx.x, row = tid % ROWS, part = tid / ROWS;
+    for (long long b = blockIdx.x; b < a.ntile * PARTS; b += gridDim.x) {
+        const int slot = pa_slot(a, b / PARTS, &PotSlot::tile0);
+        const PotSlot S = a.slots[slot];
+        const int i = (int)(b - S.tile0 * PARTS) * ROWS + row;
+        const bool in = i < S.n;
+        float m = 0.0f;
+        int io = 0;
+        if (in && part == 0) {
+            m = a.rm[S.row0 + i].w;
+            io = a.rio[S.row0 + i];
+        }
+        double v[NA] = {};
+        if (in) {
+            const int c1 = (int)((long long)S.nchunk * (part + 1) / PARTS);
+#pragma unroll 8
+            for (int c = (int)((long long)S.nchunk * part / PARTS); c < c1; ++c) {
+                const size_t o = S.part0 + (size_t)c * S.n + i;
+                const float2 p = a.pphi[o];
+                v[0] += (double)p.x + (double)p.y;
+                if (GRAD) {
+                    v[1 % NA] += (double)a.pgx[o];
+                    v[2 % NA] += (double)a.pgy[o];
+                    v[3 % NA] += (double)a.pgz[o];
+                }
+            }
+        }
+        if (PARTS > 1) {
+            __syncthreads();
+            for (int d = 0; d < NA; ++d) sums[part][d][row] = v[d];
+            __syncthreads();
+            if (part == 0)
+                for (int k = 1; k < PARTS; ++k)
+                    for (int d = 0; d < NA; ++d) v[d] += sums[k][d][row];
+        }
+        double e = 0.0;
+        if (in && part == 0) {
+            e = -0.5 * (double)a.G * (double)m * (double)(float)v[0];
+            if (GRAD) {
+                const float c = -a.G * m * S.v;
+                float *o = a.grad + 3 * (size_t)io;
+                for (int d = 0; d < 3; ++d) o[d] = c * (float)v[(d + 1) % NA];
+            }
+        }
+        e = pa_block_sum(e);
+        const int nb = (S.n + PA_TILE - 1) / PA_TILE * PARTS;
+        if (nb > 1) {
+            if (tid == 0) {
+                a.eblock[b] = e;
+                __threadfence();
+                last = atomicAdd(a.done + slot, 1) == nb - 1;
+            }
+            __syncthreads();
+            if (!last) continue;
+            __threadfence();
+            e = 0.0;
+            for (int k = tid; k < nb; k += PA_TILE) e += __ldcg(&a.eblock[S.tile0 * PARTS + k]);
+            e = pa_block_sum(e);
+        }
+        if (tid == 0) a.E[slot] = e;
     }
 }
 
@@ -884,42 +939,45 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
     int chunk = PA_CHUNK;
     while (chunk > PA_CHUNK_MIN && pairs < (double)(PA_FILL * num_sms()) * PA_TILE * chunk) chunk >>= 1;
     std::vector<PotSlot> slots(nSel);
-    long long nitems = 0, nrows = 0, ntile = 0;
+    long long nitems = 0, nrows = 0, ntile = 0, npart = 0;
     for (int s = 0; s < nSel; ++s) {
         const int c = counts[h_sel[s]];
         PotSlot &S = slots[s];
         S.item0 = nitems;
         S.row0 = nrows;
         S.tile0 = ntile;
+        S.part0 = npart;
         S.g = h_sel[s];
         S.n = c;
-        S.nchunk = (c + chunk - 1) / chunk;
+        S.chunk = std::max(chunk, ((c + PA_MAX_CHUNKS - 1) / PA_MAX_CHUNKS + PA_TILE - 1) / PA_TILE * PA_TILE);
+        S.nchunk = (c + S.chunk - 1) / S.chunk;
         S.v = h_v ? h_v[s] : 0.0f;
         nitems += (long long)((c + PA_TILE - 1) / PA_TILE) * S.nchunk;
         nrows += c;
         ntile += (c + PA_TILE - 1) / PA_TILE;
+        npart += (long long)c * S.nchunk;
     }
-    const int na = want_grad ? 4 : 1;
+    // energies, then the counts of finished blocks, cleared together
+    const size_t nE = nSel > 0 ? nSel : 1, nclear = nE + (nE + 1) / 2;
     if ((e = dalloc(A.slots, (size_t)(nSel > 0 ? nSel : 1) * sizeof(PotSlot))) ||
-        (e = dalloc(A.E, nSel > 0 ? nSel : 1)) || (e = dalloc(A.out, 3 * (size_t)(n > 0 ? n : 1))) ||
+        (e = dalloc(A.E, nclear)) || (e = dalloc(A.out, 3 * (size_t)(n > 0 ? n : 1))) ||
         (e = dalloc(A.rm, (size_t)(nrows > 0 ? nrows : 1))) ||
         (e = dalloc(A.re, (size_t)(nrows > 0 ? nrows : 1))) ||
         (e = dalloc(A.rio, (size_t)(nrows > 0 ? nrows : 1))) ||
         (e = dalloc(A.tbox, 2 * (size_t)(ntile > 0 ? ntile : 1))) ||
-        (e = dalloc(A.acc, (size_t)na * (nrows > 0 ? nrows : 1))))
+        (e = dalloc(A.eblock, (size_t)PA_PARTS * (ntile > 0 ? ntile : 1))) ||
+        (e = dalloc(A.part, (size_t)(want_grad ? 5 : 2) * (npart > 0 ? npart : 1))))
         return e;
     if (nSel) {
         if ((e = cudaMemcpyAsync(A.slots.p, slots.data(), nSel * sizeof(PotSlot), cudaMemcpyHostToDevice, st)))
             return e;
-        if ((e = cudaMemsetAsync(A.E.p, 0, nSel * sizeof(double), st))) return e;
+        if ((e = cudaMemsetAsync(A.E.p, 0, nclear * sizeof(double), st))) return e;
     }
     if ((e = cudaMemsetAsync(A.out.p, 0, 3 * (size_t)(n > 0 ? n : 1) * sizeof(float), st))) return e;
     if (!nitems) return cudaSuccess;
-    if ((e = cudaMemsetAsync(A.acc.p, 0, (size_t)na * nrows * sizeof(double), st))) return e;
     PotAdjArgs a;
     a.slots = reinterpret_cast<const PotSlot *>(A.slots.p);
     a.nslot = nSel;
-    a.chunk = chunk;
     a.nitems = nitems;
     a.nrows = nrows;
     a.gstart = G.start.p;
@@ -938,8 +996,13 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
     a.tlo = A.tbox.p;
     a.thi = A.tbox.p + ntile;
     a.ntile = ntile;
-    a.acc = A.acc.p;
+    a.pphi = reinterpret_cast<float2 *>(A.part.p);
+    a.pgx = A.part.p + 2 * npart;
+    a.pgy = a.pgx + npart;
+    a.pgz = a.pgy + npart;
+    a.eblock = A.eblock.p;
     a.E = A.E.p;
+    a.done = reinterpret_cast<int *>(A.E.p + nE);
     a.grad = want_grad ? A.out.p : nullptr;
     const long long most = (long long)num_sms() * 32;
     const int rgrid = grid_for((int)(nrows < (1 << 30) ? nrows : 1 << 30));
@@ -958,13 +1021,18 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
     pa_pack<<<rgrid, 256, 0, st>>>(a); note_launch();
     pa_boxes<<<grid_for((int)(ntile < (1 << 25) ? ntile * 32 : 1 << 30)), 256, 0, st>>>(a); note_launch();
     const int blocks = (int)(nitems < most ? nitems : most);
-    if (want_grad) potential_adjoint_kernel<true><<<blocks, PA_THREADS, 0, st>>>(a);
-    else potential_adjoint_kernel<false><<<blocks, PA_THREADS, 0, st>>>(a);
-    note_launch();
-    pa_energy<<<nSel < num_sms() * 4 ? nSel : num_sms() * 4, PE_THREADS, 0, st>>>(a); note_launch();
+    const bool parts = npart >= PA_PARTS_MIN * nrows;
+    const int fblocks = (int)std::min(most, ntile * (parts ? PA_PARTS : 1));
     if (want_grad) {
-        pa_gradient<<<rgrid, 256, 0, st>>>(a); note_launch();
+        potential_adjoint_kernel<true><<<blocks, PA_THREADS, 0, st>>>(a); note_launch();
+        if (parts) pa_finish<true, PA_PARTS><<<fblocks, PA_TILE, 0, st>>>(a);
+        else pa_finish<true, 1><<<fblocks, PA_TILE, 0, st>>>(a);
+    } else {
+        potential_adjoint_kernel<false><<<blocks, PA_THREADS, 0, st>>>(a); note_launch();
+        if (parts) pa_finish<false, PA_PARTS><<<fblocks, PA_TILE, 0, st>>>(a);
+        else pa_finish<false, 1><<<fblocks, PA_TILE, 0, st>>>(a);
     }
+    note_launch();
     return cudaGetLastError();
 }
 
