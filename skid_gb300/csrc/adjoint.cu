@@ -551,6 +551,23 @@ __device__ __forceinline__ int pa_slot(const PotAdjArgs &a, long long k, long lo
     return lo;
 }
 
+// The same for a whole warp and one k, 32 slots at a time: each step of the
+// search is a load that the next one waits for, the most of a call on many
+// small groups.
+__device__ __forceinline__ int pa_slot_warp(const PotAdjArgs &a, long long k, long long PotSlot::*start)
+{
+    const int lane = threadIdx.x & 31;
+    int lo = 0, count = a.nslot;
+    while (count > 1) {
+        const int step = (count + 31) / 32;
+        const bool before = lane * step < count && (lane == 0 || a.slots[lo + lane * step].*start <= k);
+        const int j = 31 - __clz(__ballot_sync(SKID_FULL, before));
+        lo += j * step;
+        count = min(step, count - j * step);
+    }
+    return lo;
+}
+
 __device__ __forceinline__ float3 pa_rel(const PotAdjArgs &a, const PotSlot &S, float4 p)
 {
     const float *rel = a.rec[S.g].rel;
@@ -592,38 +609,33 @@ __global__ void pa_keys(PotAdjArgs a, const unsigned *ext, uint64_t *keys, uint3
     }
 }
 
+// Pack the rows, a warp to each tile of PA_TILE, and the tile's box and largest
+// softening with them (one launch: a call on a small group is launches).
 __global__ void pa_pack(PotAdjArgs a)
-{
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < a.nrows;
-         k += (long long)gridDim.x * blockDim.x) {
-        const PotSlot S = a.slots[pa_slot(a, k, &PotSlot::row0)];
-        const long long from = a.perm ? (long long)a.perm[k] : k;
-        const int io = a.members[a.gstart[S.g] + (int)(from - S.row0)];
-        const float4 p = a.pos4[io];
-        const float3 r = pa_rel(a, S, p);
-        a.rm[k] = make_float4(r.x, r.y, r.z, p.w);
-        a.re[k] = a.vel4[io].w;
-        a.rio[k] = io;
-    }
-}
-
-// The box and largest softening of every tile of PA_TILE packed rows, a warp
-// each.
-__global__ void pa_boxes(PotAdjArgs a)
 {
     const int lane = threadIdx.x & 31;
     const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long t = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); t < a.ntile;
          t += nw) {
-        const PotSlot S = a.slots[pa_slot(a, t, &PotSlot::tile0)];
+        const PotSlot S = a.slots[pa_slot_warp(a, t, &PotSlot::tile0)];
         float4 lo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0.0f);
         float4 hi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f);
-        const int i0 = (int)(t - S.tile0) * PA_TILE;
-        for (int i = i0 + lane; i < min(i0 + PA_TILE, S.n); i += 32) {
-            const float4 r = a.rm[S.row0 + i];
+        const int i0 = (int)(t - S.tile0) * PA_TILE + lane, gs = a.gstart[S.g];
+#pragma unroll
+        for (int q = 0; q < PA_TILE / 32; ++q) {
+            const int i = i0 + 32 * q;
+            if (i >= S.n) continue;
+            const long long k = S.row0 + i;
+            const int io = a.members[gs + (a.perm ? (int)(a.perm[k] - S.row0) : i)];
+            const float4 p = a.pos4[io];
+            const float e = a.vel4[io].w;
+            const float3 r = pa_rel(a, S, p);
+            a.rm[k] = make_float4(r.x, r.y, r.z, p.w);
+            a.re[k] = e;
+            a.rio[k] = io;
             lo.x = fminf(lo.x, r.x); lo.y = fminf(lo.y, r.y); lo.z = fminf(lo.z, r.z);
             hi.x = fmaxf(hi.x, r.x); hi.y = fmaxf(hi.y, r.y); hi.z = fmaxf(hi.z, r.z);
-            lo.w = fmaxf(lo.w, a.re[S.row0 + i]);
+            lo.w = fmaxf(lo.w, e);
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) {
@@ -679,14 +691,54 @@ struct PaCol {
     ulonglong2 xy, zm;
 };
 
+// The sum of a tile's rows' values in row order, warps first: thread t holds
+// row t (and, Q = 2, row t + PA_TILE / 2).
+template <int Q>
+__device__ __forceinline__ double pa_tile_sum(const double (&v)[Q])
+{
+    __shared__ double red[PA_TILE / 32];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        double x = v[q];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(SKID_FULL, x, o);
+        if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) + q * (PA_TILE / 32 / Q)] = x;
+    }
+    __syncthreads();
+    double t = red[0];
+    for (int k = 1; k < PA_TILE / 32; ++k) t += red[k];
+    return t;
+}
+
+// A row's gradient by iOrder from its sums v over all columns, and its share
+// -1/2 G m phi of the energy.
 template <bool GRAD>
+__device__ __forceinline__ double pa_row_out(const PotAdjArgs &a, const PotSlot &S, float m, int io,
+                                             const double *v)
+{
+    if (GRAD) {
+        const float c = -a.G * m * S.v;
+        float *o = a.grad + 3 * (size_t)io;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) o[d] = c * (float)v[d + 1];
+    }
+    return -0.5 * (double)a.G * (double)m * (double)(float)v[0];
+}
+
+// ONE: every group of the call is one tile (and one chunk), and its energy and
+// gradient are written here: no pa_finish, the most of a call on small groups
+// being launches (100 groups of 50: 0.076 / 0.094 ms a call without / with the
+// gradient, 0.071 / 0.086 so).
+template <bool GRAD, bool ONE>
 __global__ void __launch_bounds__(PA_THREADS) potential_adjoint_kernel(PotAdjArgs a)
 {
     __shared__ PaCol sc[PA_TILE];
     __shared__ float ss[PA_TILE];
     const int tid = threadIdx.x;
     for (long long it = blockIdx.x; it < a.nitems; it += gridDim.x) {
-        const PotSlot S = a.slots[pa_slot(a, it, &PotSlot::item0)];
+        const int slot = pa_slot_warp(a, it, &PotSlot::item0);
+        const PotSlot S = a.slots[slot];
         const int tile = (int)(it - S.item0) / S.nchunk, ch = (int)(it - S.item0) - tile * S.nchunk;
         const int n = S.n;
         const float4 *rm = a.rm + S.row0;
@@ -764,6 +816,20 @@ __global__ void __launch_bounds__(PA_THREADS) potential_adjoint_kernel(PotAdjArg
         }
         const float2 phi = unpack2(w.phi), phic = unpack2(w.phic);
         const float2 hx = unpack2(w.gx), hy = unpack2(w.gy), hz = unpack2(w.gz);
+        if (ONE) {
+            double e[2] = {};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int i = q ? i1 : i0;
+                if (i >= n) continue;
+                const double v[4] = {q ? (double)phi.y + (double)phic.y : (double)phi.x + (double)phic.x,
+                                     q ? hx.y : hx.x, q ? hy.y : hy.x, q ? hz.y : hz.x};
+                e[q] = pa_row_out<GRAD>(a, S, q ? q1.w : q0.w, a.rio[S.row0 + i], v);
+            }
+            const double sum = pa_tile_sum(e);
+            if (tid == 0) a.E[slot] = sum;
+            continue;
+        }
         const size_t first = S.part0 + (size_t)ch * n;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -779,20 +845,6 @@ __global__ void __launch_bounds__(PA_THREADS) potential_adjoint_kernel(PotAdjArg
     }
 }
 
-// A sum over the block's threads in a fixed order.
-__device__ __forceinline__ double pa_block_sum(double v)
-{
-    __shared__ double red[PA_TILE / 32];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(SKID_FULL, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = red[0];
-    for (int k = 1; k < PA_TILE / 32; ++k) t += red[k];
-    return t;
-}
-
 // A block takes a row tile's rows (with PARTS = 4 a quarter of them, a warp to
 // each quarter of the chunks): their sums over all chunks, their gradient by
 // iOrder, and their energy -1/2 G sum_i m_i phi_i in FP64; the block that is
@@ -802,12 +854,12 @@ __device__ __forceinline__ double pa_block_sum(double v)
 template <bool GRAD, int PARTS>
 __global__ void __launch_bounds__(PA_TILE) pa_finish(PotAdjArgs a)
 {
-    constexpr int NA = GRAD ? 4 : 1, ROWS = PA_TILE / PARTS;
-    __shared__ double sums[PARTS][NA][ROWS];
+    constexpr int NA = 4, ROWS = PA_TILE / PARTS;
+    __shared__ double sums[PARTS][GRAD ? NA : 1][ROWS];
     __shared__ int last;
     const int tid = threadIdx.x, row = tid % ROWS, part = tid / ROWS;
     for (long long b = blockIdx.x; b < a.ntile * PARTS; b += gridDim.x) {
-        const int slot = pa_slot(a, b / PARTS, &PotSlot::tile0);
+        const int slot = pa_slot_warp(a, b / PARTS, &PotSlot::tile0);
         const PotSlot S = a.slots[slot];
         const int i = (int)(b - S.tile0 * PARTS) * ROWS + row;
         const bool in = i < S.n;
@@ -826,30 +878,22 @@ __global__ void __launch_bounds__(PA_TILE) pa_finish(PotAdjArgs a)
                 const float2 p = a.pphi[o];
                 v[0] += (double)p.x + (double)p.y;
                 if (GRAD) {
-                    v[1 % NA] += (double)a.pgx[o];
-                    v[2 % NA] += (double)a.pgy[o];
-                    v[3 % NA] += (double)a.pgz[o];
+                    v[1] += (double)a.pgx[o];
+                    v[2] += (double)a.pgy[o];
+                    v[3] += (double)a.pgz[o];
                 }
             }
         }
         if (PARTS > 1) {
             __syncthreads();
-            for (int d = 0; d < NA; ++d) sums[part][d][row] = v[d];
+            for (int d = 0; d < (GRAD ? NA : 1); ++d) sums[part][d][row] = v[d];
             __syncthreads();
             if (part == 0)
                 for (int k = 1; k < PARTS; ++k)
-                    for (int d = 0; d < NA; ++d) v[d] += sums[k][d][row];
+                    for (int d = 0; d < (GRAD ? NA : 1); ++d) v[d] += sums[k][d][row];
         }
-        double e = 0.0;
-        if (in && part == 0) {
-            e = -0.5 * (double)a.G * (double)m * (double)(float)v[0];
-            if (GRAD) {
-                const float c = -a.G * m * S.v;
-                float *o = a.grad + 3 * (size_t)io;
-                for (int d = 0; d < 3; ++d) o[d] = c * (float)v[(d + 1) % NA];
-            }
-        }
-        e = pa_block_sum(e);
+        double mine[1] = {in && part == 0 ? pa_row_out<GRAD>(a, S, m, io, v) : 0.0};
+        double e = pa_tile_sum(mine);
         const int nb = (S.n + PA_TILE - 1) / PA_TILE * PARTS;
         if (nb > 1) {
             if (tid == 0) {
@@ -860,9 +904,9 @@ __global__ void __launch_bounds__(PA_TILE) pa_finish(PotAdjArgs a)
             __syncthreads();
             if (!last) continue;
             __threadfence();
-            e = 0.0;
-            for (int k = tid; k < nb; k += PA_TILE) e += __ldcg(&a.eblock[S.tile0 * PARTS + k]);
-            e = pa_block_sum(e);
+            mine[0] = 0.0;
+            for (int k = tid; k < nb; k += PA_TILE) mine[0] += __ldcg(&a.eblock[S.tile0 * PARTS + k]);
+            e = pa_tile_sum(mine);
         }
         if (tid == 0) a.E[slot] = e;
     }
@@ -940,6 +984,7 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
     while (chunk > PA_CHUNK_MIN && pairs < (double)(PA_FILL * num_sms()) * PA_TILE * chunk) chunk >>= 1;
     std::vector<PotSlot> slots(nSel);
     long long nitems = 0, nrows = 0, ntile = 0, npart = 0;
+    bool one = true;            // every group one tile of one chunk
     for (int s = 0; s < nSel; ++s) {
         const int c = counts[h_sel[s]];
         PotSlot &S = slots[s];
@@ -956,6 +1001,7 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
         nrows += c;
         ntile += (c + PA_TILE - 1) / PA_TILE;
         npart += (long long)c * S.nchunk;
+        one = one && c <= std::min(PA_TILE, S.chunk);
     }
     // energies, then the counts of finished blocks, cleared together
     const size_t nE = nSel > 0 ? nSel : 1, nclear = nE + (nE + 1) / 2;
@@ -973,7 +1019,7 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
             return e;
         if ((e = cudaMemsetAsync(A.E.p, 0, nclear * sizeof(double), st))) return e;
     }
-    if ((e = cudaMemsetAsync(A.out.p, 0, 3 * (size_t)(n > 0 ? n : 1) * sizeof(float), st))) return e;
+    if (want_grad && (e = cudaMemsetAsync(A.out.p, 0, 3 * (size_t)(n > 0 ? n : 1) * sizeof(float), st))) return e;
     if (!nitems) return cudaSuccess;
     PotAdjArgs a;
     a.slots = reinterpret_cast<const PotSlot *>(A.slots.p);
@@ -1018,17 +1064,22 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
         if ((e = radix_sort(ss, (int)nrows, PA_KEY_BITS + sbits, st))) return e;
         a.perm = ss.v0.p;
     }
-    pa_pack<<<rgrid, 256, 0, st>>>(a); note_launch();
-    pa_boxes<<<grid_for((int)(ntile < (1 << 25) ? ntile * 32 : 1 << 30)), 256, 0, st>>>(a); note_launch();
+    pa_pack<<<grid_for((int)(ntile < (1 << 25) ? ntile * 32 : 1 << 30), 128), 128, 0, st>>>(a); note_launch();
     const int blocks = (int)(nitems < most ? nitems : most);
+    if (one) {
+        if (want_grad) potential_adjoint_kernel<true, true><<<blocks, PA_THREADS, 0, st>>>(a);
+        else potential_adjoint_kernel<false, true><<<blocks, PA_THREADS, 0, st>>>(a);
+        note_launch();
+        return cudaGetLastError();
+    }
     const bool parts = npart >= PA_PARTS_MIN * nrows;
     const int fblocks = (int)std::min(most, ntile * (parts ? PA_PARTS : 1));
     if (want_grad) {
-        potential_adjoint_kernel<true><<<blocks, PA_THREADS, 0, st>>>(a); note_launch();
+        potential_adjoint_kernel<true, false><<<blocks, PA_THREADS, 0, st>>>(a); note_launch();
         if (parts) pa_finish<true, PA_PARTS><<<fblocks, PA_TILE, 0, st>>>(a);
         else pa_finish<true, 1><<<fblocks, PA_TILE, 0, st>>>(a);
     } else {
-        potential_adjoint_kernel<false><<<blocks, PA_THREADS, 0, st>>>(a); note_launch();
+        potential_adjoint_kernel<false, false><<<blocks, PA_THREADS, 0, st>>>(a); note_launch();
         if (parts) pa_finish<false, PA_PARTS><<<fblocks, PA_TILE, 0, st>>>(a);
         else pa_finish<false, 1><<<fblocks, PA_TILE, 0, st>>>(a);
     }
