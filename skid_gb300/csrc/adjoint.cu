@@ -485,24 +485,38 @@ __device__ __forceinline__ float wrap_rel(float d, float h)
 // and a count per item, cost 8 % at short chunks.)
 constexpr int PA_TILE = 128;
 constexpr int PA_THREADS = PA_TILE / 2;
-// Columns per item: long ones (fewer partial sums) once the pairs fill every
-// SM with PA_FILL items of that length, short ones below, where an item's
-// serial walk over its columns would set the time.
-constexpr int PA_CHUNK = 1024, PA_CHUNK_MIN = 128;
-constexpr long long PA_FILL = 32;
-// From this many pairs the members are packed in Hilbert order: a warp takes
-// the softened pair factor (divides, a root) whenever any of its pairs lies
-// inside the softening, and with members in file order some pair of 64 does
-// in 40-50 % of the steps of a halo whose pairs are 2-3 % inside it; in
-// Hilbert order in 12-20 %.  2.9e9 pairs: 3.14 ms
-// (with gradient) and 2.31 ms in file order, 2.49 and 1.75 ms in Hilbert
-// order, for 0.1 ms of sorting.
-constexpr double PA_SORT_PAIRS = 1.5e8;
-
-// A group has at most this many chunks (longer ones from 64 x PA_CHUNK members
-// on), which bounds the memory its rows' partial sums take.
-constexpr int PA_MAX_CHUNKS = 64;
+// Columns per item: 1024 once the pairs make PA_FILL items of that length for
+// every SM, halved below until they do, at least 128.  A long walk over columns
+// saves partial sums, and leaves SMs idle at the end.  A call's time without /
+// with the gradient at 128, 256, 512, 1024 columns (chosen: *), ms:
+//   one group of 8,660           .15 / .21*    .16 / .22     .17 / .22     .25 / .30
+//   one group of 17,000          .36 / .47*    .39 / .51     .47 / .58     .70 / .85
+//   20 groups of up to 19,700    .72 / 1.03    .70 / .93*    .79 / 1.04    .84 / 1.07
+//   8 groups of 17,000          1.64 / 2.36   1.56 / 2.18   1.69 / 2.33*  1.94 / 2.43
+//   300 groups of 3,000         2.51 / 3.43   2.30 / 3.11   2.25 / 3.00   2.27 / 2.97*
+//   4,000 groups of 1,000       5.85 / 9.55   5.23 / 8.75   4.87 / 8.26   4.36 / 7.58*
+// A group has at most PA_MAX_CHUNKS (longer ones from 131,072 members on), which
+// bounds the memory of its rows' partial sums (20 B each with the gradient, 8 B
+// without); 64 took 0.43 / 0.54 for the group of 17,000.
+constexpr int PA_CHUNK = 1024, PA_CHUNK_MIN = 128, PA_MAX_CHUNKS = 128;
+constexpr long long PA_FILL = 128;
+// From PA_SORT_PAIRS pairs an SM (4e8 on 152) where a row meets PA_SORT_COLS
+// columns or more, and from PA_SORT_ANY (2e9) in any case, the members are
+// packed in Hilbert order: a warp takes the softened pair factor (divides, a
+// root) whenever any of its pairs lies inside the softening, and with members
+// in file order some pair of 64 does in 40-50 % of the steps of a halo whose
+// pairs are 2-3 % inside it; in Hilbert order in 12-20 %, and in a group of
+// many tiles most pairs of tiles are beyond the softening as a whole; for 0.1 ms
+// of sorting and more with a million rows.  File order / Hilbert order without
+// the gradient, ms:
+//   one group of 17,000 (2.9e8 pairs)    .35 / .43    20 of up to 19,700 (8.7e8)  .79 / .70
+//   8 of 8,660 (6e8)                     .68 / .63    one of 35,000 (1.2e9)      1.21 / .89
+//   300 of up to 6,600 (9.3e8)           .78 / .85    8 of 17,000 (2.3e9)        2.22 / 1.70
+//   1,000 of up to 4,900 (1.8e9)        1.43 / 1.50   300 of 3,000 (2.7e9)       2.75 / 2.20
+constexpr double PA_SORT_PAIRS = 2.6e6, PA_SORT_COLS = 4000.0, PA_SORT_ANY = 1.3e7;
 // Rows with this many chunks on average have them added by PA_PARTS warps.
+// One / four: one group of 8,660 (68 chunks) with the gradient .228 / .211 ms,
+// 150 groups of 1,000 (8) .472 / .492, 4,000 of 1,000 (1) 7.57 / 7.94.
 constexpr int PA_PARTS = 4, PA_PARTS_MIN = 16;
 
 struct PotSlot {
@@ -1052,7 +1066,9 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
     a.grad = want_grad ? A.out.p : nullptr;
     const long long most = (long long)num_sms() * 32;
     const int rgrid = grid_for((int)(nrows < (1 << 30) ? nrows : 1 << 30));
-    if (pairs >= PA_SORT_PAIRS && nrows < (1ll << 31)) {
+    const double perSM = pairs / num_sms();
+    if ((perSM >= PA_SORT_ANY || (perSM >= PA_SORT_PAIRS && pairs >= PA_SORT_COLS * nrows)) &&
+        nrows < (1ll << 31)) {
         int sbits = 0;
         while ((1ll << sbits) < nSel) ++sbits;
         if ((e = dalloc(ss.k0, (size_t)nrows)) || (e = dalloc(ss.k1, (size_t)nrows)) ||
