@@ -132,13 +132,16 @@ __device__ __forceinline__ float warp_max(float v)
 // call with its tree, 2^18 points: k = 128 3.81 to 2.78 ms, 32 1.24 to 1.05, 24
 // 1.06 to 0.94, 16 0.83 to 0.84 (so the heaps keep small k; above 128 the
 // buffers would leave too few warps an SM).  Bound by instruction issue at
-// half the slots: 12 warps an SM, each a chain.  Room for 48 or 96 values
+// half the slots: 13 warps an SM, each a chain.  Room for 48 or 96 values
 // beyond k, and cutting closer or less, were slower.  Counting distances into
 // radial bins instead, with a second walk to pick from the k-th one's, took
 // 62k instructions and had a longer tail: no faster.
 constexpr int KB_MINK = 24, KB_MAXK = 128;
 constexpr int KB_SLACK = 64;         // values a buffer holds beyond k
 constexpr int KB_STEP = 8;           // candidates tested between checks for room
+// Counts at guessed values, and all counts before the values themselves are
+// asked (few lanes are left by then where distances differ; sooner costs 6 %).
+constexpr int KB_GUESSES = 6, KB_TIGHTEN = 10;
 
 struct KnnBuf {
     float *b;        // this lane's values, stride 32
@@ -188,20 +191,51 @@ __device__ __forceinline__ float kb_largest(const KnnBuf &B, int m)
     return v;
 }
 
+// The least value's pattern above l, and the largest up to h.
+__device__ __noinline__ int2 kb_span(const float *values, int m, int l, int h)
+{
+    const int *b = reinterpret_cast<const int *>(values);
+    int2 v = make_int2(0x7f800000, 0);
+#pragma unroll 8
+    for (int i = 0; i < m; ++i) {
+        const int x = b[i * 32];
+        v.x = x > l ? min(v.x, x) : v.x;
+        v.y = x <= h ? max(v.y, x) : v.y;
+    }
+    return v;
+}
+
 // The k-th smallest of the values that S lanes hold together (each its own
 // buffer), between lo (fewer than k values at or below it; -1: none are) and hi
 // (k or more): guesses from the counts, of which lo's is cl and hi's near ch,
-// then bisection of the bit patterns.  Lanes that are done have no use for it.
+// then bisection of the bit patterns, then (it >= KB_TIGHTEN) of those between
+// the least and the largest value left: where many distances are equal but for
+// rounding (a lattice, a shell of it at the k-th) no count is k and the values
+// are a few patterns apart.  200,000 points of a lattice, k = 128: 2.53 to 2.20
+// ms.  Lanes that are done have no use for it.
 template <int S>
 __device__ __forceinline__ float kb_kth(const KnnBuf &B, int m, int k, int lo, float hi, int cl, int ch,
-                                        bool done)
+                                        bool done, int it = 0)
 {
     int l = lo, h = __float_as_int(hi);
     bool largest = false;
-    for (int it = 0; __any_sync(SKID_FULL, !done); ++it) {
+    for (; __any_sync(SKID_FULL, !done); ++it) {
         if (!done && h - l <= 1) done = true;      // h is the answer
+        if (it == KB_TIGHTEN) {
+            int2 v = kb_span(B.b, m, l, h);
+#pragma unroll
+            for (int o = 1; o < S; o <<= 1) {
+                v.x = min(v.x, __shfl_xor_sync(SKID_FULL, v.x, o));
+                v.y = max(v.y, __shfl_xor_sync(SKID_FULL, v.y, o));
+            }
+            if (!done) {
+                l = v.x - 1;
+                h = v.y;
+                done = h - l <= 1;
+            }
+        }
         int mid = l + (h - l) / 2;
-        if (it < 6) {
+        if (it < KB_GUESSES) {
             const float a = l < 0 ? 0.0f : __int_as_float(l), b = __int_as_float(h);
             float t = (k + 0.0f - cl) / fmaxf((float)(ch - cl), 1.0f);
             if (cl == 0) t = exp2f(0.6666667f * log2f(t));
@@ -248,7 +282,7 @@ __device__ __noinline__ KnnBuf kb_cut(KnnBuf B, int k, int most)
     bool done = ch <= k + (most - k) / 4;
     const bool skip = done;
     const float aim = k + 0.15f * (most - k);
-    for (int it = 0; it < 6 && __any_sync(SKID_FULL, !done); ++it) {
+    for (int it = 0; it < KB_GUESSES && __any_sync(SKID_FULL, !done); ++it) {
         float t = (aim - cl) / fmaxf((float)(ch - cl), 1.0f);
         if (cl == 0) t = exp2f(0.6666667f * log2f(t));
         const float mid = fmaf(hi - lo, fminf(fmaxf(t, 0.02f), 0.98f), lo);
@@ -269,7 +303,7 @@ __device__ __noinline__ KnnBuf kb_cut(KnnBuf B, int k, int most)
     const bool tight = !done && (SHARED || B.n >= k);
     int room = 0x7fffffff;
     if (__any_sync(SKID_FULL, tight)) {
-        const float e = kb_kth<1>(B, m, k, cl == 0 ? -1 : __float_as_int(lo), hi, cl, ch, !tight);
+        const float e = kb_kth<1>(B, m, k, cl == 0 ? -1 : __float_as_int(lo), hi, cl, ch, !tight, KB_TIGHTEN);
         int below = 0;
 #pragma unroll 8
         for (int i = 0; i < m; ++i) below += B.b[i * 32] < e;
