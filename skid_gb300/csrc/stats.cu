@@ -13,11 +13,11 @@
 //   2. a stable radix sort of (key, iOrder) puts every group's members in
 //      radius order, ties in iOrder order;
 //   3. one thread per sorted slot marks where each group's run starts;
-//   4. one warp per group walks its run outwards with the reference's own
-//      float and double operations, each rounded as gcc rounds it, so the
-//      running sums and the maximum / half-mass decisions are the
-//      reference's (the sums are inherently sequential: each depends on the
-//      float rounding of the previous one).
+//   4. one warp (for a few members, one thread) per group walks its run
+//      outwards with the reference's own float and double operations, each
+//      rounded as gcc rounds it, so the running sums and the maximum /
+//      half-mass decisions are the reference's (the sums are inherently
+//      sequential: each depends on the float rounding of the previous one).
 #include <cfloat>
 
 #include "ctx.h"
@@ -80,6 +80,7 @@ struct StatArgs {
     float3 h;
     float G, fExp, fExpHub, fDensMin, fTempMax;
     skid_stat *out;
+    int small;                  // groups of up to so many members take a thread
 };
 
 // The running float sums of one group are a serial chain: each add waits for
@@ -93,6 +94,14 @@ struct StatArgs {
 // one thread per group (every load, divide and root in the one chain) the 150k
 // mixed-species snapshot took 19.5 ms, its largest group of some 14k members
 // setting the time; now about 0.36 ms.
+//
+// Where there are ST_MANY groups an SM, those of up to ST_THREAD_MAX members
+// take a thread each after all: their FP64 roots and divides (a member's
+// circular velocity, five more a group) use as many issue slots for one group
+// as for 32.  A warp / a thread a group, ms a call: 3,000 groups of 8 .13 / .13,
+// of 30 .14 / .18; 10,000 of 8 .18 / .14, of 30 .21 / .20; 40,000 of 5 .37 /
+// .20, of 16 .42 / .28, of 30 .47 / .35.
+constexpr int ST_THREAD_MAX = 32, ST_MANY = 64;
 constexpr int ST_WARPS = 2;
 constexpr int ST_ROW = 97;   // 3 adds for each of 32 members, one word of padding
 
@@ -117,6 +126,94 @@ __device__ __forceinline__ void stat_load(const StatArgs &A, int s, int n, int j
     q.gas = q.io < A.nGas && A.rho[q.io] >= A.fDensMin && A.temp[q.io] <= A.fTempMax;
 }
 
+// dv = fExp*(v - vcm) + fExpHub*r (float, kd.c:1792-1796), squared.
+__device__ __forceinline__ float stat_dv2(const StatArgs &A, float v, float vcm, float r)
+{
+    const float dv = fadd(fmul(A.fExp, fsub(v, vcm)), fmul(A.fExpHub, r));
+    return fmul(dv, dv);
+}
+
+// What follows the walk (kd.c:1798-1803); r2 is the outermost member's.
+__device__ __forceinline__ void stat_store(const StatArgs &A, int g, int n, float fTot, float fGas,
+                                           float fStar, float fVc, float fmVc, float fRVmax, float fRh,
+                                           float r2, float fVd)
+{
+    const float flVc = (float)__ddiv_rn((double)fmul(A.G, fTot), __dsqrt_rn((double)r2));
+    if (fVc == 0.0f) {
+        fVc = flVc;
+        fRVmax = (float)__dsqrt_rn((double)r2);
+    }
+    fVd = (float)__dsqrt_rn(__ddiv_rn((double)fVd, __dmul_rn(3.0, (double)n)));
+    skid_stat o;
+    o.nMembers = n;
+    o.fTotMass = fTot;
+    o.fGasMass = fGas;
+    o.fStarMass = fStar;
+    o.fVcirc2Max = fVc;
+    o.fVcirc2Half = fmVc;
+    o.fVcirc2Outer = flVc;
+    o.fRVmax = fRVmax;
+    o.fRHalf = fRh;
+    o.fROuter2 = r2;
+    o.fVdisp = fVd;
+    A.out[g] = o;
+}
+
+// A group without members.
+__device__ __forceinline__ void stat_none(const StatArgs &A, int g, int n)
+{
+    skid_stat o = {};
+    o.nMembers = n;
+    A.out[g] = o;
+}
+
+// A group on one thread, member by member.
+__device__ void stat_thread(const StatArgs &A, int g)
+{
+    const skid_group rg = A.rec[g];
+    const int n = rg.nMembers, s = A.start[g];
+    if (n <= 0) return stat_none(A, g, n);
+    // kd.c:1766-1767: fHalfMass += 0.5*fMass (FP64 sum rounded to float)
+    float fHalf = 0.0f;
+    for (int j = 0; j < n; ++j)
+        fHalf = (float)__dadd_rn((double)fHalf, __dmul_rn(0.5, (double)A.pos4[A.vals[s + j]].w));
+    float fTot = 0.0f, fGas = 0.0f, fStar = 0.0f, fVc = 0.0f, fmVc = 0.0f, fVd = 0.0f;
+    float fRVmax = 0.0f, fRh = 0.0f;
+    StatMember q, nx;
+    stat_load(A, s, n, 0, nx);
+    for (int j = 0; j < n; ++j) {
+        q = nx;
+        stat_load(A, s, n, j + 1, nx);
+        fTot = fadd(fTot, q.p.w);
+        // kd.c:1774-1778: r2 > 4.0*soft*soft && G*fTot/sqrt(r2) > fVcirc
+        // (FP64 comparisons); fRVmax = sqrt(r2), fVcirc = G*fTot/fRVmax (float)
+        const double d2 = (double)q.r2;
+        const float gm = fmul(A.G, fTot);
+        if (d2 > __dmul_rn(__dmul_rn(4.0, (double)q.v.w), (double)q.v.w) &&
+            __ddiv_rn((double)gm, __dsqrt_rn(d2)) > (double)fVc) {
+            fRVmax = (float)__dsqrt_rn(d2);
+            fVc = __fdiv_rn(gm, fRVmax);
+        }
+        if (q.gas) fGas = fadd(fGas, q.p.w);
+        if (q.io >= A.nGas + A.nDark) fStar = fadd(fStar, q.p.w);
+        if (fTot > fHalf && fmVc == 0.0f) {
+            fRh = (float)__dsqrt_rn(d2);
+            fmVc = __fdiv_rn(gm, fRh);
+        }
+        const float3 r = stat_rel(q.p, rg, A.h);
+        fVd = fadd(fVd, stat_dv2(A, q.v.x, rg.vcm[0], r.x));
+        fVd = fadd(fVd, stat_dv2(A, q.v.y, rg.vcm[1], r.y));
+        fVd = fadd(fVd, stat_dv2(A, q.v.z, rg.vcm[2], r.z));
+    }
+    stat_store(A, g, n, fTot, fGas, fStar, fVc, fmVc, fRVmax, fRh, q.r2, fVd);
+}
+
+__global__ void stat_small_groups(StatArgs A)
+{
+    const int g = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    if (g < A.nGroup && A.rec[g].nMembers <= A.small) stat_thread(A, g);
+}
+
 __global__ void __launch_bounds__(ST_WARPS * 32) stat_groups(StatArgs A)
 {
     __shared__ float term_s[ST_WARPS][4][ST_ROW];
@@ -128,13 +225,9 @@ __global__ void __launch_bounds__(ST_WARPS * 32) stat_groups(StatArgs A)
     float *tot = tot_s[w];
     const skid_group rg = A.rec[g];
     const int n = rg.nMembers, s = A.start[g];
-    skid_stat o;
-    o.nMembers = n;
+    if (A.small && n <= A.small) return;
     if (n <= 0) {
-        o.fTotMass = o.fGasMass = o.fStarMass = 0.0f;
-        o.fVcirc2Max = o.fVcirc2Half = o.fVcirc2Outer = 0.0f;
-        o.fRVmax = o.fRHalf = o.fROuter2 = o.fVdisp = 0.0f;
-        if (lane == 0) A.out[g] = o;
+        if (lane == 0) stat_none(A, g, n);
         return;
     }
     // kd.c:1766-1767: fHalfMass += 0.5*fMass (FP64 sum rounded to float).  The
@@ -188,9 +281,8 @@ __global__ void __launch_bounds__(ST_WARPS * 32) stat_groups(StatArgs A)
         const float vv[3] = {q.v.x, q.v.y, q.v.z}, rr[3] = {r.x, r.y, r.z};
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            // kd.c:1792-1796: dv = fExp*(v - vcm) + fExpHub*r (float)
-            const float dv = fadd(fmul(A.fExp, fsub(vv[k], rg.vcm[k])), fmul(A.fExpHub, rr[k]));
-            term[3][3 * lane + k] = in ? fmul(dv, dv) : 0.0f;
+            const float d = stat_dv2(A, vv[k], rg.vcm[k], rr[k]);
+            term[3][3 * lane + k] = in ? d : 0.0f;
         }
         __syncwarp();
         if (lane < 4) {
@@ -247,30 +339,12 @@ __global__ void __launch_bounds__(ST_WARPS * 32) stat_groups(StatArgs A)
             cur = l + 1;
         }
     }
-    // kd.c:1798-1803: r2 is the outermost member's
     const float r2 = __shfl_sync(SKID_FULL, q.r2, (n - 1) & 31);
     const float fTot = __shfl_sync(SKID_FULL, sum, 0);
     const float fGas = __shfl_sync(SKID_FULL, sum, 1);
     const float fStar = __shfl_sync(SKID_FULL, sum, 2);
-    float fVd = __shfl_sync(SKID_FULL, sum, 3);
-    if (lane != 0) return;
-    const float flVc = (float)__ddiv_rn((double)fmul(A.G, fTot), __dsqrt_rn((double)r2));
-    if (fVc == 0.0f) {
-        fVc = flVc;
-        fRVmax = (float)__dsqrt_rn((double)r2);
-    }
-    fVd = (float)__dsqrt_rn(__ddiv_rn((double)fVd, __dmul_rn(3.0, (double)n)));
-    o.fTotMass = fTot;
-    o.fGasMass = fGas;
-    o.fStarMass = fStar;
-    o.fVcirc2Max = fVc;
-    o.fVcirc2Half = fmVc;
-    o.fVcirc2Outer = flVc;
-    o.fRVmax = fRVmax;
-    o.fRHalf = fRh;
-    o.fROuter2 = r2;
-    o.fVdisp = fVd;
-    A.out[g] = o;
+    const float fVd = __shfl_sync(SKID_FULL, sum, 3);
+    if (lane == 0) stat_store(A, g, n, fTot, fGas, fStar, fVc, fmVc, fRVmax, fRh, r2, fVd);
 }
 
 int bits_for_groups(int ng)
@@ -322,6 +396,10 @@ extern "C" int skid_group_stats(skid_ctx *ctx, float G, float fExp, float fExpHu
     A.fDensMin = fDensMin;
     A.fTempMax = fTempMax;
     A.out = ctx->stat_out.p;
+    A.small = ng - 1 >= ST_MANY * num_sms() ? ST_THREAD_MAX : 0;
+    if (A.small) {
+        stat_small_groups<<<(ng - 1 + 63) / 64, 64, 0, st>>>(A); note_launch();
+    }
     stat_groups<<<(ng - 1 + ST_WARPS - 1) / ST_WARPS, ST_WARPS * 32, 0, st>>>(A); note_launch();
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(stats, ctx->stat_out.p, ng * sizeof(skid_stat), cudaMemcpyDeviceToHost, st));
