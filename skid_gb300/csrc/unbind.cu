@@ -1109,7 +1109,12 @@ struct BlockGroup {
     int *qid;
     long long *pot;
     float *sm;                       // records in shared memory
-    float4 *ga, *gb;                 // state in global memory, by slot
+    // state in global memory, by slot: (u, v, w, x), (y, z) and, all that a
+    // pass writes, (p, c): whole sectors, where a member's 32 bytes in two
+    // float4s had two sectors written for four bytes each.  Without a
+    // potential to take off a pass reads no y and z.
+    float4 *gux;
+    float2 *gyz, *gpc;
     int cap;                         // slots in shared memory
     int tid, lane, w;
     int n, nfl;                      // live members; slots below nfl have potentials as of then
@@ -1127,6 +1132,13 @@ struct BlockGroup {
         return (((k >> 1) * BC + t) << 2) + (k & 1);
     }
     // (x, y, z, p) and (u, v, w, c) of a slot
+    __device__ __forceinline__ void gget(int i, float4 &a, float4 &b, bool yz = true) const
+    {
+        const float4 r = gux[i];
+        const float2 p = gpc[i], v = yz ? gyz[i] : make_float2(0.0f, 0.0f);
+        a = make_float4(r.w, v.x, v.y, p.x);
+        b = make_float4(r.x, r.y, r.z, p.y);
+    }
     __device__ __forceinline__ void get(int i, float4 &a, float4 &b) const
     {
         if (i < cap) {
@@ -1135,8 +1147,7 @@ struct BlockGroup {
             a = make_float4(q[0], q[2], q[c2], q[c2 + 2]);
             b = make_float4(q[2 * c2], q[2 * c2 + 2], q[3 * c2], q[3 * c2 + 2]);
         } else {
-            a = ga[i];
-            b = gb[i];
+            gget(i, a, b);
         }
     }
     __device__ __forceinline__ void put(int i, float4 a, float4 b) const
@@ -1147,8 +1158,9 @@ struct BlockGroup {
             q[0] = a.x; q[2] = a.y; q[c2] = a.z; q[c2 + 2] = a.w;
             q[2 * c2] = b.x; q[2 * c2 + 2] = b.y; q[3 * c2] = b.z; q[3 * c2 + 2] = b.w;
         } else {
-            ga[i] = a;
-            gb[i] = b;
+            gux[i] = make_float4(b.x, b.y, b.z, a.x);
+            gyz[i] = make_float2(a.y, a.z);
+            gpc[i] = make_float2(a.w, b.w);
         }
     }
 
@@ -1280,12 +1292,13 @@ __device__ void block_group(const RemoveArgs &A, int g, BlockShared<BS> &S, floa
     // slots in shared memory: whole records of a row of BC threads
     const int cap = A.lcap / (2 * BC) * (2 * BC);
     float *sm = reinterpret_cast<float *>(dyn);
-    float4 *ga = A.qa + s, *gb = A.qw + s;
+    float4 *gux = A.qa + s;
+    float2 *gyz = reinterpret_cast<float2 *>(A.qw + s), *gpc = gyz + n0;
     int n = n0, nfl = n0;
     bool force = false;
     const float epot = A.inv_scale * A.opz;
     auto view = [&]() {
-        return BG{A, S, qr, qv, qid, pot, sm, ga, gb, cap, tid, lane, w, n, nfl, epot, force};
+        return BG{A, S, qr, qv, qid, pot, sm, gux, gyz, gpc, cap, tid, lane, w, n, nfl, epot, force};
     };
     double m = 0.0, c[6] = {0, 0, 0, 0, 0, 0};
     for (int i = tid; i < n0; i += BS) {
@@ -1517,12 +1530,12 @@ __device__ void block_group(const RemoveArgs &A, int g, BlockShared<BS> &S, floa
                 float4 a[RG], b[RG];
 #pragma unroll
                 for (int k = 0; k < RG; ++k)
-                    if (i + k * BC < n) { a[k] = ga[i + k * BC]; b[k] = gb[i + k * BC]; }
+                    if (i + k * BC < n) B.gget(i + k * BC, a[k], b[k], sub);
 #pragma unroll
                 for (int k = 0; k < RG; ++k) {
                     if (i + k * BC >= n) break;
                     single(i + k * BC, a[k], b[k]);
-                    if (sub) { ga[i + k * BC].w = a[k].w; gb[i + k * BC].w = b[k].w; }
+                    if (sub) gpc[i + k * BC] = make_float2(a[k].w, b[k].w);
                 }
             }
             // the warp's largest energy and its member, and its second largest
