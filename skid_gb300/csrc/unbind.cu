@@ -500,7 +500,14 @@ __global__ void pot_fill(const uint32_t *__restrict__ order, const int *d_nvalid
 // boundary, tiny terms) to pot_pair: 300 groups of 400,000 particles 1.41 to
 // 1.15 ms, the groups of a 2^21-particle run 7.7 to 5.7.  Two columns a step
 // for more independent work took 1.9 and 6.1.
+//
+// Where such pairs are many, the packed operations come on top of pot_pair's:
+// when POT_SLOW of a tile pair's first POT_PROBE steps have one, its other
+// steps leave them out.  400,000 particles in one clump, most steps with a pair
+// inside the softening, 893 to 790 ms (769 without any packed operations); with
+// POT_SLOW 4 the 300 groups take 1.17 ms, 8 and 12 1.11.
 constexpr int POT_THREADS = POT_TILE / 2;
+constexpr int POT_PROBE = 16, POT_SLOW = 8;
 
 struct PotRow {
     float4 r;     // position, G m 2^S
@@ -624,48 +631,61 @@ pot_sym_kernel(const int2 *__restrict__ items, const int *d_nitems, int nitems_h
             const f32x2 zero = pack2(zero_arg, zero_arg), one = pack2(1.0f, 1.0f), half = pack2(0.5f, 0.5f),
                         neg1 = pack2(-1.0f, -1.0f);
             const float least = fmaxf(far, 1e-30f);
-            for (int k = 0; k < T; ++k) {
-                const int jl = (t + k) & (T - 1);
-                if (jl < nj) {
-                    const float4 rj = sr[jl];
-                    long long col;
-                    // pot_pair of both rows at once; ref_rsqrt's steps, where they decide
-                    const f32x2 dx = sub2(rx, pack2(rj.x, rj.x)), dy = sub2(ry, pack2(rj.y, rj.y)),
-                                dz = sub2(rz, pack2(rj.z, rj.z));
-                    const f32x2 x = add2(add2(sq2(dx, zero), sq2(dy, zero)), sq2(dz, zero));
-                    const float2 d2 = unpack2(x);
-                    const f32x2 y = pack2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y)), ny = mul2(y, neg1);
-                    const f32x2 nph = mul2(x, ny), pl = fma2(x, y, nph);
-                    const f32x2 r = fma2(pl, ny, fma2(nph, y, one));
-                    const f32x2 d = mul2(mul2(half, y), r), s2 = add2(y, d);
-                    const float2 e = unpack2(fma2(add2(s2, ny), neg1, d)), dir = unpack2(s2);
-                    const f32x2 wj = pack2(rj.w, rj.w);
-                    const float2 f = unpack2(mul2(wj, s2));
-                    const bool fast = fminf(d2.x, d2.y) >= least && fmaxf(d2.x, d2.y) <= 1e30f &&
-                                      rsqrt_decided(dir.x, e.x) && rsqrt_decided(dir.y, e.y) &&
-                                      fx_large(f.x) && fx_large(f.y);
-                    if (fast) {
-                        const long long ta = fx_shift(f.x), tb = fx_shift(f.y);
-                        acca += ta;
-                        accb += tb;
-                        if (rj.w == ra.r.w && rj.w == rb.r.w) {
-                            col = ta + tb;
-                        } else {
-                            const float2 c = unpack2(mul2(rw, s2));
-                            col = fx(c.x, 1.0f) + fx(c.y, 1.0f);
-                        }
-                    } else {
-                        long long tr, tc;
-                        pot_pair(ra, rj, ss[jl], plummer, far, tr, tc);
-                        acca += tr;
-                        col = tc;
-                        pot_pair(rb, rj, ss[jl], plummer, far, tr, tc);
-                        accb += tr;
-                        col += tc;
-                    }
-                    acc_w[wid][jl] += col;
+            // pot_pair of both rows at once, where every decision is plain:
+            // ref_rsqrt's steps, and the terms' mantissas shifted
+            auto both = [&](float4 rj, long long &col) {
+                const f32x2 dx = sub2(rx, pack2(rj.x, rj.x)), dy = sub2(ry, pack2(rj.y, rj.y)),
+                            dz = sub2(rz, pack2(rj.z, rj.z));
+                const f32x2 x = add2(add2(sq2(dx, zero), sq2(dy, zero)), sq2(dz, zero));
+                const float2 d2 = unpack2(x);
+                const f32x2 y = pack2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y)), ny = mul2(y, neg1);
+                const f32x2 nph = mul2(x, ny), pl = fma2(x, y, nph);
+                const f32x2 r = fma2(pl, ny, fma2(nph, y, one));
+                const f32x2 d = mul2(mul2(half, y), r), s2 = add2(y, d);
+                const float2 e = unpack2(fma2(add2(s2, ny), neg1, d)), dir = unpack2(s2);
+                const float2 f = unpack2(mul2(pack2(rj.w, rj.w), s2));
+                if (!(fminf(d2.x, d2.y) >= least && fmaxf(d2.x, d2.y) <= 1e30f &&
+                      rsqrt_decided(dir.x, e.x) && rsqrt_decided(dir.y, e.y) && fx_large(f.x) &&
+                      fx_large(f.y)))
+                    return false;
+                const long long ta = fx_shift(f.x), tb = fx_shift(f.y);
+                acca += ta;
+                accb += tb;
+                if (rj.w == ra.r.w && rj.w == rb.r.w) {
+                    col = ta + tb;
+                } else {
+                    const float2 c = unpack2(mul2(rw, s2));
+                    col = fx(c.x, 1.0f) + fx(c.y, 1.0f);
                 }
-                __syncwarp();
+                return true;
+            };
+            bool packed = true;
+            unsigned slow = 0;           // steps with a pair that was not
+            int k = 0;
+#pragma unroll 1
+            for (int end = POT_PROBE;; end = T) {
+#pragma unroll 1
+                for (; k < end; ++k) {
+                    const int jl = (t + k) & (T - 1);
+                    if (jl < nj) {
+                        const float4 rj = sr[jl];
+                        long long col;
+                        if (!(packed && both(rj, col))) {
+                            long long tr, tc;
+                            slow |= 1u << (k & 31);
+                            pot_pair(ra, rj, ss[jl], plummer, far, tr, tc);
+                            acca += tr;
+                            col = tc;
+                            pot_pair(rb, rj, ss[jl], plummer, far, tr, tc);
+                            accb += tr;
+                            col += tc;
+                        }
+                        acc_w[wid][jl] += col;
+                    }
+                    __syncwarp();
+                }
+                if (end == T) break;
+                packed = __popc(__reduce_or_sync(SKID_FULL, slow)) < POT_SLOW;
             }
         } else {
             // offset (column - row) mod T in 1..T/2 for row t (k = 1..H),
