@@ -2089,8 +2089,9 @@ __global__ void __launch_bounds__(RW_THREADS) remove_warps_kernel(const __grid_c
         if (item >= nvalid) break;
         warp_group(A, (int)A.order[item]);
     }
-    // the blocks' kernel, if it is still running, ends before this one does
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // the blocks' kernel, if it is still running, ends before this one does (one
+    // block sees to it: blocks that wait keep their SMs from other streams)
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Raise a removal kernel's shared-memory limit to all it can have, once per
