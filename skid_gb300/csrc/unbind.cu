@@ -1050,9 +1050,19 @@ __device__ void warp_group(const RemoveArgs &A, int g)
     __syncwarp();
 }
 
-// At most this many members near an extreme are evaluated exactly one warp
-// each; more bring every member's potential up to date.
+// Members near an extreme are evaluated exactly one by one, each with the terms
+// of all members removed since potentials were last brought up to date (a unit
+// of work per 32 of them, latency, takes some UNIT_COST times as long as one
+// term does in bulk).  When these have cost as much as bringing every member up
+// to date would, or there are more than CAND_MAX of them, that is done instead:
+// exact ties come back pass after pass.  6,000 members with 600 fast ones, by
+// threes at one place each 5.2 ms, by thirties 15 (25 with a block to each
+// candidate and no limit but CAND_MAX, 19 with that at 8; 10 where every pass
+// was exact, which takes 5 for 600 places against 1.5).  Where candidates are
+// few neither limit matters: CAND_MAX 8, 32 and 128 and UNIT_COST 10 to 2000
+// time alike within 1 % on the groups of 20,000- to 400,000-particle catalogues.
 constexpr int CAND_MAX = 32;
+constexpr float UNIT_COST = 50.0f;
 
 template <int BS>
 struct BlockShared {
@@ -1076,6 +1086,7 @@ struct BlockShared {
     float4 wa[2][BS / 32], wb[2][BS / 32];
     float pub_w[2][3], pub_mW[2], pub_mass[2];   // W, its magnitude and the group's mass
     int ncand;
+    int spent;                  // candidates' terms (per 32) since potentials were brought up to date
     ArgRed cand[CAND_MAX];
     unsigned long long candq[CAND_MAX];
 };
@@ -1248,17 +1259,17 @@ struct BlockGroup {
             return MAX ? x.v > best.v || (x.v == best.v && x.i < best.i)
                        : x.v < best.v || (x.v == best.v && x.i < best.i);
         };
-        if (nc <= CAND_MAX && !force) {
-            if (A.subpot && nfl > n) {
-                for (int k = 0; k < nc; ++k) {
-                    const int i = S.cand[k].i;
-                    long long q = pending(qr[i], qv[i].w, n + tid, BS);
+        // (a warp for each 32 removed members of a candidate)
+        const int m = A.subpot ? nfl - n : 0, mw = (m + 31) / 32, units = nc * mw, spent = S.spent + units;
+        if (nc <= CAND_MAX && !force && (m == 0 || spent * UNIT_COST <= (float)n * (float)m)) {
+            for (int u = w; u < units; u += NW) {
+                const int k = u / mw, i = S.cand[k].i, e = n + (u - k * mw) * 32 + lane;
+                long long q = e < nfl ? pending(qr[i], qv[i].w, e, nfl) : 0;
 #pragma unroll
-                    for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(SKID_FULL, q, o);
-                    if (lane == 0 && q) atomicAdd(&S.candq[k], (unsigned long long)q);
-                }
-                __syncthreads();
+                for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(SKID_FULL, q, o);
+                if (lane == 0) atomicAdd(&S.candq[k], (unsigned long long)q);
             }
+            __syncthreads();
             if (tid < nc) {
                 const int i = S.cand[tid].i;
                 S.cand[tid].v =
@@ -1267,6 +1278,7 @@ struct BlockGroup {
             __syncthreads();
             for (int k = 0; k < nc; ++k)
                 if (better(S.cand[k])) best = S.cand[k];
+            if (tid == 0) S.spent = spent;
             __syncthreads();
             return best;
         }
@@ -1287,6 +1299,7 @@ struct BlockGroup {
             }
         }
         *flushed = true;
+        if (tid == 0) S.spent = 0;
         best = MAX ? warp_argmax(best) : warp_argmin(best);
         if (lane == 0) S.smax[w] = best;
         __syncthreads();
@@ -1404,6 +1417,7 @@ __device__ void block_group(const RemoveArgs &A, int g, BlockShared<BS> &S, floa
         S.pub_mW[0] = centre_mag(A, S.d_cm);
         S.pub_mass[0] = (float)t[0];
         S.s_imin = 0;
+        S.spent = 0;
     }
     __syncthreads();
     int nrem = 0, par = 0;           // the same on every thread
