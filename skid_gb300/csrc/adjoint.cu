@@ -1019,24 +1019,34 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
     }
     // energies, then the counts of finished blocks, cleared together
     const size_t nE = nSel > 0 ? nSel : 1, nclear = nE + (nE + 1) / 2;
-    if ((e = dalloc(A.slots, (size_t)(nSel > 0 ? nSel : 1) * sizeof(PotSlot))) ||
-        (e = dalloc(A.E, nclear)) || (e = dalloc(A.out, 3 * (size_t)(n > 0 ? n : 1))) ||
-        (e = dalloc(A.rm, (size_t)(nrows > 0 ? nrows : 1))) ||
-        (e = dalloc(A.re, (size_t)(nrows > 0 ? nrows : 1))) ||
-        (e = dalloc(A.rio, (size_t)(nrows > 0 ? nrows : 1))) ||
-        (e = dalloc(A.tbox, 2 * (size_t)(ntile > 0 ? ntile : 1))) ||
-        (e = dalloc(A.eblock, (size_t)PA_PARTS * (ntile > 0 ? ntile : 1))) ||
-        (e = dalloc(A.part, (size_t)(want_grad ? 5 : 2) * (npart > 0 ? npart : 1))))
-        return e;
+    // one buffer for all of a call's scratch, the same with and without the
+    // gradient: allocations cost as much as a small call, and the torch wrapper
+    // makes a context per pass and asks for the energies first
+    size_t bytes = 0;
+    auto take = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return at;
+    };
+    const size_t oE = take(nclear * sizeof(double)), oslots = take(nSel * sizeof(PotSlot)),
+                 orm = take(nrows * sizeof(float4)), ore = take(nrows * sizeof(float)),
+                 orio = take(nrows * sizeof(int)), obox = take(2 * ntile * sizeof(float4)),
+                 oeb = take(PA_PARTS * ntile * sizeof(double)),
+                 opart = take(one ? 0 : 5 * npart * sizeof(float));
+    if ((e = dalloc(A.ws, bytes)) || (e = dalloc(A.out, 3 * (size_t)(n > 0 ? n : 1)))) return e;
+    unsigned char *ws = A.ws.p;
+    PotSlot *d_slots = reinterpret_cast<PotSlot *>(ws + oslots);
+    float *part = reinterpret_cast<float *>(ws + opart);
+    A.E = reinterpret_cast<double *>(ws + oE);
     if (nSel) {
-        if ((e = cudaMemcpyAsync(A.slots.p, slots.data(), nSel * sizeof(PotSlot), cudaMemcpyHostToDevice, st)))
+        if ((e = cudaMemcpyAsync(d_slots, slots.data(), nSel * sizeof(PotSlot), cudaMemcpyHostToDevice, st)))
             return e;
-        if ((e = cudaMemsetAsync(A.E.p, 0, nclear * sizeof(double), st))) return e;
+        if ((e = cudaMemsetAsync(A.E, 0, nclear * sizeof(double), st))) return e;
     }
     if (want_grad && (e = cudaMemsetAsync(A.out.p, 0, 3 * (size_t)(n > 0 ? n : 1) * sizeof(float), st))) return e;
     if (!nitems) return cudaSuccess;
     PotAdjArgs a;
-    a.slots = reinterpret_cast<const PotSlot *>(A.slots.p);
+    a.slots = d_slots;
     a.nslot = nSel;
     a.nitems = nitems;
     a.nrows = nrows;
@@ -1050,19 +1060,19 @@ cudaError_t potential_adjoint(const GroupState &G, const float4 *pos4, const flo
     a.G = Gc;
     a.plummer = plummer;
     a.perm = nullptr;
-    a.rm = A.rm.p;
-    a.re = A.re.p;
-    a.rio = A.rio.p;
-    a.tlo = A.tbox.p;
-    a.thi = A.tbox.p + ntile;
+    a.rm = reinterpret_cast<float4 *>(ws + orm);
+    a.re = reinterpret_cast<float *>(ws + ore);
+    a.rio = reinterpret_cast<int *>(ws + orio);
+    a.tlo = reinterpret_cast<float4 *>(ws + obox);
+    a.thi = a.tlo + ntile;
     a.ntile = ntile;
-    a.pphi = reinterpret_cast<float2 *>(A.part.p);
-    a.pgx = A.part.p + 2 * npart;
+    a.pphi = reinterpret_cast<float2 *>(part);
+    a.pgx = part + 2 * npart;
     a.pgy = a.pgx + npart;
     a.pgz = a.pgy + npart;
-    a.eblock = A.eblock.p;
-    a.E = A.E.p;
-    a.done = reinterpret_cast<int *>(A.E.p + nE);
+    a.eblock = reinterpret_cast<double *>(ws + oeb);
+    a.E = A.E;
+    a.done = reinterpret_cast<int *>(A.E + nE);
     a.grad = want_grad ? A.out.p : nullptr;
     const long long most = (long long)num_sms() * 32;
     const int rgrid = grid_for((int)(nrows < (1 << 30) ? nrows : 1 << 30));

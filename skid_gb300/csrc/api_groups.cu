@@ -179,7 +179,7 @@ int skid_potential_adjoint(skid_ctx *ctx, int iSoftType, float G, int nSel, cons
                                       ctx->adj, ctx->ss, st);
     if (e == cudaErrorMemoryAllocation) return ctx->fail(SKID_ENOMEM);
     CK(e);
-    if (nSel) CK(cudaMemcpyAsync(E, ctx->adj.E.p, nSel * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (nSel) CK(cudaMemcpyAsync(E, ctx->adj.E, nSel * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (dLdx)
         CK(cudaMemcpyAsync(dLdx, ctx->adj.out.p, 3 * (size_t)ctx->n * sizeof(float), cudaMemcpyDeviceToHost,
                            st));

@@ -122,14 +122,8 @@ struct AdjointState {
     DBuf<int> nbr, ncnt;        // stored ball lists, `cap` per scatterer
     int cap = 0;
     bool lists = false;         // lists match the current density
-    DBuf<unsigned char> slots;  // selected groups of a potential call
-    DBuf<float4> rm;            // their members packed: relative position, mass
-    DBuf<float> re;             // softening
-    DBuf<int> rio;              // iOrder
-    DBuf<float4> tbox;          // boxes of their row tiles
-    DBuf<float> part;           // their rows' sums over each chunk of columns
-    DBuf<double> eblock;        // energies of blocks of their rows
-    DBuf<double> E;             // energies, then counts of finished blocks (ints)
+    DBuf<unsigned char> ws;     // a potential call's scratch
+    double *E = nullptr;        // in it: the energies
 };
 cudaError_t density_adjoint(const Tree &t, const float *ball2_sorted, const int *sidx, const float *w_io,
                             int n_io, float3 L, bool per, int mode, int k, AdjointState &A,
@@ -420,7 +414,7 @@ struct skid_ctx {
         dfree(probe_f); dfree(probe_acc); dfree(probe_p4); dfree(probe_i); dfree(probe_i2);
         dfree(stat_start); dfree(stat_out); dfree(tipsy_raw); dfree(knn_heap); dfree(split_acc); dfree(split_cnt); dfree(ms_dev);
         dfree(adj.win); dfree(adj.w); dfree(adj.g); dfree(adj.out); dfree(adj.nbr); dfree(adj.ncnt);
-        dfree(adj.slots); dfree(adj.rm); dfree(adj.re); dfree(adj.rio); dfree(adj.tbox); dfree(adj.part); dfree(adj.eblock); dfree(adj.E);
+        dfree(adj.ws);
         std::lock_guard<std::recursive_mutex> lk(skid::device_mutex());
         if (d_scal) cudaFree(d_scal);
         if (d_fbytes) cudaFree(d_fbytes);
