@@ -1122,11 +1122,11 @@ __device__ __forceinline__ float centre_mag(const RemoveArgs &A, const double *d
 //    decision and the next centre to one float step; the block's last warp
 //    (the keeper) meanwhile brings the FP64 centre and the records in global
 //    memory up to date behind the pass that follows.
-// Removal at 2^21 (264 groups above 1024 members, the largest 10.7k, up to
-// 1008 removed from one) 10.4 ms with the exact terms every pass, members in
-// L2 and three barriers, now 4.6; 300 groups of up to 6.6k 2.2 to 0.73; 5k
-// particles 1.51 to 0.63.  A pass over 600 members takes 3300 cycles, over
-// 3700 3700, over 9000 (2300 of them in global memory) 11000.  What was
+// Removal at 2^21 (271 groups above 1024 members, the largest of 10,024, up to
+// 1,092 removed from one of 9,620) 4.65 ms, 10.4 with the exact terms every
+// pass, members in L2 and three barriers; 300 groups of up to 6.6k 2.2 to 0.66;
+// 5k particles 1.51 to 0.63.  A pass over 600 members takes 3300 cycles, over
+// 3700 3700.  What was
 // measured and left out: members in packed records in global memory too, the
 // next record loaded ahead, and velocities instead of w in the records (so
 // that the keeper reads none) were each no faster.
@@ -1259,9 +1259,10 @@ struct BlockGroup {
             return MAX ? x.v > best.v || (x.v == best.v && x.i < best.i)
                        : x.v < best.v || (x.v == best.v && x.i < best.i);
         };
-        // (a warp for each 32 removed members of a candidate)
+        // (a warp for each 32 removed members of a candidate; in bulk, each thread
+        // all of them in turn for its members)
         const int m = A.subpot ? nfl - n : 0, mw = (m + 31) / 32, units = nc * mw, spent = S.spent + units;
-        if (nc <= CAND_MAX && !force && (m == 0 || spent * UNIT_COST <= (float)n * (float)m)) {
+        if (nc <= CAND_MAX && !force && (m == 0 || spent * UNIT_COST <= (float)max(n, BS) * (float)m)) {
             for (int u = w; u < units; u += NW) {
                 const int k = u / mw, i = S.cand[k].i, e = n + (u - k * mw) * 32 + lane;
                 long long q = e < nfl ? pending(qr[i], qv[i].w, e, nfl) : 0;
@@ -2136,7 +2137,10 @@ cudaError_t remove_smem_limit(int *dyn_max)
 }
 
 // Shared memory a block of a plain removal launch takes: 32 B for each member
-// of the largest group, up to LCAP_KB.
+// of the largest group, up to LCAP_KB.  One block an SM for every other group
+// then, and still the fastest: at 220 / 110 / 48 KB a group of 10,000 members
+// over 2,000 of 1,300 takes 2.26 / 2.81 / 3.18 ms, over 300 of 3,000 2.09 /
+// 2.78 / 3.13.
 #ifndef SKID_LCAP_KB
 #define SKID_LCAP_KB 220
 #endif
