@@ -20,7 +20,7 @@ time over ranks.
 
 The metric compares two GPU forms at identical accuracy: the default form
 (moves driven by the fused density-field adjoint kernel, every unbinding
-group in one autotuned launch) is ``value``; the plain form (a separate
+group in one autotuned pass) is ``value``; the plain form (a separate
 gradient pass then a move kernel every step, and one potential and one
 removal launch per group, the reference's serial loop) is timed the same way
 and reported under ``config.plain`` with its per-particle catalogue agreement
@@ -595,7 +595,7 @@ def run_gpu(args):
                    "step_ms": [round(x, 3) for x in step_ms],
                    "e2e_step_ms": [round(x, 3) for x in e2e_ms],
                    "form": "fused density-field adjoint + move kernel; every unbinding group "
-                           "in one autotuned launch",
+                           "in one autotuned pass",
                    "unbind_schedule": sched, "plain": plain, "nsp": nsp},
         "e2e": {"value": job_value(world, n, args.steps, e2e_tot), "unit": UNIT,
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

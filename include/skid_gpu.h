@@ -352,9 +352,10 @@ int skid_field_adjoint(skid_ctx *ctx, int nm, const float *mpos, const float *w,
  * before skid_unbind), E[s] = -1/2 sum_{i != j in g} G m_i m_j
  * psi(r_ij, eps_i + eps_j) with kdCellPot's pair potential (grav.c:8-36,
  * grav.h:11-31) on coordinates relative to the group's reference point
- * (kd.c:1338-1352); FP32 pair sums, FP64 group totals.  With dLdx non-NULL,
- * dLdx[3n] (by iOrder) receives sum_s v[s] dE[s]/dx (0 outside the selected
- * groups). */
+ * (kd.c:1338-1352); FP32 pair sums, FP64 group totals, the same bits on every
+ * call.  With dLdx non-NULL, dLdx[3n] (by iOrder) receives sum_s v[s] dE[s]/dx
+ * (0 outside the selected groups).  A group selected more than once has its
+ * energy in each place, and the gradient of one of them. */
 int skid_potential_adjoint(skid_ctx *ctx, int iSoftType, float G, int nSel, const int *sel,
                            const float *v, double *E, float *dLdx);
 

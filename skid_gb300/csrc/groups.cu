@@ -141,7 +141,10 @@ __device__ __forceinline__ void group_store(const GroupSums &S, int c, const flo
 
 // One warp per group of up to GP_WARP_MAX members, the whole block for a
 // larger one: a warp alone walks 35k members in 1.04 ms (latency and the slow
-// FP64 adds), 0.155 ms for the block.
+// FP64 adds), 0.155 ms for the block.  A call that groups and sums, at limits
+// of 256 / 1024 / 4096, ms: 3,000 groups of 300 .74 / .68 / .68, of 600 1.37 /
+// 1.31 / 1.30, 100 of 2,000 .20 / .20 / .22, 50 of 4,000 .21 / .21 / .27, 500 of
+// 4,000 1.42 / 1.41 / 1.52.
 constexpr int GP_WARP_MAX = 1024;
 
 __global__ void __launch_bounds__(GP_THREADS)

@@ -211,7 +211,7 @@ __device__ __noinline__ int2 kb_span(const float *values, int m, int l, int h)
 // then bisection of the bit patterns, then (it >= KB_TIGHTEN) of those between
 // the least and the largest value left: where many distances are equal but for
 // rounding (a lattice, a shell of it at the k-th) no count is k and the values
-// are a few patterns apart.  200,000 points of a lattice, k = 128: 2.53 to 2.20
+// are a few patterns apart.  200,000 points of a lattice, k = 128: 2.53 to 2.06
 // ms.  Lanes that are done have no use for it.
 template <int S>
 __device__ __forceinline__ float kb_kth(const KnnBuf &B, int m, int k, int lo, float hi, int cl, int ch,
