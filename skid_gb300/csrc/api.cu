@@ -346,6 +346,8 @@ __global__ void unsort_xyz(const int *__restrict__ perm, const float *__restrict
 //   random, 5,003 scatterers     .06 / .15   .33 / .42   .31 / .37   .34 / .27  .38 / .21
 //   neighbours, 131,072          .06 / .14   .09 / .17   .14 / .20   .20 / .20  .49 / .25
 //   neighbours, 5,003            .06 / .15   .09 / .17   .12 / .18   .14 / .19     -
+// With one mover per warp no walk is shared, and the order is left alone (5,000
+// random positions .09 / .15, 50,000 .27 / .28).
 // A position's sum runs over the copies in tree order whichever positions share
 // its warp, so the order does not change the values -- but for 4, 8 or 16
 // movers per warp, when asked for: which of a position's lanes sums a copy then
@@ -365,7 +367,8 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
         return ctx->fail(SKID_ENOMEM);
     CK(cudaMemcpyAsync(xyz.p, mpos, 3 * (size_t)nm * sizeof(float), cudaMemcpyHostToDevice, st));
     xyz_to_pos4<<<grid_for(nm), 256, 0, st>>>(xyz.p, nm, p4.p); skid::note_launch();
-    const bool sorted = nm >= PROBE_SORT_MIN;
+    const int G = ctx->opt_G ? ctx->opt_G : 32;   // a forced movers-per-warp applies here too
+    const bool sorted = G > 1 && nm >= PROBE_SORT_MIN;
     if (sorted) {
         CK(curve_order(p4.p, nm, ctx->ss, st));
         CK(cudaMemcpyAsync(act.p, ctx->ss.v0.p, (size_t)nm * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -378,7 +381,7 @@ static int field_probe(skid_ctx *ctx, int nm, const float *mpos)
     a.mpos = p4.p;
     a.act = act.p;
     a.d_nA = act.p + nm;
-    a.G = ctx->opt_G ? ctx->opt_G : 32;   // a forced movers-per-warp applies here too
+    a.G = G;
     a.stats = nullptr;
     a.part_acc = nullptr;   // a probe walks each position in one warp
     a.part_cnt = nullptr;

@@ -31,4 +31,11 @@ def test_few_positions_are_not_sorted(gpu_ready):
             # pack, order, field
             assert launched <= 3 or nm >= 128, (nm, launched)
             assert np.array_equal(ctx.field_adjoint(y[:nm], w[:nm]), -w[:nm, None] * a), nm
+        # one position per warp: no walk is shared
+        ctx.set_option("field_movers_per_warp", 1)
+        before = ctx.timings()["kernel_launches"]
+        a = ctx.field(y)
+        assert ctx.timings()["kernel_launches"] - before <= 3
+        assert np.array_equal(ctx.field(y[::-1])[::-1], a)
+        ctx.set_option("field_movers_per_warp", 0)
         assert ctx.field(y[:0]).shape == (0, 3)
